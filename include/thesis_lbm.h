@@ -304,7 +304,12 @@ long long lbm_fluid_nodes(lbm_handle h);
  * kernel.  THESIS_LBM_KERNEL=scalar|pair|tma|jit|jit2 in the environment at
  * lbm_create selects one (jit2: the run-time specialised two-node kernel); a
  * variant the lattice does not admit falls back to 1, except jit and jit2,
- * whose build failure lbm_create reports. */
+ * whose build failure lbm_create reports.  With the default choice, calls of
+ * several steps on a 2D lattice that fits the SMs' shared memory (about
+ * 440,000 nodes; F32, or F16S in physics mode; boundaries that touch only
+ * the node's own populations) run in one cooperative launch with the same
+ * node arithmetic (lbm_resident.cu); a stream under capture records a launch
+ * per step. */
 int lbm_kernel_variant(lbm_handle h);
 
 /* Empty when the handle runs the kernel lbm_create meant to use; otherwise

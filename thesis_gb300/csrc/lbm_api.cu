@@ -17,6 +17,7 @@
 
 #include "lbm_flags.h"
 #include "lbm_jit.h"
+#include "lbm_resident.h"
 #include "lbm_step_tma.cuh"
 
 namespace lbm {
@@ -124,6 +125,12 @@ struct lbm_handle_s {
     unsigned int *tma_err = nullptr;
     int tma_nrows = 0, tma_stages = 0, tma_grid = 0;
     size_t tma_smem = 0;
+    // many steps per launch with the populations on chip (2D lattices that fit)
+    const void *res_kern = nullptr;
+    ResidentPlan res_plan;
+    unsigned long long *res_mail = nullptr;
+    unsigned *res_err = nullptr;
+    unsigned res_tag = 0;
     double omega = 1, omega_m = 1, gshift = 0;
     float scale = 1024.f;
 };
@@ -180,7 +187,7 @@ static void free_handle(lbm_handle_s *H) {
     void *ptrs[] = {H->fbuf[0], H->fbuf[1], H->word, H->slot, H->mask, H->kind, H->uvw,
                     H->rho, H->ux, H->uy, H->uz, H->pux, H->puy, H->puz, H->partial, H->norms,
                     H->tma_row, H->tma_lmask, H->tma_omask, H->tma_err, H->mdiff_prev, H->fd_snap,
-                    H->bcq, H->bc_macro};
+                    H->bcq, H->bc_macro, H->res_mail, H->res_err};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (H->stepped) cudaEventDestroy(H->stepped);
@@ -350,9 +357,46 @@ static int setup_jit(lbm_handle_s *H, const HostArray<uint32_t> &word, bool pair
     return LBM_OK;
 }
 
-// A bounded wait inside the row-staged kernel that gave up leaves a code in
-// tma_err; report it once the stream is idle.
+// The on-chip multi-step kernel for the default kernel choice of a 2D lattice
+// that fits (resident_plan), whose boundary conditions touch only the node's
+// own populations: open outlets and curved walls read neighbours from the
+// read buffer, which that kernel does not keep.  F16S in reference mode and
+// F64 keep the launch per step.
+static int setup_resident(lbm_handle_s *H) {
+    if (H->q != 9 || !H->jit_kernel || H->jit_key.pair || one_node_boundaries(H->P, H->q) || H->bc_macro) return LBM_OK;
+    const bool phys = H->P.mode == LBM_MODE_PHYSICS;
+    if (H->P.storage != LBM_STORE_F32 && !(H->P.storage == LBM_STORE_F16S && phys)) return LBM_OK;
+    int dev = 0, sms = 0, coop = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop || !resident_plan(H->n, H->m, (int)H->elem, sms, &H->res_plan)) return LBM_OK;
+    const void *kern = resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan);
+    if (!kern) return LBM_OK;
+    const size_t bytes = sizeof(unsigned long long) * 16 * (size_t)H->N;
+    cudaError_t e = cudaMalloc((void **)&H->res_mail, bytes);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&H->res_err, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(H->res_mail, 0, bytes);
+    if (e == cudaSuccess) e = cudaMemset(H->res_err, 0, sizeof(unsigned));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // no room for the messages: a launch per step
+        return LBM_OK;
+    }
+    H->res_kern = kern;
+    return LBM_OK;
+}
+
+// A bounded wait inside the row-staged or the on-chip kernel that gave up
+// leaves a code on the device; report it once the stream is idle.
 static int check_tma(lbm_handle_s *H) {
+    if (H->res_kern) {
+        unsigned int err = 0;
+        CUDA_TRY(cudaMemcpy(&err, H->res_err, sizeof(err), cudaMemcpyDeviceToHost));
+        if (err) {
+            H->status = LBM_ERR_CUDA;
+            return fail(LBM_ERR_CUDA, "on-chip steps: a wait for a neighbouring tile gave up");
+        }
+    }
     if (!H->tma_kernel) return LBM_OK;
     unsigned int err = 0;
     CUDA_TRY(cudaMemcpy(&err, H->tma_err, sizeof(err), cudaMemcpyDeviceToHost));
@@ -430,7 +474,7 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
     long long fl = 0;
     for (long long i = 0; i < N; ++i) fl += (L->node_type[i] & 1);
     H->fluid = fl;
-    bool want_tma = false, want_jit = false, jit_required = false, jit_pair = false;
+    bool want_tma = false, want_jit = false, jit_required = false, jit_pair = false, kernel_chosen = false;
     int jit_hspace = -1;
     {
         // Default: the one-node kernel specialised at run time for this
@@ -439,6 +483,7 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
         // the run-time build is unavailable.  THESIS_LBM_KERNEL=scalar|pair|
         // tma|jit selects a variant explicitly (jit then fails loudly).
         const char *kv = getenv("THESIS_LBM_KERNEL");
+        kernel_chosen = kv && *kv;
         // the two-node kernels have no curved-wall or extrapolation-outlet path
         const bool can_pair = (L->n % 2 == 0) && (P->storage == LBM_STORE_F32 || P->storage == LBM_STORE_F16S) &&
                               !one_node_boundaries(*P, q);
@@ -568,6 +613,13 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
     if (e != cudaSuccess) {
         free_handle(H);
         return fail(LBM_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
+    }
+    if (!kernel_chosen) {
+        rc = setup_resident(H);
+        if (rc) {
+            free_handle(H);
+            return rc;
+        }
     }
     *out = H;
     return LBM_OK;
@@ -784,11 +836,49 @@ static int pair_graph(lbm_handle_s *H, int c) {
     return LBM_OK;
 }
 
+// Fewest steps of a call that the on-chip kernel takes: it moves the state
+// on and off the chip once per call.
+constexpr int RESIDENT_MIN_STEPS = 4;
+constexpr int RESIDENT_CHUNK = 8192;  // steps per launch, tens of milliseconds
+
+static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cudaStream_t s) {
+    for (int done = 0; done < nsteps;) {
+        const int k = std::min(nsteps - done, RESIDENT_CHUNK);
+        ResidentArgs a;
+        a.p = make_params(H, H->cur, 0);
+        a.last = make_params(H, H->cur, write_macro_last && done + k == nsteps);
+        a.steps = k;
+        a.gx = H->res_plan.gx;
+        a.gy = H->res_plan.gy;
+        a.compute = H->res_plan.compute;
+        a.wrap = H->jit_key.wrap;
+        a.tag = H->res_tag;
+        a.mail = H->res_mail;
+        a.err = H->res_err;
+        const int e = resident_launch(H->res_kern, H->res_plan, a, s);
+        if (e != cudaSuccess) {
+            H->status = LBM_ERR_CUDA;
+            return fail(LBM_ERR_CUDA, std::string("on-chip step launch: ") + cudaGetErrorString((cudaError_t)e));
+        }
+        H->res_tag += (unsigned)k;
+        H->cur ^= 1;
+        done += k;
+    }
+    CUDA_TRY(cudaEventRecord(H->stepped, s));
+    return LBM_OK;
+}
+
 int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     if (!H->initialised) return fail(LBM_ERR_INVALID, "lbm_init has not been called");
     if (nsteps < 0) return fail(LBM_ERR_INVALID, "negative step count");
     cudaStream_t s = stream ? (cudaStream_t)stream : H->stream;
+    if (H->res_kern && nsteps >= RESIDENT_MIN_STEPS) {
+        // a stream under capture records plain launches, as it always did
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (stream && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap == cudaStreamCaptureStatusNone) return resident_steps(H, nsteps, write_macro_last, s);
+    }
     int plain = nsteps - (write_macro_last && nsteps > 0 ? 1 : 0);
     int rc;
     if (plain >= 8) {
