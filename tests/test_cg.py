@@ -320,3 +320,23 @@ def test_cg_gpu_storage_laplace_against_f64():
     # above it)
     assert errs[N.STORE_F32][0] < 5e-2 and errs[N.STORE_F32][1] < 5e-2
     assert errs[N.STORE_F16S][0] < 0.1 and errs[N.STORE_F16S][1] < 8.0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m", [(5, 5), (31, 7), (32, 8), (33, 9), (34, 17), (63, 15), (66, 6)])
+@pytest.mark.parametrize("ho,enh", COMBOS)
+def test_cg_gpu_tile_edges(n, m, ho, enh):
+    """Lattices around the step's 32 x 8 tiles: one partial tile, exact tiles,
+    one or two nodes into the next (the ring around a tile then wraps or
+    falls on threads beyond the lattice).  Tolerance as
+    test_cg_gpu_matches_oracle: a few ulps of O(1) values."""
+    a, p, r0, b0 = _gpu_case(n, m, ho, enh, seed=n)
+    orc = po.run_oracle_cg(n, m, p, r0, b0, 7, fp64=False, extra_collide=True)
+    with mp.CgSolver(n, m, a) as s:
+        s.init(r0, b0)
+        s.step(3, write_macro=False)
+        s.step(4, write_macro=True)
+        rf, bf = s.populations()
+        mac = s.macro()
+    for g, o in zip([rf, bf] + list(mac), (orc.rfc, orc.bfc, orc.rr, orc.br, orc.u, orc.v)):
+        assert np.abs(g - o).max() < 2e-5

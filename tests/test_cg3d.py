@@ -173,3 +173,21 @@ def test_cg3d_gpu_laplace_law():
     assert abs(s8 - s12) < 0.1 * pred, (s8, s12)
     assert abs(s8 - pred) < 0.15 * pred and abs(s12 - pred) < 0.15 * pred, (s8, s12, pred)
     print("3D Laplace: sigma = R dp / 2 = %.4e (R 8), %.4e (R 12); predicted %.4e" % (s8, s12, pred))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m,h", [(5, 5, 5), (31, 7, 6), (32, 8, 5), (33, 9, 7), (64, 5, 33), (66, 6, 17)])
+@pytest.mark.parametrize("enh", [0, 1])
+def test_cg3d_gpu_tile_edges(n, m, h, enh):
+    """Lattices around the marching step's 32 x 4 tiles and its cuts along z
+    (18-neighbour gradient).  Tolerance as test_cg3d_gpu_matches_oracle."""
+    a, p, r0, b0 = _gpu_case(n, m, h, 0, enh, seed=n)
+    orc = po.run_oracle_cg3(n, m, h, p, r0, b0, 6, fp64=False, extra_collide=True)
+    with mp.CgSolver(n, m, a, h=h) as s:
+        s.init(r0, b0)
+        s.step(2, write_macro=False)
+        s.step(4, write_macro=True)
+        rf, bf = s.populations()
+        mac = s.macro()
+    for g, o in zip([rf, bf] + list(mac), (orc.rfc, orc.bfc, orc.rr, orc.br, orc.u, orc.v, orc.w)):
+        assert np.abs(g - o).max() < 2e-5

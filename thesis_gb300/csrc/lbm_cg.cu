@@ -4,21 +4,23 @@
 // gpuUpdateMacro2DCG, GpuUpdateMacro.cu:43-135; Laplace-law sums,
 // Iterate.cu:496-499).
 //
-// The collision of a node needs the colour field (rho_r - rho_b)/rho of its
-// 8 (3x3 stencil) or 24 (5x5 stencil) neighbours after streaming, so a step is
-// two launches over the lattice:
-//   cg_density_kernel  pull both colours, write the colour field
-//                      phi = (rho_r - rho_b)/rho and rho per node;
-//   cg_collide_kernel  pull both colours again, take the neighbours' phi and
-//                      rho for the gradients, collide, perturb, recolour,
-//                      write both post-collision colours and rho_r, rho_b.
+// The collision of a node needs the colour field phi = (rho_r - rho_b)/rho of
+// its 8 (3x3 stencil) or 24 (5x5 stencil) neighbours after streaming.  One
+// launch does a step: a block owns a tile of nodes, pulls both colours of each
+// into registers, and of a ring of 1 (or 2) nodes around the tile pulls them
+// only to form phi and rho; those meet in shared memory for the gradients,
+// and the collision, perturbation and recolouring continue from the registers.
 // State between steps: post-collision red and blue populations, SoA by
-// direction, pull double buffer.  Both kernels are HBM-bound: 72 B of
-// populations read by each, 72 B written by the second, 8 B of densities.
+// direction, pull double buffer.  HBM-bound: 72 B of populations read and 72 B
+// written per node in FP32; the ring's loads (1.33x with a 32 x 8 tile) are the
+// neighbouring blocks' own and hit L2.  In practice the issue of about 900
+// instructions per 32 nodes binds it (73 % of issue slots): 1024^2, FP32, 52 us
+// a step in two launches that pulled twice, 40 us in one; F16S 54 and 42 us.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 #include <string>
 #include <vector>
@@ -31,20 +33,21 @@
 namespace lbm {
 namespace {
 
+template <class V>
 struct CgArgs {
-    const void *in;          // slot c of direction d at (c*9 + d)*N (lbm_cg_store.cuh)
-    void *out;
-    float *R, *B;            // colour densities (output)
-    void *phi, *dn;          // colour field and density of the streamed state (gradients), arithmetic type
+    CgSlots<9> s;            // lbm_cg_store.cuh
+    float *R, *B;            // colour densities (output, when write_rb)
     float *rho, *ux, *uy;    // macroscopic output (when write_macro)
     int nx, ny;
     long long N;
-    int write_macro;
-    double r_alpha, b_alpha, r_visc, b_visc, beta, A, g_limit;
-    float scale, inv_scale;  // F16S: S and 1/S of the summed population
+    int write_macro, write_rb;
+    CgModel<V> p;
 };
 
-constexpr int CG_BLOCK = 128;
+constexpr int CG_TX = 32, CG_TY = 8;  // tile of a block, one node per thread
+// rest weights phi_k + theta_k alpha; in constant memory, where they cost an
+// operand: as literals they change which products the compiler fuses, and so
+// the last bits of a droplet's small velocities
 __constant__ float c_phi[9] = {0.f, 0.2f, 0.2f, 0.2f, 0.2f, 0.05f, 0.05f, 0.05f, 0.05f};
 __constant__ float c_teta[9] = {1.f, -0.2f, -0.2f, -0.2f, -0.2f, -0.05f, -0.05f, -0.05f, -0.05f};
 __constant__ double c_phi_d[9] = {0., 0.2, 0.2, 0.2, 0.2, 0.05, 0.05, 0.05, 0.05};
@@ -62,68 +65,98 @@ template <class R> __device__ __forceinline__ R cg_rest_teta(int k) {
 __device__ __forceinline__ int wrapi(int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); }
 
 // PULL: gather from the neighbours (a time step); otherwise read the node's
-// own populations (the first collision from a given post-stream state).
+// own populations (the first collision from a given post-stream state).  Node
+// indices are unsigned 32-bit (fewer than 2^31 nodes), added to a base per
+// direction that is the same for every thread: no 64-bit index per load.
 template <int ST, bool PULL>
-__device__ __forceinline__ void cg_gather(const CgArgs &a, int x, int y, typename CgStore<ST>::R (&r)[9],
-                                          typename CgStore<ST>::R (&b)[9]) {
+__device__ __forceinline__ void cg_gather(const CgArgs<typename CgStore<ST>::R> &a, int x, int y,
+                                          typename CgStore<ST>::R (&r)[9], typename CgStore<ST>::R (&b)[9]) {
     using L = Lat<9>;
     using S = CgStore<ST>;
     using T = typename S::T;
     using R = typename S::R;
-    const T *in = (const T *)a.in;
+    const unsigned X[3] = {(unsigned)(x == 0 ? a.nx - 1 : x - 1), (unsigned)x, (unsigned)(x == a.nx - 1 ? 0 : x + 1)};
+    const unsigned Y[3] = {(unsigned)a.nx * (unsigned)(y == 0 ? a.ny - 1 : y - 1), (unsigned)a.nx * (unsigned)y,
+                           (unsigned)a.nx * (unsigned)(y == a.ny - 1 ? 0 : y + 1)};
 #pragma unroll
     for (int d = 0; d < 9; ++d) {
-        const int sx = PULL ? wrapi(x - L::cx(d), a.nx) : x;
-        const int sy = PULL ? wrapi(y - L::cy(d), a.ny) : y;
-        const long long s = sx + (long long)a.nx * sy;
-        S::load(in + d * a.N + s, in + (9 + d) * a.N + s, (R)L::w(d), (R)a.inv_scale, r[d], b[d]);
+        const unsigned s = PULL ? X[1 - L::cx(d)] + Y[1 - L::cy(d)] : X[1] + Y[1];
+        S::load((const T *)a.s.in[d] + s, (const T *)a.s.in[9 + d] + s, (R)L::w(d), a.p.inv_scale, r[d], b[d]);
     }
-}
-
-template <int ST, bool PULL>
-__global__ void __launch_bounds__(CG_BLOCK) cg_density_kernel(const CgArgs a) {
-    using R = typename CgStore<ST>::R;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= a.nx) return;
-    R r[9], b[9];
-    cg_gather<ST, PULL>(a, x, y, r, b);
-    R rr = 0, bb = 0;
-#pragma unroll
-    for (int d = 0; d < 9; ++d) {
-        rr += r[d];
-        bb += b[d];
-    }
-    const int node = x + a.nx * y;
-    const R rho = rr + bb;
-    ((R *)a.phi)[node] = (rr - bb) / rho;
-    ((R *)a.dn)[node] = rho;
 }
 
 template <int ST, bool PULL, bool HO, bool ENH>
-__global__ void __launch_bounds__(CG_BLOCK) cg_collide_kernel(const CgArgs a) {
+__global__ void __launch_bounds__(CG_TX * CG_TY, 6) cg_step_kernel(const CgArgs<typename CgStore<ST>::R> a) {
     using L = Lat<9>;
     using SP = CgStore<ST>;
     using T = typename SP::T;
     using R = typename SP::R;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= a.nx) return;
-    const int node = x + a.nx * y;
-    const R *phi = (const R *)a.phi, *dn = (const R *)a.dn;
-    R r[9], b[9];
-    cg_gather<ST, PULL>(a, x, y, r, b);
+    constexpr int H = HO ? 2 : 1, W = CG_TX + 2 * H, RING = 2 * H * W + 2 * H * CG_TY;
+    static_assert(RING <= CG_TX * CG_TY, "one ring node per thread");
+    __shared__ R s_phi[(CG_TY + 2 * H) * W];
+    __shared__ R s_dn[ENH ? (CG_TY + 2 * H) * W : 1];
+    const int tid = threadIdx.x, lx = tid % CG_TX, ly = tid / CG_TX;
+    const int x0 = blockIdx.x * CG_TX, y0 = blockIdx.y * CG_TY, x = x0 + lx, y = y0 + ly;
+    // colour field and density of tile position (cx, cy), from -H; past a
+    // lattice face the position is the wrapped node's
+    auto put = [&](int cx, int cy, R rr, R bb) {
+        const R rho = rr + bb;
+        const int c = (cy + H) * W + cx + H;
+        s_phi[c] = (rr - bb) / rho;
+        if (ENH) s_dn[c] = rho;
+    };
     R f[9], r_r = 0, b_r = 0, jx = 0, jy = 0;
+    {
+        const bool own = x < a.nx && y < a.ny;
+        if (x < a.nx + H && y < a.ny + H) {
+            R r[9], b[9];
+            cg_gather<ST, PULL>(a, own ? x : wrapi(x, a.nx), own ? y : wrapi(y, a.ny), r, b);
 #pragma unroll
-    for (int d = 0; d < 9; ++d) {
-        f[d] = r[d] + b[d];
-        r_r += r[d];
-        b_r += b[d];
-        if (L::cx(d)) jx += (R)L::cx(d) * f[d];
-        if (L::cy(d)) jy += (R)L::cy(d) * f[d];
+            for (int d = 0; d < 9; ++d) {
+                f[d] = r[d] + b[d];
+                r_r += r[d];
+                b_r += b[d];
+                if (L::cx(d)) jx += (R)L::cx(d) * f[d];
+                if (L::cy(d)) jy += (R)L::cy(d) * f[d];
+            }
+            put(lx, ly, r_r, b_r);
+        }
+        if (tid < RING) {
+            // rows below and above the tile, then the columns beside it
+            int cx, cy;
+            if (tid < 2 * H * W) {
+                const int row = tid / W;
+                cx = tid % W - H;
+                cy = row < H ? row - H : CG_TY + row - H;
+            } else {
+                const int j = tid - 2 * H * W, col = j / CG_TY;
+                cx = col < H ? col - H : CG_TX + col - H;
+                cy = j % CG_TY;
+            }
+            const int gx = x0 + cx, gy = y0 + cy;
+            if (gx < a.nx + H && gy < a.ny + H) {
+                R r[9], b[9];
+                cg_gather<ST, PULL>(a, wrapi(gx, a.nx), wrapi(gy, a.ny), r, b);
+                R rr = 0, bb = 0;
+#pragma unroll
+                for (int d = 0; d < 9; ++d) {
+                    rr += r[d];
+                    bb += b[d];
+                }
+                put(cx, cy, rr, bb);
+            }
+        }
+        __syncthreads();
+        if (!own) return;
     }
+    const int node = x + a.nx * y;
+    const R *phi = s_phi + (ly + H) * W + lx + H, *dn = s_dn + (ENH ? (ly + H) * W + lx + H : 0);
     const R rho = r_r + b_r;
     const R u = jx / rho, v = jy / rho;
-    a.R[node] = (float)r_r;
-    a.B[node] = (float)b_r;
+    if (a.write_rb) {
+        a.R[node] = (float)r_r;
+        a.B[node] = (float)b_r;
+    }
     if (a.write_macro) {
         a.rho[node] = (float)rho;
         a.ux[node] = (float)u;
@@ -138,9 +171,9 @@ __global__ void __launch_bounds__(CG_BLOCK) cg_collide_kernel(const CgArgs a) {
                                    84.,  32.,  1.,   32.,  84.,  32.,  1.,   32.,  84., 32., 1., 32.};
 #pragma unroll
         for (int k = 0; k < 24; ++k) {
-            const int j = wrapi(x + hx[k], a.nx) + a.nx * wrapi(y + hy[k], a.ny);
+            const int j = hx[k] + W * hy[k];
             const R w = (R)(hw[k] / 5040.0);
-            const R a1 = w * __ldg(phi + j), a2 = ENH ? w * __ldg(dn + j) : (R)0;
+            const R a1 = w * phi[j], a2 = ENH ? w * dn[j] : (R)0;
             if (ENH) {
                 grx += a2 * (R)hx[k];
                 gry += a2 * (R)hy[k];
@@ -151,9 +184,9 @@ __global__ void __launch_bounds__(CG_BLOCK) cg_collide_kernel(const CgArgs a) {
     } else {
 #pragma unroll
         for (int k = 1; k < 9; ++k) {
-            const int j = wrapi(x + L::cx(k), a.nx) + a.nx * wrapi(y + L::cy(k), a.ny);
+            const int j = L::cx(k) + W * L::cy(k);
             const R w = k <= 4 ? (R)(4.0 / 12.0) : (R)(1.0 / 12.0);
-            const R a1 = w * __ldg(phi + j), a2 = ENH ? w * __ldg(dn + j) : (R)0;
+            const R a1 = w * phi[j], a2 = ENH ? w * dn[j] : (R)0;
             if (ENH) {
                 grx += a2 * (R)L::cx(k);
                 gry += a2 * (R)L::cy(k);
@@ -162,19 +195,18 @@ __global__ void __launch_bounds__(CG_BLOCK) cg_collide_kernel(const CgArgs a) {
             cgy += a1 * (R)L::cy(k);
         }
     }
-    const R r_visc = (R)a.r_visc, b_visc = (R)a.b_visc, beta = (R)a.beta, A = (R)a.A;
+    const R r_visc = a.p.r_visc, b_visc = a.p.b_visc, beta = a.p.beta, A = a.p.A;
     const R mean_nu = (R)1 / (r_r / (rho * r_visc) + b_r / (rho * b_visc));
     const R omega_eff = (R)1 / ((R)3 * mean_nu + (R)0.5);
-    const R mean_alpha = (R)a.r_alpha * r_r / rho + (R)a.b_alpha * b_r / rho;
+    const R mean_alpha = a.p.r_alpha * r_r / rho + a.p.b_alpha * b_r / rho;
     const R gnorm = sqrt(cgx * cgx + cgy * cgy);
     const R k_r = r_r / rho, k_b = b_r / rho, k_k = beta * r_r * b_r / rho;
     const R cu1 = u * u + v * v;
     const R G1 = (R)2 * u * grx, G2 = u * gry + v * grx, G4 = (R)2 * v * gry;
     const R ugr = u * grx + v * gry;
-    const bool interface = gnorm > (R)a.g_limit;
+    const bool interface = gnorm > a.p.g_limit;
     // one reciprocal per node instead of two divisions per direction
     const R inv_g = interface ? (R)1 / gnorm : (R)0, inv_g2 = inv_g * inv_g;
-    T *out = (T *)a.out;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const R cxk = (R)L::cx(k), cyk = (R)L::cy(k);
@@ -196,7 +228,7 @@ __global__ void __launch_bounds__(CG_BLOCK) cg_collide_kernel(const CgArgs a) {
             feq += mean_nu * (chi * ugr + psi * TC);
         }
         const R fp = omega_eff * feq + ((R)1 - omega_eff) * f[k] + pert;
-        SP::store(out + k * a.N + node, out + (9 + k) * a.N + node, (R)L::w(k), (R)a.scale,
+        SP::store((T *)a.s.out[k] + (unsigned)node, (T *)a.s.out[9 + k] + (unsigned)node, (R)L::w(k), a.p.scale,
                   k_r * fp + k_k * cosin * rest, k_b * fp - k_k * cosin * rest);
     }
 }
@@ -292,9 +324,10 @@ struct lbm_cg_handle_s {
     int st = LBM_STORE_F32;          // population storage (lbm_cg_store.cuh)
     void *buf = nullptr;             // 2 buffers x 2 slots x q directions x N values
     float *R = nullptr, *B = nullptr, *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr;
-    void *phi = nullptr, *dn = nullptr;  // colour field and density for the gradients (arithmetic type)
+    void *phi = nullptr, *dn = nullptr;  // 3D high order: colour field and density (arithmetic type)
     double *partial = nullptr, *sums = nullptr;
     int cur = 0;
+    int sms = 1;
     float scale = 1024.f;            // F16S: scale of the summed population's deviation
     cudaStream_t stream = nullptr;
     cudaEvent_t stepped = nullptr;  // after the last lbm_cg_step, on its stream
@@ -303,13 +336,14 @@ struct lbm_cg_handle_s {
 };
 
 template <class A>
-static void cg_fill_common(const lbm_cg_handle_s *H, int from, int write_macro, A &a) {
-    a.in = H->buffer(from);
-    a.out = H->buffer(1 - from);
+static void cg_fill_common(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, A &a) {
+    const size_t one = (size_t)H->N * cg_elem_bytes(H->st);
+    for (int k = 0; k < 2 * H->q; ++k) {
+        a.s.in[k] = (const char *)H->buffer(from) + k * one;
+        a.s.out[k] = (char *)H->buffer(1 - from) + k * one;
+    }
     a.R = H->R;
     a.B = H->B;
-    a.phi = H->phi;
-    a.dn = H->dn;
     a.rho = H->rho;
     a.ux = H->ux;
     a.uy = H->uy;
@@ -317,72 +351,88 @@ static void cg_fill_common(const lbm_cg_handle_s *H, int from, int write_macro, 
     a.ny = H->m;
     a.N = H->N;
     a.write_macro = write_macro;
-    a.r_alpha = H->P.r_alpha;
-    a.b_alpha = H->P.b_alpha;
-    a.r_visc = H->P.r_viscosity;
-    a.b_visc = H->P.b_viscosity;
-    a.beta = H->P.beta;
-    a.A = H->P.A;
-    a.g_limit = H->P.g_limit;
-    a.scale = H->scale;
-    a.inv_scale = 1.0f / H->scale;
+    a.write_rb = write_rb;
+    using R = decltype(a.p.A);
+    a.p = CgModel<R>{(R)H->P.r_alpha, (R)H->P.b_alpha, (R)H->P.r_viscosity, (R)H->P.b_viscosity, (R)H->P.beta,
+                     (R)H->P.A, (R)H->P.g_limit, (R)H->scale, (R)(1.0f / H->scale)};
 }
 
-static CgArgs cg_args(const lbm_cg_handle_s *H, int from, int write_macro) {
-    CgArgs a;
+template <class R>
+static CgArgs<R> cg_args(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb) {
+    CgArgs<R> a;
     memset(&a, 0, sizeof(a));
-    cg_fill_common(H, from, write_macro, a);
+    cg_fill_common(H, from, write_macro, write_rb, a);
     return a;
 }
 
-static Cg3Args cg3_args(const lbm_cg_handle_s *H, int from, int write_macro) {
-    Cg3Args a;
+template <class R>
+static Cg3Args<R> cg3_args(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb) {
+    Cg3Args<R> a;
     memset(&a, 0, sizeof(a));
-    cg_fill_common(H, from, write_macro, a);
+    cg_fill_common(H, from, write_macro, write_rb, a);
+    a.phi = H->phi;
+    a.dn = H->dn;
     a.uz = H->uz;
     a.nz = H->h;
     return a;
 }
 
 template <int ST, bool PULL>
-static void cg3_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, cudaStream_t s) {
-    const Cg3Args a = cg3_args(H, from, write_macro);
-    const dim3 grid((unsigned)((H->n + CG3_BLOCK - 1) / CG3_BLOCK), (unsigned)H->m, (unsigned)H->h);
-    cg3_density_kernel<ST, PULL><<<grid, CG3_BLOCK, 0, s>>>(a);
+static void cg3_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
+    const auto a = cg3_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
     if (H->P.high_order) {
-        if (H->P.enhanced) cg3_collide_kernel<ST, PULL, true, true><<<grid, CG3_BLOCK, 0, s>>>(a);
-        else cg3_collide_kernel<ST, PULL, true, false><<<grid, CG3_BLOCK, 0, s>>>(a);
-    } else {
-        if (H->P.enhanced) cg3_collide_kernel<ST, PULL, false, true><<<grid, CG3_BLOCK, 0, s>>>(a);
-        else cg3_collide_kernel<ST, PULL, false, false><<<grid, CG3_BLOCK, 0, s>>>(a);
+        const dim3 grid((unsigned)((H->n + CG3_BLOCK - 1) / CG3_BLOCK), (unsigned)H->m, (unsigned)H->h);
+        cg3_density_kernel<ST, PULL><<<grid, CG3_BLOCK, 0, s>>>(a);
+        if (H->P.enhanced) cg3_collide_kernel<ST, PULL, true><<<grid, CG3_BLOCK, 0, s>>>(a);
+        else cg3_collide_kernel<ST, PULL, false><<<grid, CG3_BLOCK, 0, s>>>(a);
+        return;
     }
+    // The planes a block marches over: the cut along z with the fewest plane
+    // steps in a row, waves of resident blocks times a block's planes and the
+    // two it pulls for phi alone (256^3: 10 blocks along z, against 1 that
+    // leaves a third of the SMs' places empty, 1.41 against 1.22 ms)
+    const unsigned tx = (unsigned)((H->n + CG3_TX - 1) / CG3_TX), ty = (unsigned)((H->m + CG3_TY - 1) / CG3_TY);
+    const long long tiles = (long long)tx * ty, places = (long long)H->sms * CG3_RESIDENT;
+    int planes = H->h;
+    long long best = -1;
+    for (int c = 1; c <= (H->h + 1) / 2; ++c) {
+        const int k = (H->h + c - 1) / c;
+        const long long cost = (tiles * c + places - 1) / places * (k + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            planes = k;
+        }
+    }
+    const dim3 grid(tx, ty, (unsigned)((H->h + planes - 1) / planes));
+    if (H->P.enhanced) cg3_step_kernel<ST, PULL, true><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, planes);
+    else cg3_step_kernel<ST, PULL, false><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, planes);
 }
 
 template <int ST, bool PULL>
-static void cg_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, cudaStream_t s) {
-    const CgArgs a = cg_args(H, from, write_macro);
-    const dim3 grid((unsigned)((H->n + CG_BLOCK - 1) / CG_BLOCK), (unsigned)H->m);
-    cg_density_kernel<ST, PULL><<<grid, CG_BLOCK, 0, s>>>(a);
+static void cg_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
+    const auto a = cg_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
+    const dim3 grid((unsigned)((H->n + CG_TX - 1) / CG_TX), (unsigned)((H->m + CG_TY - 1) / CG_TY));
+    constexpr int CG_BLOCK = CG_TX * CG_TY;
     if (H->P.high_order) {
-        if (H->P.enhanced) cg_collide_kernel<ST, PULL, true, true><<<grid, CG_BLOCK, 0, s>>>(a);
-        else cg_collide_kernel<ST, PULL, true, false><<<grid, CG_BLOCK, 0, s>>>(a);
+        if (H->P.enhanced) cg_step_kernel<ST, PULL, true, true><<<grid, CG_BLOCK, 0, s>>>(a);
+        else cg_step_kernel<ST, PULL, true, false><<<grid, CG_BLOCK, 0, s>>>(a);
     } else {
-        if (H->P.enhanced) cg_collide_kernel<ST, PULL, false, true><<<grid, CG_BLOCK, 0, s>>>(a);
-        else cg_collide_kernel<ST, PULL, false, false><<<grid, CG_BLOCK, 0, s>>>(a);
+        if (H->P.enhanced) cg_step_kernel<ST, PULL, false, true><<<grid, CG_BLOCK, 0, s>>>(a);
+        else cg_step_kernel<ST, PULL, false, false><<<grid, CG_BLOCK, 0, s>>>(a);
     }
 }
 
 // One step (PULL) or the first collision from a given post-stream state.
 template <bool PULL>
-static void cg_any_launch(const lbm_cg_handle_s *H, int from, int write_macro, cudaStream_t s) {
+static void cg_any_launch(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
     if (H->q == 19) {
-        if (H->st == LBM_STORE_F16S) cg3_launch_st<LBM_STORE_F16S, PULL>(H, from, write_macro, s);
-        else if (H->st == LBM_STORE_F64) cg3_launch_st<LBM_STORE_F64, PULL>(H, from, write_macro, s);
-        else cg3_launch_st<LBM_STORE_F32, PULL>(H, from, write_macro, s);
+        if (H->st == LBM_STORE_F16S) cg3_launch_st<LBM_STORE_F16S, PULL>(H, from, write_macro, write_rb, s);
+        else if (H->st == LBM_STORE_F64) cg3_launch_st<LBM_STORE_F64, PULL>(H, from, write_macro, write_rb, s);
+        else cg3_launch_st<LBM_STORE_F32, PULL>(H, from, write_macro, write_rb, s);
     } else {
-        if (H->st == LBM_STORE_F16S) cg_launch_st<LBM_STORE_F16S, PULL>(H, from, write_macro, s);
-        else if (H->st == LBM_STORE_F64) cg_launch_st<LBM_STORE_F64, PULL>(H, from, write_macro, s);
-        else cg_launch_st<LBM_STORE_F32, PULL>(H, from, write_macro, s);
+        if (H->st == LBM_STORE_F16S) cg_launch_st<LBM_STORE_F16S, PULL>(H, from, write_macro, write_rb, s);
+        else if (H->st == LBM_STORE_F64) cg_launch_st<LBM_STORE_F64, PULL>(H, from, write_macro, write_rb, s);
+        else cg_launch_st<LBM_STORE_F32, PULL>(H, from, write_macro, write_rb, s);
     }
 }
 
@@ -408,11 +458,17 @@ static int cg_create(int n, int m, int h, const lbm_cg_params *P, lbm_cg_handle 
     H->N = (long long)n * m * h;
     H->P = *P;
     H->st = P->storage;
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&H->sms, cudaDevAttrMultiProcessorCount, dev);
+        if (H->sms < 1) H->sms = 1;
+    }
     const size_t N = (size_t)H->N;
     const size_t rbytes = H->st == LBM_STORE_F64 ? sizeof(double) : sizeof(float);
     cudaError_t e = cudaMalloc((void **)&H->buf, 4 * H->slot_bytes());
     if (e == cudaSuccess) e = cudaMalloc((void **)&H->R, sizeof(float) * 6 * N);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&H->phi, rbytes * 2 * N);
+    if (e == cudaSuccess && H->q == 19 && H->P.high_order) e = cudaMalloc((void **)&H->phi, rbytes * 2 * N);
     if (e == cudaSuccess) e = cudaMalloc((void **)&H->partial, sizeof(double) * (LAP_BLOCKS * 5 + 5));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&H->stepped, cudaEventDisableTiming);
@@ -425,10 +481,10 @@ static int cg_create(int n, int m, int h, const lbm_cg_params *P, lbm_cg_handle 
     H->ux = H->R + 3 * N;
     H->uy = H->R + 4 * N;
     H->uz = H->R + 5 * N;
-    H->dn = (char *)H->phi + rbytes * N;
+    if (H->phi) H->dn = (char *)H->phi + rbytes * N;
     H->sums = H->partial + LAP_BLOCKS * 5;
     cudaMemset(H->R, 0, sizeof(float) * 6 * N);
-    cudaMemset(H->phi, 0, rbytes * 2 * N);
+    if (H->phi) cudaMemset(H->phi, 0, rbytes * 2 * N);
     *out = H;
     return LBM_OK;
 }
@@ -476,7 +532,7 @@ int lbm_cg_init(lbm_cg_handle H, const float *r_f, const float *b_f) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (own) cudaFree(stage_r);
     if (e != cudaSuccess) return cg_fail(LBM_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
-    cg_any_launch<false>(H, 1, 1, H->stream);
+    cg_any_launch<false>(H, 1, 1, 1, H->stream);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) return cg_fail(LBM_ERR_CUDA, std::string("init: ") + cudaGetErrorString(e));
@@ -488,8 +544,8 @@ int lbm_cg_step(lbm_cg_handle H, int nsteps, int write_macro_last, void *stream)
     if (!H || nsteps < 0) return cg_fail(LBM_ERR_INVALID, "invalid argument");
     cudaStream_t s = stream ? (cudaStream_t)stream : H->stream;
     for (int i = 0; i < nsteps; ++i) {
-        const int wm = write_macro_last && i == nsteps - 1;
-        cg_any_launch<true>(H, H->cur, wm, s);
+        const int last = i == nsteps - 1;  // the colour densities of the call's last step are kept
+        cg_any_launch<true>(H, H->cur, write_macro_last && last, last, s);
         H->cur ^= 1;
     }
     cudaError_t e = cudaGetLastError();

@@ -91,6 +91,24 @@ template <> struct CgStore<LBM_STORE_F16S> {
     }
 };
 
+// The model's parameters in the arithmetic type, converted on the host: a
+// conversion from FP64 in every thread costs more than the operation that
+// uses it.
+template <class R>
+struct CgModel {
+    R r_alpha, b_alpha, r_visc, b_visc, beta, A, g_limit;
+    R scale, inv_scale;  // F16S: S and 1/S of the summed population
+};
+
+// Where a kernel finds slot c of direction d, formed on the host: in[c*Q + d]
+// is read from the kernel's parameters and indexed by node, where a base plus
+// (c*Q + d)*N would cost each access a 64-bit multiply-add or two.
+template <int Q>
+struct CgSlots {
+    const void *in[2 * Q];
+    void *out[2 * Q];
+};
+
 // Bytes of one stored value.
 __host__ __device__ constexpr int cg_elem_bytes(int st) {
     return st == LBM_STORE_F64 ? 8 : (st == LBM_STORE_F16S ? 2 : 4);
