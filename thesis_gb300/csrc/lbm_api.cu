@@ -1,6 +1,6 @@
 // C ABI of the lattice-Boltzmann engine (include/thesis_lbm.h): handle
 // lifetime, device allocation, initial collision, the step loop (with a
-// captured two-step CUDA graph for short steps) and read-back.
+// captured CUDA graphs for short steps) and read-back.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdlib.h>
@@ -111,7 +111,7 @@ struct lbm_handle_s {
     // recorded after the steps of every lbm_step, on the stream they ran on;
     // the handle's own stream waits for it before reductions and read-back
     cudaEvent_t stepped = nullptr;
-    cudaGraphExec_t pair[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // GRAPH_STEPS steps from buffer 0 and from buffer 1
     int status = LBM_OK;
     bool initialised = false;
     bool pair_kernel = false;  // two nodes per thread (even nx, F32/F16S)
@@ -183,7 +183,7 @@ static StepParams make_params(const lbm_handle_s *H, int from, int write_macro) 
 static void free_handle(lbm_handle_s *H) {
     if (!H) return;
     for (int c = 0; c < 2; ++c)
-        if (H->pair[c]) cudaGraphExecDestroy(H->pair[c]);
+        if (H->graph[c]) cudaGraphExecDestroy(H->graph[c]);
     void *ptrs[] = {H->fbuf[0], H->fbuf[1], H->word, H->slot, H->mask, H->kind, H->uvw,
                     H->rho, H->ux, H->uy, H->uz, H->pux, H->puy, H->puz, H->partial, H->norms,
                     H->tma_row, H->tma_lmask, H->tma_omask, H->tma_err, H->mdiff_prev, H->fd_snap,
@@ -328,7 +328,17 @@ static int setup_jit(lbm_handle_s *H, const HostArray<uint32_t> &word, bool pair
     k.hspace = !pair && (hspace > 0 || (hspace < 0 && H->P.mode == LBM_MODE_PHYSICS &&
                                         H->P.storage != LBM_STORE_F64));
     k.pred = k.hspace && hspace == 2;
-    k.zwalk = k.hspace && H->zwalk_request > 1 ? H->zwalk_request : 1;
+    // From about 400,000 nodes up, a 3D step that no one tuned takes blocks of
+    // 64 at 56 registers: 36 warps per SM hide the round trip from flag word
+    // to populations, which 20 do not.  128x128x256 duct, F16S: 88 -> 81 us a
+    // step; 192x192x256, F32: 252 -> 216; 128^3 F32: 56 -> 52; 64x64x128,
+    // F16S: 13.5 -> 11.4.  Below, the grid does not fill the SMs and the
+    // uncapped kernel is faster: 75x61x47 7.7 against 8.4.
+    if (k.hspace && hspace < 0 && H->q == 19 && H->N >= 400000) {
+        k.block = 64;
+        k.minb = 18;
+    }
+    if (k.hspace && H->zwalk_request > 1) k.zwalk = H->zwalk_request;
     if (k.hspace && H->block_request >= 32 && H->block_request <= 1024 && H->block_request % 32 == 0)
         k.block = H->block_request;
     if (k.hspace && H->minb_request > 1) k.minb = H->minb_request;
@@ -820,17 +830,21 @@ static int launch(lbm_handle_s *H, int from, int write_macro, cudaStream_t s) {
     return rc ? fail(LBM_ERR_UNSUPPORTED, "no kernel for this configuration") : LBM_OK;
 }
 
-// Two steps (from buffer c back to buffer c) captured once as a graph.
-static int pair_graph(lbm_handle_s *H, int c) {
-    if (H->pair[c]) return LBM_OK;
+// GRAPH_STEPS steps (from buffer c back to buffer c) captured once as a graph.
+// A replay costs about 2 us between graphs, which two steps per graph put on
+// every second step: a 75 x 61 x 47 MRT step took 9.7 us, 7.7 us with sixteen.
+// Calls shorter than two replays launch step by step.
+constexpr int GRAPH_STEPS = 16, GRAPH_MIN = 32;
+static int step_graph(lbm_handle_s *H, int c) {
+    if (H->graph[c]) return LBM_OK;
     cudaGraph_t g;
     CUDA_TRY(cudaStreamBeginCapture(H->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = launch(H, c, 0, H->stream);
-    if (!rc) rc = launch(H, 1 - c, 0, H->stream);
+    int rc = LBM_OK;
+    for (int k = 0; k < GRAPH_STEPS && !rc; ++k) rc = launch(H, c ^ (k & 1), 0, H->stream);
     cudaError_t e = cudaStreamEndCapture(H->stream, &g);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&H->pair[c], g, 0);
+    e = cudaGraphInstantiate(&H->graph[c], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
     return LBM_OK;
@@ -881,18 +895,14 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
     }
     int plain = nsteps - (write_macro_last && nsteps > 0 ? 1 : 0);
     int rc;
-    if (plain >= 8) {
-        if ((rc = pair_graph(H, H->cur))) return rc;
-        for (int i = 0; i + 1 < plain; i += 2) CUDA_TRY(cudaGraphLaunch(H->pair[H->cur], s));
-        if (plain & 1) {
-            if ((rc = launch(H, H->cur, 0, s))) return rc;
-            H->cur ^= 1;
-        }
-    } else {
-        for (int i = 0; i < plain; ++i) {
-            if ((rc = launch(H, H->cur, 0, s))) return rc;
-            H->cur ^= 1;
-        }
+    int done = 0;
+    if (plain >= GRAPH_MIN) {
+        if ((rc = step_graph(H, H->cur))) return rc;
+        for (; done + GRAPH_STEPS <= plain; done += GRAPH_STEPS) CUDA_TRY(cudaGraphLaunch(H->graph[H->cur], s));
+    }
+    for (; done < plain; ++done) {
+        if ((rc = launch(H, H->cur, 0, s))) return rc;
+        H->cur ^= 1;
     }
     if (nsteps > plain) {
         if ((rc = launch(H, H->cur, 1, s))) return rc;
@@ -1290,9 +1300,9 @@ int lbm_autotune(lbm_handle H, int trial_steps, int *block, int *hint, int *pred
     H->jit_key = cand[best_i];
     H->jit_fn = fn[best_i];
     for (int c = 0; c < 2; ++c)
-        if (H->pair[c]) {
-            cudaGraphExecDestroy(H->pair[c]);
-            H->pair[c] = nullptr;
+        if (H->graph[c]) {
+            cudaGraphExecDestroy(H->graph[c]);
+            H->graph[c] = nullptr;
         }
     {
         std::lock_guard<std::mutex> lock(g_tuned_mutex);
