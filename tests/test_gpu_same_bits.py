@@ -1,0 +1,60 @@
+"""Every storage-unit kernel form of a lattice gives the same bits: the
+default choice, one node per thread, walks along z, two z nodes on packed
+FP32x2, the batch and the on-chip kernel share their node arithmetic, whose
+roundings are written out.  Block and walk choices follow the extents, so the
+extents here sit around them (rows that fill blocks of 64, 96, 160 threads or
+leave lanes idle, columns that end inside a walk)."""
+import numpy as np
+import pytest
+
+from thesis_gb300 import lattice
+from thesis_gb300 import native as N
+from thesis_gb300.batch import Batch
+from thesis_gb300.solver import Arguments, Solver
+
+pytestmark = pytest.mark.gpu
+
+
+def state(monkeypatch, kernel, lat, args, steps):
+    if kernel:
+        monkeypatch.setenv("THESIS_LBM_KERNEL", kernel)
+    else:
+        monkeypatch.delenv("THESIS_LBM_KERNEL", raising=False)
+    nn = lat.num_nodes
+    with Solver(lat, args) as s:
+        s.init(np.ones(nn), np.zeros(nn), np.zeros(nn), np.zeros(nn))
+        s.step(steps)
+        return s.get_state()
+
+
+@pytest.mark.parametrize("shape", [(64, 64, 49), (96, 96, 110), (75, 61, 47), (150, 90, 75), (33, 100, 65)])
+@pytest.mark.parametrize("coll", [N.BGKW, N.TRT, N.MRT])
+@pytest.mark.parametrize("storage", [N.STORE_F32, N.STORE_F16S])
+def test_duct(monkeypatch, shape, coll, storage):
+    lat = lattice.sphere_duct(*shape, porosity=0.8, rmin=4, rmax=8, seed=2)
+    args = Arguments(viscosity=0.1, collision_model=coll, mode=N.MODE_PHYSICS, storage=storage, init_equilibrium=1,
+                     inlet_profile=N.INLET_PRESSURE, outlet_profile=N.OUTLET_PRESSURE, rho_in=1.005, rho_out=1.0)
+    want = state(monkeypatch, "jith", lat, args, 20)
+    for kernel in ("", "jithz3b96m12", "jithz4b64m10q"):
+        assert np.array_equal(state(monkeypatch, kernel, lat, args, 20), want), kernel
+
+
+@pytest.mark.parametrize("coll", [N.BGKW, N.TRT, N.MRT])
+@pytest.mark.parametrize("storage", [N.STORE_F32, N.STORE_F16S])
+def test_channel(monkeypatch, coll, storage):
+    lat = lattice.channel2d(197, 83, seed=3, size_scale=0.3)
+    args = Arguments(u=0.05, viscosity=0.03, collision_model=coll, mode=N.MODE_PHYSICS, storage=storage,
+                     init_equilibrium=1, outlet_profile=N.OUTLET_PRESSURE, rho_out=1.0)
+    want = state(monkeypatch, "jith", lat, args, 20)
+    assert np.array_equal(state(monkeypatch, "", lat, args, 20), want)
+    nn = lat.num_nodes
+    z = np.zeros(nn)
+    with Solver(lat, args) as s, Batch([lat, lat], [args, args]) as b:
+        s.init(np.ones(nn), z, z, z)
+        s.step(20)
+        b.init()
+        for d in range(2):
+            b.init_fields(d, np.ones(nn), z, z, z)
+        b.step(20)
+        for d in range(2):
+            assert np.array_equal(b.populations(d), s.populations())

@@ -328,15 +328,28 @@ static int setup_jit(lbm_handle_s *H, const HostArray<uint32_t> &word, bool pair
     k.hspace = !pair && (hspace > 0 || (hspace < 0 && H->P.mode == LBM_MODE_PHYSICS &&
                                         H->P.storage != LBM_STORE_F64));
     k.pred = k.hspace && hspace == 2;
-    // From about 400,000 nodes up, a 3D step that no one tuned takes blocks of
-    // 64 at 56 registers: 36 warps per SM hide the round trip from flag word
-    // to populations, which 20 do not.  128x128x256 duct, F16S: 88 -> 81 us a
-    // step; 192x192x256, F32: 252 -> 216; 128^3 F32: 56 -> 52; 64x64x128,
-    // F16S: 13.5 -> 11.4.  Below, the grid does not fill the SMs and the
-    // uncapped kernel is faster: 75x61x47 7.7 against 8.4.
-    if (k.hspace && hspace < 0 && H->q == 19 && H->N >= 400000) {
-        k.block = 64;
-        k.minb = 18;
+    // A 3D step that no one tuned runs 36 warps per SM (56 registers): they
+    // hide the round trip from flag word to populations, which the uncapped
+    // kernel's 20 do not.  Its blocks are the multiple of 32 threads, 64 to
+    // 224, that covers a row with the fewest idle lanes.  128x128x256 duct,
+    // F16S: 88 -> 81 us a step; 192x192x256, F32: 252 -> 216; 150x140x130,
+    // F16S: 72 -> 58 (blocks of 64: 62); 75x61x47, F32: 7.9 -> 7.4 (8.4).
+    // Below 200,000 nodes the grid does not fill the SMs either way (32^3:
+    // 3.5 against 4.0 us).  16-bit storage of a million nodes and more also
+    // walks three nodes along z per thread with the next flag word in flight:
+    // 81 -> 74, 58 -> 54.5, 224^3 220 -> 202; with FP32, whose loads take
+    // twice the bytes, the walk gains nothing (216 and 212, 39.3 and 40.7).
+    if (k.hspace && hspace < 0 && H->q == 19 && H->N >= 200000) {
+        long long best = -1;
+        for (int b = 64; b <= 224; b += 32) {
+            const long long lanes = ((long long)H->n + b - 1) / b * b;
+            if (best < 0 || lanes < best) {
+                best = lanes;
+                k.block = b;
+            }
+        }
+        k.minb = 36 * 32 / k.block;
+        if (H->elem == 2 && H->N >= 1000000) k.zwalk = 3;
     }
     if (k.hspace && H->zwalk_request > 1) k.zwalk = H->zwalk_request;
     if (k.hspace && H->block_request >= 32 && H->block_request <= 1024 && H->block_request % 32 == 0)

@@ -36,16 +36,21 @@ __device__ __forceinline__ f2 operator-(f2 a) { return f2(__fmul2_rn(a.v, make_f
 __device__ __forceinline__ f2 &operator+=(f2 &a, f2 b) { return a = a + b; }
 __device__ __forceinline__ f2 &operator-=(f2 &a, f2 b) { return a = a - b; }
 
-// One lane: the same collision code on one node per thread (h_node).
+// One lane: the same collision code on one node per thread (h_node).  Its
+// operations round one by one, like the pair's, and multiply-adds are written
+// out (fma2) wherever one is meant: left to the compiler, which products it
+// fuses changes with the code around them (a loop along z was enough), and
+// with 16-bit storage one bit decides a rounding that the flow never forgets.
+// So every kernel form, one node or two, gives the same bits.
 struct f1 {
     float v;
     __device__ __forceinline__ f1() {}
     __device__ __forceinline__ f1(float s) : v(s) {}
 };
-__device__ __forceinline__ f1 operator+(f1 a, f1 b) { return f1(a.v + b.v); }
-__device__ __forceinline__ f1 operator*(f1 a, f1 b) { return f1(a.v * b.v); }
+__device__ __forceinline__ f1 operator+(f1 a, f1 b) { return f1(__fadd_rn(a.v, b.v)); }
+__device__ __forceinline__ f1 operator*(f1 a, f1 b) { return f1(__fmul_rn(a.v, b.v)); }
 __device__ __forceinline__ f1 fma2(f1 a, f1 b, f1 c) { return f1(fmaf(a.v, b.v, c.v)); }
-__device__ __forceinline__ f1 operator-(f1 a, f1 b) { return f1(a.v - b.v); }
+__device__ __forceinline__ f1 operator-(f1 a, f1 b) { return f1(__fsub_rn(a.v, b.v)); }
 __device__ __forceinline__ f1 operator-(f1 a) { return f1(-a.v); }
 __device__ __forceinline__ f1 &operator+=(f1 &a, f1 b) { return a = a + b; }
 __device__ __forceinline__ f1 &operator-=(f1 &a, f1 b) { return a = a - b; }
@@ -85,9 +90,10 @@ template <> struct Pair<LBM_STORE_F16S> {
 // D3Q19 MRT shift w~ has (rho, e, eps) = (1, -11, 0); the other moments
 // vanish by isotropy.
 
-// BGK / TRT in h units: h_eq,d = S w_d [(rho - sigma) + rho (3 cu + 4.5 cu^2 - 1.5 u^2)].
+// BGK / TRT in h units: h - h_eq,d for a value h of direction d, with
+// h_eq,d = S w_d [(rho - sigma) + rho (3 cu + 4.5 cu^2 - 1.5 u^2)].
 template <int Q, class V>
-__device__ __forceinline__ V heq(int d, V rho_m_sigma, V rho, V ux, V uy, V uz, V usq15, float S) {
+__device__ __forceinline__ V minus_heq(V h, int d, V rho_m_sigma, V rho, V ux, V uy, V uz, V usq15, float S) {
     using L = Lat<Q>;
     V cu = 0.f;
     if (L::cx(d)) cu = L::cx(d) > 0 ? ux : -ux;
@@ -95,7 +101,7 @@ __device__ __forceinline__ V heq(int d, V rho_m_sigma, V rho, V ux, V uy, V uz, 
     if (L::cz(d)) cu = L::cz(d) > 0 ? cu + uz : cu - uz;
     // rho (3 cu + 4.5 cu^2 - 1.5 u^2) = rho (cu (3 + 4.5 cu) - usq15)
     const V poly = fma2(cu, fma2(cu, V(4.5f), V(3.f)), -usq15);
-    return V((float)(L::w(d)) * S) * fma2(rho, poly, rho_m_sigma);
+    return fma2(V(-((float)(L::w(d)) * S)), fma2(rho, poly, rho_m_sigma), h);
 }
 
 template <int Q, class V>
@@ -104,7 +110,7 @@ __device__ __forceinline__ void collide_bgk_x2(V (&h)[Q], V rho, V rms, V ux, V 
     const V usq15 = V(1.5f) * fma2(ux, ux, fma2(uy, uy, uz * uz));
     const V om(omega);
 #pragma unroll
-    for (int d = 0; d < Q; ++d) h[d] = fma2(-om, h[d] - heq<Q>(d, rms, rho, ux, uy, uz, usq15, S), h[d]);
+    for (int d = 0; d < Q; ++d) h[d] = fma2(-om, minus_heq<Q>(h[d], d, rms, rho, ux, uy, uz, usq15, S), h[d]);
 }
 
 template <int Q, class V>
@@ -112,25 +118,29 @@ __device__ __forceinline__ void collide_trt_x2(V (&h)[Q], V rho, V rms, V ux, V 
                                                float omega_m, float S) {
     using L = Lat<Q>;
     const V usq15 = V(1.5f) * fma2(ux, ux, fma2(uy, uy, uz * uz));
-    V e[Q];
+    V n[Q];
 #pragma unroll
-    for (int d = 0; d < Q; ++d) e[d] = heq<Q>(d, rms, rho, ux, uy, uz, usq15, S);
-    V out[Q];
+    for (int d = 0; d < Q; ++d) n[d] = minus_heq<Q>(h[d], d, rms, rho, ux, uy, uz, usq15, S);
     const V hp(0.5f * omega), hm(0.5f * omega_m);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
         const int o = L::opp(d);
-        const V nd = h[d] - e[d], no = h[o] - e[o];
-        out[d] = h[d] - fma2(hp, nd + no, hm * (nd - no));
+        h[d] = h[d] - fma2(hp, n[d] + n[o], hm * (n[d] - n[o]));
     }
-#pragma unroll
-    for (int d = 0; d < Q; ++d) h[d] = out[d];
 }
 
 // D3Q19 MRT in h units, in the pair-sum form of collide_mrt19 (lbm_device.cuh):
 // d_k = s_k/|m_k|^2 (m_k(h) - S (m_eq,k - sigma m_k(w~))), with w~ the
 // model's rest state (rest_shift): m(w~) = (1, -11, 0, 0, ...).
-template <bool REF, class V>
+// UNIT: the scale S is 1 (a compile-time fact for FP32 storage), so a product
+// equilibrium joins its moment in one multiply-add.
+template <bool UNIT, class V>
+__device__ __forceinline__ V minus_scaled(V m, float S, V a, V b) {  // m - S a b
+    if (UNIT) return fma2(-a, b, m);
+    return m - V(S) * (a * b);
+}
+
+template <bool REF, bool UNIT, class V>
 __device__ __forceinline__ void collide_mrt19_x2(V (&h)[19], V rho, V rms, V ux, V uy, V uz, float omega,
                                                  float sigma, float S) {
     const V sX = h[1] + h[2], aX = h[1] - h[2];
@@ -167,24 +177,22 @@ __device__ __forceinline__ void collide_mrt19_x2(V (&h)[19], V rho, V rms, V ux,
     const V Sv(S);
     // S (m_eq,k - sigma m_k(w)) for the non-conserved moments
     const V E1 = Sv * fma2(V(-11.f), rms, V(19.f) * jsq);
-    // the storage shift is this model's rest state, whose eps moment is 0
-    const V E2 = Sv * (V((float)(-475.0 / 63.0)) * jsq);
-    const V c23 = V((float)(-2.0 / 3.0) * S);
+    const V nc23 = V(-((float)(-2.0 / 3.0) * S));
     const V d1 = V((float)(1.19 / 2394.0)) * (m1 - E1);
-    const V d2 = V((float)(1.4 / 252.0)) * (m2 - E2);
-    const V d4 = V((float)(1.2 / 40.0)) * (m4 - c23 * jx);
-    const V d6 = V((float)(1.2 / 40.0)) * (m6 - c23 * jy);
-    const V d8 = V((float)(1.2 / 40.0)) * (m8 - c23 * jz);
+    // the storage shift is this model's rest state, whose eps moment is 0
+    const V d2 = V((float)(1.4 / 252.0)) * minus_scaled<UNIT>(m2, S, V((float)(-475.0 / 63.0)), jsq);
+    const V d4 = V((float)(1.2 / 40.0)) * fma2(nc23, jx, m4);
+    const V d6 = V((float)(1.2 / 40.0)) * fma2(nc23, jy, m6);
+    const V d8 = V((float)(1.2 / 40.0)) * fma2(nc23, jz, m8);
     const V d9 = V(omega / 36.f) * (m9 - Sv * (fma2(V(2.f), jx2, -jy2) - jz2));
     const V d10 = V((float)(1.4 / 72.0)) * m10;
     const V d11 = V(omega / 12.f) * (m11 - Sv * (jy2 - jz2));
     const V d12 = V((float)(1.4 / 24.0)) * m12;
-    const V w4(0.25f * omega);
-    const V d13 = w4 * (m13 - Sv * (jx * jy));
-    const V d14 = w4 * (m14 - Sv * (jy * jz));
-    const V d15 = w4 * (m15 - Sv * (jx * jz));
-    const V g16(1.98f / 8.f);
-    const V d16 = g16 * m16, d17 = g16 * m17, d18 = g16 * m18;
+    const V w4(0.25f * omega), nw4(-(0.25f * omega));
+    const V x13 = minus_scaled<UNIT>(m13, S, jy, jx), x14 = minus_scaled<UNIT>(m14, S, jz, jy),
+            x15 = minus_scaled<UNIT>(m15, S, jz, jx);
+    const V g16(1.98f / 8.f), ng16(-(1.98f / 8.f));
+    const V d16 = g16 * m16, d17 = g16 * m17;
     const V P = fma2(V(-11.f), d1, V(-4.f) * d2);
     const V EX = fma2(V(2.f), d9, fma2(V(-4.f), d10, P));
     const V EYZb = fma2(V(2.f), d10, P - d9);
@@ -193,9 +201,9 @@ __device__ __forceinline__ void collide_mrt19_x2(V (&h)[19], V rho, V rms, V ux,
     const V G = fma2(V(8.f), d1, d2), H = d9 + d10, K = d11 + d12;
     const V GH = G + H;
     const V GHp = GH + K, GHm = GH - K, G2H = fma2(V(-2.f), H, G);
-    const V OA = (d4 + d6) + (d16 - d17), OB = (d6 - d4) - (d16 + d17);
-    const V OC = (d4 + d8) + (d18 - d16), OD = (d8 - d4) + (d16 + d18);
-    const V OE = (d6 + d8) + (d17 - d18), OF = (d8 - d6) - (d17 + d18);
+    const V OA = (d4 + d6) + fma2(g16, m16, -d17), OB = (d6 - d4) - fma2(g16, m16, d17);
+    const V OC = (d4 + d8) + fma2(g16, m18, -d16), OD = (d8 - d4) + fma2(g16, m18, d16);
+    const V OE = (d6 + d8) + fma2(ng16, m18, d17), OF = (d8 - d6) - fma2(g16, m18, d17);
     const V m4d4 = V(-4.f) * d4, m4d6 = V(-4.f) * d6, m4d8 = V(-4.f) * d8;
     h[0] = h0 - fma2(V(-30.f), d1, V(12.f) * d2);
     h[1] -= EX + m4d4;
@@ -204,7 +212,8 @@ __device__ __forceinline__ void collide_mrt19_x2(V (&h)[19], V rho, V rms, V ux,
     h[4] -= EY - m4d6;
     h[5] -= EZ + m4d8;
     h[6] -= EZ - m4d8;
-    const V eA = GHp + d13, eB = GHp - d13, eC = GHm + d15, eD = GHm - d15, eE = G2H + d14, eF = G2H - d14;
+    const V eA = fma2(w4, x13, GHp), eB = fma2(nw4, x13, GHp), eC = fma2(w4, x15, GHm), eD = fma2(nw4, x15, GHm),
+            eE = fma2(w4, x14, G2H), eF = fma2(nw4, x14, G2H);
     h[7] -= eA + OA;
     h[10] -= eA - OA;
     h[8] -= eB + OB;
@@ -222,23 +231,13 @@ __device__ __forceinline__ void collide_mrt19_x2(V (&h)[19], V rho, V rms, V ux,
 
 // D2Q9 MRT in h units (CellFunctions.cu:7-63 basis and rates); REF keeps the
 // reference's energy equilibria with the extra density factor.
-template <bool REF, class V>
+template <bool REF, bool UNIT, class V>
 __device__ __forceinline__ void collide_mrt9_x2(V (&h)[9], V rho, V rms, V ux, V uy, float omega, float sigma,
                                                 float S) {
     const V usq = fma2(ux, ux, uy * uy);
-    const V ef = REF ? rho : V(1.f);
     const V Sv(S);
-    const V rs = rho * usq * ef;
-    V E[9];
-    E[0] = 0.f;
-    E[1] = Sv * fma2(V(3.f), rs, V(-2.f) * rms);
-    E[2] = Sv * fma2(V(-3.f), rs, rms);
-    E[3] = Sv * (rho * ux);
-    E[4] = -E[3];
-    E[5] = Sv * (rho * uy);
-    E[6] = -E[5];
-    E[7] = Sv * (rho * (ux * ux - uy * uy));
-    E[8] = Sv * (rho * (ux * uy));
+    const V ru = rho * usq, rs = REF ? ru * rho : ru;
+    const V E1 = Sv * fma2(V(3.f), rs, V(-2.f) * rms), E2 = Sv * fma2(V(-3.f), rs, rms);
     // The moment transform of the D2Q9 matrix (mrt2) in pair form: with
     // opposite pairs (1,3), (2,4), (5,7), (6,8), the even moments (e, eps,
     // pxx, pxy) take the pair sums and the odd ones (qx, qy) the pair
@@ -254,11 +253,15 @@ __device__ __forceinline__ void collide_mrt9_x2(V (&h)[9], V rho, V rms, V ux, V
     const V m6 = fma2(V(-2.f), b, c + d);                      // qy
     const V m7 = A - B;                                        // pxx
     const V m8 = C - D;                                        // pxy
-    const V dm1 = V(1.4f / 36.f) * (m1 - E[1]), dm2 = V(1.4f / 36.f) * (m2 - E[2]);
-    const V dm4 = V(1.2f / 12.f) * (m4 - E[4]), dm6 = V(1.2f / 12.f) * (m6 - E[6]);
-    const V dm7 = V(omega / 4.f) * (m7 - E[7]), dm8 = V(omega / 4.f) * (m8 - E[8]);
+    const V dm1 = V(1.4f / 36.f) * (m1 - E1), dm2 = V(1.4f / 36.f) * (m2 - E2);
+    const V k2(1.2f / 12.f);
+    const V dm4 = k2 * (UNIT ? fma2(rho, ux, m4) : m4 + Sv * (rho * ux));
+    const V dm6 = k2 * (UNIT ? fma2(rho, uy, m6) : m6 + Sv * (rho * uy));
+    const V x7 = minus_scaled<UNIT>(m7, S, rho, fma2(ux, ux, -(uy * uy)));
+    const V x8 = minus_scaled<UNIT>(m8, S, rho, ux * uy);
+    const V o4(omega / 4.f), no4(-(omega / 4.f));
     const V t1 = fma2(V(-2.f), dm2, -dm1), t2 = fma2(V(2.f), dm1, dm2);
-    const V S13 = t1 + dm7, S24 = t1 - dm7, S57 = t2 + dm8, S68 = t2 - dm8;
+    const V S13 = fma2(o4, x7, t1), S24 = fma2(no4, x7, t1), S57 = fma2(o4, x8, t2), S68 = fma2(no4, x8, t2);
     const V O13 = V(-2.f) * dm4, O24 = V(-2.f) * dm6, O57 = dm4 + dm6, O68 = dm6 - dm4;
     h[0] -= V(4.f) * (dm2 - dm1);
     h[1] -= S13 + O13;
@@ -273,18 +276,19 @@ __device__ __forceinline__ void collide_mrt9_x2(V (&h)[9], V rho, V rms, V ux, V
 
 // rms = rho - sigma, the density's deviation from the shift's density,
 // formed as sum(h)/S by the caller: no FP32 cancellation of rho - 1.
-template <int Q, int COLL, bool PHYS, class V>
+template <int Q, int COLL, int ST, bool PHYS, class V>
 __device__ __forceinline__ void collide_x2(V (&h)[Q], V rho, V rms, V ux, V uy, V uz, const StepParams &p,
                                            float sigma, float S) {
+    constexpr bool UNIT = ST != LBM_STORE_F16S && ST != LBM_STORE_F16C;
     if (COLL == LBM_BGKW) {
         collide_bgk_x2<Q>(h, rho, rms, ux, uy, uz, (float)p.omega, S);
     } else if (COLL == LBM_TRT) {
         collide_trt_x2<Q>(h, rho, rms, ux, uy, uz, (float)p.omega, (float)p.omega_m, S);
     } else {
         if constexpr (Q == 9)
-            collide_mrt9_x2<!PHYS>(h, rho, rms, ux, uy, (float)p.omega, sigma, S);
+            collide_mrt9_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, (float)p.omega, sigma, S);
         else
-            collide_mrt19_x2<!PHYS>(h, rho, rms, ux, uy, uz, (float)p.omega, sigma, S);
+            collide_mrt19_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, uz, (float)p.omega, sigma, S);
     }
 }
 
@@ -435,7 +439,7 @@ __device__ __forceinline__ void pair_node(const StepParams &p, const G &g, int x
         if (L::cy(d) == 1) jy += h[d]; else if (L::cy(d) == -1) jy -= h[d];
         if (L::cz(d) == 1) jz += h[d]; else if (L::cz(d) == -1) jz -= h[d];
     }
-    f2 rms = sum * f2(invS);
+    f2 rms = F16 ? sum * f2(invS) : sum;
     f2 rho = rms + f2(sigma);
     const f2 irho(1.f / rho.v.x, 1.f / rho.v.y);
     const f2 sc = irho * f2(invS);
@@ -459,7 +463,7 @@ __device__ __forceinline__ void pair_node(const StepParams &p, const G &g, int x
         }
     }
 
-    collide_x2<Q, COLL, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
+    collide_x2<Q, COLL, ST, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
 
     // a solid node of a mixed pair keeps the zero encoding
     if (!fl0 || !fl1) {
@@ -569,7 +573,7 @@ __device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int no
         if (L::cy(d) == 1) jy += h[d]; else if (L::cy(d) == -1) jy -= h[d];
         if (L::cz(d) == 1) jz += h[d]; else if (L::cz(d) == -1) jz -= h[d];
     }
-    f1 rms = sum * f1(invS);
+    f1 rms = F16 ? sum * f1(invS) : sum;
     f1 rho = rms + f1(sigma);
     const f1 sc = f1(invS / rho.v);
     f1 ux = fma2(jx, sc, f1((float)p.gshift)), uy = jy * sc, uz = jz * sc;
@@ -596,7 +600,7 @@ __device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int no
         p.uy[node] = uy.v;
         p.uz[node] = uz.v;
     }
-    collide_x2<Q, COLL, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
+    collide_x2<Q, COLL, ST, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
 }
 
 template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G, bool SPEC, int HB = 0>
@@ -778,7 +782,7 @@ __device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x
         if (L::cy(d) == 1) jy += h[d]; else if (L::cy(d) == -1) jy -= h[d];
         if (L::cz(d) == 1) jz += h[d]; else if (L::cz(d) == -1) jz -= h[d];
     }
-    const f2 rms = sum * f2(invS);
+    const f2 rms = F16 ? sum * f2(invS) : sum;
     const f2 rho = rms + f2(sigma);
     // a solid lane's rho is sigma + 0 = 1 (F16S/F32 shifted) or 0 (unshifted);
     // guard the reciprocal, its results are discarded
@@ -799,7 +803,7 @@ __device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x
             p.uz[node1] = uz.v.y;
         }
     }
-    collide_x2<Q, COLL, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
+    collide_x2<Q, COLL, ST, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
     if (in_row) {
 #pragma unroll
         for (int d = 0; d < Q; ++d) {
