@@ -58,3 +58,37 @@ def test_channel(monkeypatch, coll, storage):
         b.step(20)
         for d in range(2):
             assert np.array_equal(b.populations(d), s.populations())
+
+
+@pytest.mark.parametrize("periodic", [(1, 1, 1), (0, 1, 0)])
+@pytest.mark.parametrize("storage", [N.STORE_F32, N.STORE_F16S])
+@pytest.mark.parametrize("dims", [2, 3])
+def test_batch_sizes(monkeypatch, periodic, storage, dims):
+    """Domains around the batch's tiles (32 nodes by an even number of rows):
+    one row, odd rows, pairs that wrap, scattered solids; three dimensions,
+    where rows of a tile span planes."""
+    monkeypatch.setenv("THESIS_LBM_KERNEL", "jith")
+    rng = np.random.default_rng(4)
+    shapes = [(31, 1, 1), (32, 2, 1), (33, 3, 1), (65, 37, 1), (130, 64, 1)] if dims == 2 else [(20, 10, 7), (33, 5, 3)]
+    lats, args, starts = [], [], []
+    for n, m, h in shapes:
+        nn = n * m * h
+        fluid = (rng.random(nn) > 0.1).astype(np.int32)
+        lats.append(lattice.Lattice(dims, n, m, h, fluid))
+        args.append(Arguments(viscosity=0.06, collision_model=N.MRT, mode=N.MODE_PHYSICS, init_equilibrium=1,
+                              storage=storage, periodic=periodic))
+        u = np.where(fluid, 0.05 * rng.standard_normal(nn), 0.0)
+        starts.append((1 + 0.01 * rng.standard_normal(nn), u, -u, np.zeros(nn)))
+    with Batch(lats, args) as b:
+        b.init()
+        for d, st in enumerate(starts):
+            b.init_fields(d, *st)
+        b.step(17)
+        got = [b.populations(d) for d in range(len(lats))]
+    for lat, a, st, f in zip(lats, args, starts, got):
+        with Solver(lat, a) as s:
+            s.init(*st)
+            s.step(17)
+            want = s.populations()
+        fl = lat.node_type == 1
+        assert np.array_equal(f[:, fl], want[:, fl])

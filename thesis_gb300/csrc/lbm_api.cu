@@ -162,6 +162,9 @@ static StepParams make_params(const lbm_handle_s *H, int from, int write_macro) 
     p.omega = H->omega;
     p.omega_m = H->omega_m;
     p.gshift = H->gshift;
+    p.omega_f = (float)p.omega;
+    p.omega_m_f = (float)p.omega_m;
+    p.gshift_f = (float)p.gshift;
     p.rho_in = H->P.rho_in;
     p.rho_out = H->P.rho_out;
     p.rho0 = H->P.rho;

@@ -34,11 +34,15 @@ int launch_decode_q19(const StepParams &p, int st, double *out, long long n, cud
 
 namespace {
 
-// A tile is one warp's work: 32 consecutive nodes of BATCH_ROWS consecutive
+// A tile is one warp's work: 32 consecutive nodes of a batch's tile rows
 // rows of one domain.  int4: x = domain, y = first row (y + ny z), z = first
 // x, w = node index of (first x, first row) in the batch's macroscopic arrays.
 constexpr int BATCH_WARPS = STEP_BLOCK / 32;
-constexpr int BATCH_ROWS = 4;
+// consecutive rows.  The rows per tile follow the active domains
+// (batch_rows): as many as divide the work evenly over the resident warps.
+constexpr int BATCH_MIN_ROWS = 2, BATCH_MAX_ROWS = 32;
+// blocks per SM the step kernel is compiled for (D3Q19 nodes need the registers)
+constexpr int batch_resident(int q) { return q == 9 ? 7 : 4; }
 constexpr int PARAM_WORDS = (int)(sizeof(StepParams) / 4);
 static_assert(sizeof(StepParams) % 4 == 0, "StepParams is copied as 32-bit words");
 
@@ -52,11 +56,18 @@ __device__ __forceinline__ void batch_load_params(StepParams *dst, const StepPar
     __syncwarp();
 }
 
+// D2Q9 advances two rows at a time on packed FP32x2 (h_ypair_w), which puts 18
+// loads in flight per thread where a row puts 9 and halves the FP32
+// instructions; a pair that holds a boundary-slot node goes row by row, as
+// D3Q19 does (two nodes would spill).  Latency-bound at 28 warps per SM.
+// Sixteen MRT cavities of sides 64..768, F16S: 60.2 us a step row by row with
+// 4-row tiles, 43.5 (6 or 8 blocks per SM: 43.7, 48.1); eight 1024 x 256 TRT
+// channels, F32: 51.9 and 46.9.
 template <int Q, int COLL, int ST, bool PHYS>
-__global__ void __launch_bounds__(STEP_BLOCK)
+__global__ void __launch_bounds__(STEP_BLOCK, batch_resident(Q))
 batch_step_kernel(const StepParams *__restrict__ tab, const int4 *__restrict__ tiles, const int *__restrict__ count) {
     __shared__ StepParams sp[BATCH_WARPS];
-    const int ntiles = *count;
+    const int ntiles = count[0], tile_rows = count[1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     StepParams &p = sp[warp];
     int cur = -1;
@@ -69,16 +80,34 @@ batch_step_kernel(const StepParams *__restrict__ tab, const int4 *__restrict__ t
         }
         const DynGeom g{p.nx, p.ny, p.nz, p.pitch};
         const int x = tl.z + lane;
-        const int rows = g.ny * g.nz;
-        const int r_end = min(tl.y + BATCH_ROWS, rows);
+        const int r_end = min(tl.y + tile_rows, g.ny * g.nz);
         const bool in_row = x < g.nx;
-        // the next row's flag word is requested before the current row's update
-        uint32_t w = in_row ? __ldg(p.word + x + g.nx * tl.y) : 0u;
+        auto flag = [&](int r) -> uint32_t { return in_row && r < r_end ? __ldg(p.word + x + g.nx * r) : 0u; };
+        // the next rows' flag words are requested before the current rows' update
+        if constexpr (Q == 9) {
+            uint32_t wa = flag(tl.y), wb = flag(tl.y + 1);
 #pragma unroll 1
-        for (int r = tl.y; r < r_end; ++r) {
-            const uint32_t wn = in_row && r + 1 < r_end ? __ldg(p.word + x + g.nx * (r + 1)) : 0u;
-            h_node_w<Q, COLL, ST, PHYS, true, DynGeom, false, false>(p, g, x, r % g.ny, r / g.ny, w);
-            w = wn;
+            for (int r = tl.y; r < r_end; r += 2) {
+                const uint32_t wc = flag(r + 2), wd = flag(r + 3);
+                const bool two = r + 1 < r_end;
+                if (two && !__any_sync(0xffffffffu, ((wa | wb) & W_SPECIAL) != 0)) {
+                    h_ypair_w<Q, COLL, ST, PHYS, true, DynGeom, 0>(p, g, x, r, 0, wa, wb);
+                } else {
+#pragma unroll 1
+                    for (int k = 0; k < (two ? 2 : 1); ++k)
+                        h_node_w<Q, COLL, ST, PHYS, true, DynGeom, false, false>(p, g, x, r + k, 0, k ? wb : wa);
+                }
+                wa = wc;
+                wb = wd;
+            }
+        } else {
+            uint32_t w = flag(tl.y);
+#pragma unroll 1
+            for (int r = tl.y; r < r_end; ++r) {
+                const uint32_t wn = flag(r + 1);
+                h_node_w<Q, COLL, ST, PHYS, true, DynGeom, false, false>(p, g, x, r % g.ny, r / g.ny, w);
+                w = wn;
+            }
         }
     }
 }
@@ -90,14 +119,14 @@ batch_step_kernel(const StepParams *__restrict__ tab, const int4 *__restrict__ t
 __global__ void __launch_bounds__(STEP_BLOCK)
 batch_residual_partial(const StepParams *__restrict__ tab, const int4 *__restrict__ tiles,
                        const int *__restrict__ count, float *pu, double2 *partial) {
-    const int ntiles = *count;
+    const int ntiles = count[0], tile_rows = count[1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int t = blockIdx.x * BATCH_WARPS + warp; t < ntiles; t += gridDim.x * BATCH_WARPS) {
         const int4 tl = tiles[t];
         const StepParams &p = tab[tl.x];
         const int nx = p.nx, rows = p.ny * p.nz;
         const int x = tl.z + lane;
-        const int r_end = min(tl.y + BATCH_ROWS, rows);
+        const int r_end = min(tl.y + tile_rows, rows);
         double a = 0, b = 0;
         if (x < nx) {
             for (int r = tl.y; r < r_end; ++r) {
@@ -177,12 +206,10 @@ struct lbm_batch_s {
     float *pu = nullptr;     // previous velocity for residuals, 3 x total_nodes
     StepParams *tab = nullptr;  // [parity 0,1][write_macro 0,1][domain]
     int4 *tiles = nullptr;
-    int *ntiles_d = nullptr;
+    int *ntiles_d = nullptr;    // {tiles, rows per tile}
     double2 *partial = nullptr;
     int2 *ranges_d = nullptr;
     double *res_d = nullptr;
-    std::vector<int4> all_tiles;       // every tile of every domain, domain-major
-    std::vector<int> dom_tile_begin;   // into all_tiles
     std::vector<char> active;
     int ntiles = 0;
     int cur = 0;                       // buffer holding the current state
@@ -240,6 +267,9 @@ static StepParams batch_params(const lbm_batch_s *B, int d, int parity, int writ
     p.omega = 1.0 / (3.0 * P.viscosity + 0.5);
     p.omega_m = 8.0 * (2.0 - p.omega) / (8.0 - p.omega);
     p.gshift = B->dims == 3 ? P.g / p.omega : 0.0;
+    p.omega_f = (float)p.omega;
+    p.omega_m_f = (float)p.omega_m;
+    p.gshift_f = (float)p.gshift;
     p.rho_in = P.rho_in;
     p.rho_out = P.rho_out;
     p.rho0 = P.rho;
@@ -257,23 +287,54 @@ static StepParams batch_params(const lbm_batch_s *B, int d, int parity, int writ
     return p;
 }
 
-// Upload the tiles of the active domains and their ranges.
+// Tiles of domain d at `rows` rows per tile.
+static long long batch_tiles_of(const lbm_batch_s *B, int d, int rows) {
+    return (long long)((B->n[d] + 31) / 32) * (((long long)B->m[d] * B->h[d] + rows - 1) / rows);
+}
+
+// Rows per tile: each resident warp takes ceil(tiles / warps) tiles, and a
+// tile costs its rows and about one more (its parameters, the first flag
+// word); the even count that makes the busiest warp's share least.  Eight
+// 1024 x 256 channels: 4 rows leave the last of four rounds 85 % empty on
+// 3648 warps, 16 rows fill 4256 warps once.
+static int batch_rows(const lbm_batch_s *B) {
+    const long long warps = (long long)B->grid * BATCH_WARPS;
+    long long best = -1;
+    int rows = BATCH_MIN_ROWS;
+    for (int r = BATCH_MIN_ROWS; r <= BATCH_MAX_ROWS; r += 2) {
+        long long t = 0;
+        for (int d = 0; d < B->ndom; ++d)
+            if (B->active[d]) t += batch_tiles_of(B, d, r);
+        const long long cost = (t + warps - 1) / warps * (r + 1);
+        if (best < 0 || cost < best) {
+            best = cost;
+            rows = r;
+        }
+    }
+    return rows;
+}
+
+// Upload the tiles of the active domains, domain-major, and their ranges.
 static int batch_upload_tiles(lbm_batch_s *B) {
     std::vector<int4> t;
     std::vector<int2> ranges(B->ndom, make_int2(0, 0));
+    const int tile_rows = batch_rows(B);
     for (int d = 0; d < B->ndom; ++d) {
-        const int b = B->dom_tile_begin[d], e = B->dom_tile_begin[d + 1];
         ranges[d] = make_int2((int)t.size(), (int)t.size());
         if (!B->active[d]) continue;
-        t.insert(t.end(), B->all_tiles.begin() + b, B->all_tiles.begin() + e);
+        const int rows = B->m[d] * B->h[d];
+        for (int r = 0; r < rows; r += tile_rows)
+            for (int x0 = 0; x0 < B->n[d]; x0 += 32)
+                t.push_back(make_int4(d, r, x0, (int)(B->node_off[d] + (long long)r * B->n[d] + x0)));
         ranges[d].y = (int)t.size();
     }
     B->ntiles = (int)t.size();
+    const int head[2] = {B->ntiles, tile_rows};
     cudaError_t err = cudaSuccess;
     if (!t.empty())
         err = cudaMemcpyAsync(B->tiles, t.data(), sizeof(int4) * t.size(), cudaMemcpyHostToDevice, B->stream);
     if (err == cudaSuccess)
-        err = cudaMemcpyAsync(B->ntiles_d, &B->ntiles, sizeof(int), cudaMemcpyHostToDevice, B->stream);
+        err = cudaMemcpyAsync(B->ntiles_d, head, sizeof(head), cudaMemcpyHostToDevice, B->stream);
     if (err == cudaSuccess)
         err = cudaMemcpyAsync(B->ranges_d, ranges.data(), sizeof(int2) * B->ndom, cudaMemcpyHostToDevice, B->stream);
     if (err == cudaSuccess) err = cudaStreamWaitEvent(B->stream, B->stepped, 0);
@@ -350,16 +411,6 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
         B->total_fluid += fl;
     }
     const long long nslots = B->slot_off[count - 1] + (long long)flags[count - 1].slot_node.size();
-    // tiles, domain-major
-    B->dom_tile_begin.push_back(0);
-    for (int d = 0; d < count; ++d) {
-        const int rows = B->m[d] * B->h[d];
-        for (int r = 0; r < rows; ++r)
-            if (r % BATCH_ROWS == 0)
-                for (int x0 = 0; x0 < B->n[d]; x0 += 32)
-                    B->all_tiles.push_back(make_int4(d, r, x0, (int)(B->node_off[d] + (long long)r * B->n[d] + x0)));
-        B->dom_tile_begin.push_back((int)B->all_tiles.size());
-    }
     if (B->total_nodes >= (1ll << 31)) {
         batch_free(B);
         return bfail(LBM_ERR_INVALID, "a batch holds fewer than 2^31 nodes");
@@ -368,7 +419,9 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
     B->dom_steps.assign(count, 0);
     B->dom_buf.assign(count, 0);
     B->residual.assign(count, INFINITY);
-    const size_t T = (size_t)B->total_nodes, NT = B->all_tiles.size();
+    size_t NT = 0;  // most tiles an upload can hold
+    for (int d = 0; d < count; ++d) NT += (size_t)batch_tiles_of(B, d, BATCH_MIN_ROWS);
+    const size_t T = (size_t)B->total_nodes;
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void **p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes ? bytes : 16);
@@ -384,7 +437,7 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
     alloc((void **)&B->pu, sizeof(float) * 3 * T);
     alloc((void **)&B->tab, sizeof(StepParams) * 4 * count);
     alloc((void **)&B->tiles, sizeof(int4) * NT);
-    alloc((void **)&B->ntiles_d, sizeof(int));
+    alloc((void **)&B->ntiles_d, 2 * sizeof(int));
     alloc((void **)&B->partial, sizeof(double2) * NT);
     alloc((void **)&B->ranges_d, sizeof(int2) * count);
     alloc((void **)&B->res_d, sizeof(double) * count);

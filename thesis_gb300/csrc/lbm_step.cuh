@@ -45,6 +45,7 @@ struct StepParams {
     int pitch;  // elements from one row of a direction to the next (Q * nx)
     int write_macro;
     double omega, omega_m, gshift;
+    float omega_f, omega_m_f, gshift_f;  // the same rounded once, for FP32 arithmetic
     double rho_in, rho_out;
     double rho0;  // reference density (moving walls)
     int ref_hh;   // reference mode: the HH wall model instead of straight walls

@@ -281,14 +281,14 @@ __device__ __forceinline__ void collide_x2(V (&h)[Q], V rho, V rms, V ux, V uy, 
                                            float sigma, float S) {
     constexpr bool UNIT = ST != LBM_STORE_F16S && ST != LBM_STORE_F16C;
     if (COLL == LBM_BGKW) {
-        collide_bgk_x2<Q>(h, rho, rms, ux, uy, uz, (float)p.omega, S);
+        collide_bgk_x2<Q>(h, rho, rms, ux, uy, uz, p.omega_f, S);
     } else if (COLL == LBM_TRT) {
-        collide_trt_x2<Q>(h, rho, rms, ux, uy, uz, (float)p.omega, (float)p.omega_m, S);
+        collide_trt_x2<Q>(h, rho, rms, ux, uy, uz, p.omega_f, p.omega_m_f, S);
     } else {
         if constexpr (Q == 9)
-            collide_mrt9_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, (float)p.omega, sigma, S);
+            collide_mrt9_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, p.omega_f, sigma, S);
         else
-            collide_mrt19_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, uz, (float)p.omega, sigma, S);
+            collide_mrt19_x2<!PHYS, UNIT>(h, rho, rms, ux, uy, uz, p.omega_f, sigma, S);
     }
 }
 
@@ -443,7 +443,7 @@ __device__ __forceinline__ void pair_node(const StepParams &p, const G &g, int x
     f2 rho = rms + f2(sigma);
     const f2 irho(1.f / rho.v.x, 1.f / rho.v.y);
     const f2 sc = irho * f2(invS);
-    f2 ux = fma2(jx, sc, f2((float)p.gshift)), uy = jy * sc, uz = jz * sc;
+    f2 ux = fma2(jx, sc, f2(p.gshift_f)), uy = jy * sc, uz = jz * sc;
     if (zv0) uy.v.x = 0.f;
     if (zv1) uy.v.y = 0.f;
     if (keep0 || keep1) {
@@ -576,7 +576,7 @@ __device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int no
     f1 rms = F16 ? sum * f1(invS) : sum;
     f1 rho = rms + f1(sigma);
     const f1 sc = f1(invS / rho.v);
-    f1 ux = fma2(jx, sc, f1((float)p.gshift)), uy = jy * sc, uz = jz * sc;
+    f1 ux = fma2(jx, sc, f1(p.gshift_f)), uy = jy * sc, uz = jz * sc;
     if (zv) uy = 0.f;
     if (PHYS && (w & W_SPECIAL) && p.bc_macro) {
         const int sl = __ldg(p.slot + node);
@@ -707,45 +707,40 @@ __device__ __forceinline__ void h_node_w(const StepParams &p, const G &g, int x,
 
 
 
-// Two nodes of one column, (x, y, z) and (x, y, z + 1), updated together:
-// each gathers by its own flag word (pull, or its own opposite population
-// across a blocked link), then moments and collision run on packed FP32x2
-// lanes (collide_x2 with f2), so one FFMA2 serves both nodes.  Neither node
-// may be a boundary-slot node (the caller takes the one-node path for a warp
-// that holds one).  A solid node loads nothing and stores its zero encoding,
-// as in h_node_w.
-template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G, int HB>
-__device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x, int y, int z, uint32_t w0,
-                                          uint32_t w1) {
+// Two nodes updated together, the second dn nodes and dp elements after the
+// first: each gathers by its own flag word (pull, or its own opposite
+// population across a blocked link), then moments and collision run on packed
+// FP32x2 lanes (collide_x2 with f2), so one FFMA2 serves both nodes, with the
+// bits of two one-node updates.  Neither node may be a boundary-slot node
+// (the caller takes the one-node path for a warp that holds one).  A solid
+// node loads nothing and stores its zero encoding, as in h_node_w.  o0 and o1
+// are the nodes' offsets to the neighbours at -x, +x, -y, +y, -z, +z.
+struct PairOffsets {
+    int xm, xp, ym, yp, zm, zp;
+};
+template <int Q, int COLL, int ST, bool PHYS, class G, int HB>
+__device__ __forceinline__ void h_pair_w(const StepParams &p, const G &g, bool in_row, int node0, long long idx, int dn,
+                                         int dp, uint32_t w0, uint32_t w1, const PairOffsets &o0,
+                                         const PairOffsets &o1) {
     using L = Lat<Q>;
     using T = typename Store<ST>::T;
     constexpr bool F16 = ST == LBM_STORE_F16S || ST == LBM_STORE_F16C;
     const float sigma = p.sigma;
     const float S = F16 ? p.scale : 1.f;
     const float invS = F16 ? p.inv_scale : 1.f;
-    const bool in_row = x < g.nx;
-    const int row0 = y + g.ny * z;
-    const int node0 = x + g.nx * row0, node1 = node0 + g.nx * g.ny;
-    const int plane = g.pitch * g.ny;
-    const long long idx = x + (long long)g.pitch * row0;
+    const int node1 = node0 + dn;
     const T *in0 = (const T *)p.fin[0] + idx;
-    const T *in1 = in0 + plane;
+    const T *in1 = in0 + dp;
     T *out0 = (T *)p.fout[0] + idx;
-    T *out1 = out0 + plane;
+    T *out1 = out0 + dp;
     const bool fl0 = (w0 & W_FLUID) != 0, fl1 = (w1 & W_FLUID) != 0;
     if (!__ballot_sync(0xffffffffu, fl0 || fl1)) return;  // a warp of solid nodes writes nothing
-    int oxm = -1, oxp = 1, oym = -g.pitch, oyp = g.pitch;
-    int ozm0 = -plane, ozp0 = plane, ozm1 = -plane, ozp1 = plane;
-    if (WRAP) {
-        oxm = x == 0 ? g.nx - 1 : -1;
-        oxp = x == g.nx - 1 ? 1 - g.nx : 1;
-        oym = y == 0 ? (g.ny - 1) * g.pitch : -g.pitch;
-        oyp = y == g.ny - 1 ? (1 - g.ny) * g.pitch : g.pitch;
-        // node 0 (at z < nz - 1) and node 1 (at z + 1 > 0) wrap on one side only
-        ozm0 = z == 0 ? (g.nz - 1) * plane : -plane;
-        ozp1 = z + 1 == g.nz - 1 ? (1 - g.nz) * plane : plane;
-    }
     auto raw = [](const T *q) -> float { return h_raw<ST>(q); };
+    auto pull = [&](const PairOffsets &o, int d) -> int {
+        return d * g.nx + (L::cx(d) == 1 ? o.xm : (L::cx(d) == -1 ? o.xp : 0)) +
+               (L::cy(d) == 1 ? o.ym : (L::cy(d) == -1 ? o.yp : 0)) +
+               (L::cz(d) == 1 ? o.zm : (L::cz(d) == -1 ? o.zp : 0));
+    };
     f2 h[Q];
     {
         const float a0 = fl0 ? raw(in0) : 0.f, a1 = fl1 ? raw(in1) : 0.f;
@@ -753,10 +748,7 @@ __device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x
     }
 #pragma unroll
     for (int d = 1; d < Q; ++d) {
-        const int pxy = d * g.nx + (L::cx(d) == 1 ? oxm : (L::cx(d) == -1 ? oxp : 0)) +
-                        (L::cy(d) == 1 ? oym : (L::cy(d) == -1 ? oyp : 0));
-        const int pull0 = pxy + (L::cz(d) == 1 ? ozm0 : (L::cz(d) == -1 ? ozp0 : 0));
-        const int pull1 = pxy + (L::cz(d) == 1 ? ozm1 : (L::cz(d) == -1 ? ozp1 : 0));
+        const int pull0 = pull(o0, d), pull1 = pull(o1, d);
         const int own = (PHYS ? L::opp(d) : d) * g.nx;
         float a0 = 0.f, a1 = 0.f;
         if constexpr (HB == 1) {
@@ -788,7 +780,7 @@ __device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x
     // guard the reciprocal, its results are discarded
     const float r0 = fl0 ? rho.v.x : 1.f, r1 = fl1 ? rho.v.y : 1.f;
     const f2 sc(invS / r0, invS / r1);
-    const f2 ux = fma2(jx, sc, f2((float)p.gshift)), uy = jy * sc, uz = jz * sc;
+    const f2 ux = fma2(jx, sc, f2(p.gshift_f)), uy = jy * sc, uz = jz * sc;
     if (p.write_macro) {
         if (fl0) {
             p.rho[node0] = rho.v.x;
@@ -812,6 +804,51 @@ __device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x
             h_put<ST>(out1 + d * g.nx, fl1 ? h[d].v.y : zero);
         }
     }
+}
+
+// The pair (x, y, z), (x, y, z + 1) of one column.
+template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G, int HB>
+__device__ __forceinline__ void h_zpair_w(const StepParams &p, const G &g, int x, int y, int z, uint32_t w0,
+                                          uint32_t w1) {
+    const int row0 = y + g.ny * z, plane = g.pitch * g.ny;
+    PairOffsets o0{-1, 1, -g.pitch, g.pitch, -plane, plane};
+    if (WRAP) {
+        o0.xm = x == 0 ? g.nx - 1 : -1;
+        o0.xp = x == g.nx - 1 ? 1 - g.nx : 1;
+        o0.ym = y == 0 ? (g.ny - 1) * g.pitch : -g.pitch;
+        o0.yp = y == g.ny - 1 ? (1 - g.ny) * g.pitch : g.pitch;
+    }
+    PairOffsets o1 = o0;
+    if (WRAP) {
+        // node 0 (at z < nz - 1) and node 1 (at z + 1 > 0) wrap on one side only
+        o0.zm = z == 0 ? (g.nz - 1) * plane : -plane;
+        o1.zp = z + 1 == g.nz - 1 ? (1 - g.nz) * plane : plane;
+    }
+    h_pair_w<Q, COLL, ST, PHYS, G, HB>(p, g, x < g.nx, x + g.nx * row0, x + (long long)g.pitch * row0, g.nx * g.ny,
+                                       plane, w0, w1, o0, o1);
+}
+
+// The pair (x, y, z), (x, y + 1, z) of one plane.
+template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G, int HB>
+__device__ __forceinline__ void h_ypair_w(const StepParams &p, const G &g, int x, int y, int z, uint32_t w0,
+                                          uint32_t w1) {
+    const int row0 = y + g.ny * z, plane = g.pitch * g.ny;
+    PairOffsets o0{-1, 1, -g.pitch, g.pitch, -plane, plane};
+    if (WRAP) {
+        o0.xm = x == 0 ? g.nx - 1 : -1;
+        o0.xp = x == g.nx - 1 ? 1 - g.nx : 1;
+        if (Q == 19) {
+            o0.zm = z == 0 ? (g.nz - 1) * plane : -plane;
+            o0.zp = z == g.nz - 1 ? (1 - g.nz) * plane : plane;
+        }
+    }
+    PairOffsets o1 = o0;
+    if (WRAP) {
+        o0.ym = y == 0 ? (g.ny - 1) * g.pitch : -g.pitch;
+        o1.yp = y + 1 == g.ny - 1 ? (1 - g.ny) * g.pitch : g.pitch;
+    }
+    h_pair_w<Q, COLL, ST, PHYS, G, HB>(p, g, x < g.nx, x + g.nx * row0, x + (long long)g.pitch * row0, g.nx, g.pitch,
+                                       w0, w1, o0, o1);
 }
 
 // One node: its flag word, then the update.
