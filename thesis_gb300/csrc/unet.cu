@@ -626,7 +626,7 @@ void conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const fl
                                  cudaSharedmemCarveoutMaxShared);                                               \
             const int occ = std::min(std::min((int)(u->smem_per_sm / (bytes + 1024)),                           \
                                               512 / std::max(32, SM::NA * CO)),                                 \
-                                     resident_by_registers((const void *)kern, 160));                          \
+                                     resident_by_registers((const void *)kern, unet_tc::CONV_THREADS));                          \
             const long long score = (long long)occ * CH * std::min(NS - 1, 2) * 1024 + occ * 128 + CH + NS;   \
             if (occ >= 1 && score > best_score) {                                                               \
                 best_score = score;                                                                             \
@@ -645,7 +645,7 @@ void conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const fl
             cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,                          \
                                  cudaSharedmemCarveoutMaxShared);                                               \
             const long long g = (long long)u->sms * best_occ < tiles ? (long long)u->sms * best_occ : tiles;    \
-            kern<<<(unsigned)g, 160, bytes, u->stream>>>(map, cin, w, bias, op, out.cs, out.co, out32, B, H, W,  \
+            kern<<<(unsigned)g, unet_tc::CONV_THREADS, bytes, u->stream>>>(map, cin, w, bias, op, out.cs, out.co, out32, B, H, W,  \
                                                          relu, u->tc_err);                                      \
         }                                                                                                       \
         ++idx;                                                                                                  \

@@ -24,13 +24,16 @@
 // address bits, so a start moved by whole rows (or by 32 bytes for the next
 // K = 16) reads the right elements with the descriptor's base offset 0.
 //
-// Warp 4 (one thread) issues the copies and each job's 9 x CHUNK/16 MMAs
-// (M = 128, N = COUT, K = 16, BF16 in, FP32 accumulate); warps 0-3 read
-// finished tiles from NA tensor-memory accumulators (each warp its 32 lanes =
-// 32 pixels), add the bias, apply ReLU and store BF16 (and FP32 if asked),
-// while the next tiles accumulate.  Every wait is bounded: a wait that gives
-// up sets *err, both roles stop, the copies and MMAs in flight finish, the
-// tensor memory is freed and the kernel returns.
+// One thread of warp 4 issues the copies, one of warp 5 each job's
+// 9 x CHUNK/16 MMAs (M = 128, N = COUT, K = 16, BF16 in, FP32 accumulate);
+// warps 0-3 read finished tiles from NA tensor-memory accumulators (each warp
+// its 32 lanes = 32 pixels), add the bias, apply ReLU and store BF16 (and FP32
+// if asked), while the next tiles accumulate.  A job's fixed cost in the
+// issuing threads is what bounds the level-0 layers, so they carry no division
+// and no 64-bit index: tiles advance by carried coordinates (TileWalk), stages
+// by counters.  Every wait is bounded: a wait that gives up sets *err, all
+// roles stop, the copies and MMAs in flight finish, the tensor memory is freed
+// and the kernel returns.
 //
 // Weight gradient (wgrad_tc_kernel): see its comment below.
 #pragma once
@@ -63,12 +66,58 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+// Descriptors as halves: the start address sits in the low one, and offsets
+// inside shared memory never carry out of its field.
+struct Desc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc(uint64_t d) : lo((uint32_t)d), hi((uint32_t)(d >> 32)) {}
+};
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, Desc a, uint32_t a_off, Desc b, uint32_t b_off, uint32_t idesc,
+                                         uint32_t acc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}\n" ::"r"(tmem_d),
+        "r"(a.lo + a_off), "r"(a.hi), "r"(b.lo + b_off), "r"(b.hi), "r"(idesc), "r"(acc));
 }
+
+// The tiles blockIdx.x, blockIdx.x + gridDim.x, ... of a (image, row, segment)
+// space with H rows and xt segments a row, as carried coordinates.
+struct TileWalk {
+    int xb, y, n, sx, sy, sn, xt, H, left;
+    __device__ __forceinline__ TileWalk(int B, int H_, int xt_) : xt(xt_), H(H_) {
+        const int first = blockIdx.x, step = gridDim.x, total = B * H * xt;
+        xb = first % xt;
+        y = first / xt % H;
+        n = first / xt / H;
+        sx = step % xt;
+        sy = step / xt % H;
+        sn = step / xt / H;
+        left = total > first ? (total - 1 - first) / step + 1 : 0;
+    }
+    __device__ __forceinline__ void next() {
+        xb += sx;
+        const int cx = xb >= xt ? 1 : 0;
+        xb -= cx ? xt : 0;
+        y += sy + cx;
+        const int cy = y >= H ? 1 : 0;
+        y -= cy ? H : 0;
+        n += sn + cy;
+        --left;
+    }
+};
+// A ring position of N slots: the slot, its barrier phase and, past the first
+// round, the phase in which the slot was last released.
+template <int N>
+struct Ring {
+    uint32_t slot = 0, round = 0;
+    __device__ __forceinline__ void next() {
+        if (++slot == N) {
+            slot = 0;
+            ++round;
+        }
+    }
+};
 
 __device__ __forceinline__ void mma_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
@@ -112,6 +161,30 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 columns without the wait, and the wait for all of them.
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// orders the loaded registers after the wait
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+// 32 bytes in one store: a whole sector per thread
+__device__ __forceinline__ void store32(void *p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 
 // 16 bytes global -> shared without a register round trip; src_bytes 0
@@ -170,14 +243,15 @@ struct TcSmem {
 };
 
 // Warp roles: warps 0-3 read the accumulators (each its 32 TMEM lanes) and
-// store the outputs; one thread of warp 4 issues the tensor copies and the
-// MMAs.  Barriers (all counts 1 except acc_empty, 4):
+// store the outputs; one thread of warp 4 issues the tensor copies, one of
+// warp 5 the MMAs.  Barriers (all counts 1 except acc_empty, 4):
 //   full[s]      stage s holds its job's rows (tensor-copy bytes)
 //   empty[s]     the MMAs that read stage s are done (tcgen05.commit)
 //   acc_full[a]  accumulator a holds a finished tile (tcgen05.commit)
 //   acc_empty[a] the four epilogue warps have read accumulator a
+constexpr int CONV_THREADS = 192;
 template <int COUT, int CHUNK, int NS>
-__global__ void __launch_bounds__(160, 1)
+__global__ void __launch_bounds__(CONV_THREADS, 1)
 conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_bfloat16 *__restrict__ w,
                   const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out, int out_cs, int out_co,
                   float *__restrict__ out32, int B, int H, int W, int relu, int *err) {
@@ -199,10 +273,7 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * NS, accf0 = empty0 + 8 * NS, acce0 = accf0 + 8 * NA;
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NS + 2 * NA);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
-    const int xt = (W + TC_M - 1) / TC_M;
-    const long long ntiles = (long long)B * H * xt;
-    const long long my_tiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const long long jobs = my_tiles * nch;
+    TileWalk walk(B, H, (W + TC_M - 1) / TC_M);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -224,7 +295,7 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
     }
     if (tid < COUT) sbias[tid] = bias ? bias[tid] : 0.f;
     // every weight of the layer, no swizzle: byte ((t * KGall + j) * COUT + co) * 16
-    for (int i = tid; i < 9 * KGall * COUT; i += 160) {
+    for (int i = tid; i < 9 * KGall * COUT; i += CONV_THREADS) {
         const int tc = i / KGall, j = i % KGall, t = tc / COUT, co = tc % COUT;
         cp_async16(b_base + (uint32_t)(((t * KGall + j) * COUT + co) * 16), w + (size_t)i * 8, 16);
     }
@@ -239,117 +310,136 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
 
     if (warp == 4) {
         if (lane == 0) {
-            constexpr uint32_t IDESC = idesc_bf16(TC_M, COUT);
-            // the CTA's job j: tile blockIdx.x + (j / nch) gridDim.x, chunk j % nch
-            auto load = [&](long long j) {
-                const long long tile = blockIdx.x + (j / nch) * gridDim.x;
-                const int xb = (int)(tile % xt);
-                const long long ny = tile / xt;
-                const uint32_t s = (uint32_t)(j % NS), fb = full0 + 8 * s;
-                mbar_expect_tx(fb, A_STAGE);
-                tma_load4(base + s * A_STAGE, &tin, (int)(j % nch) * CHUNK, xb * TC_M - 1, (int)(ny % H) - 1,
-                          (int)(ny / H), fb);
-            };
-            long long issued = 0, committed = 0;
-            for (; issued < jobs && issued < NS; ++issued) load(issued);
-            for (long long j = 0; j < jobs && ok; ++j) {
-                const long long k = j / nch;
-                const int c = (int)(j % nch), s = (int)(j % NS), a = (int)(k % NA);
-                if (!mbar_wait(full0 + 8 * s, (uint32_t)((j / NS) & 1), abort_flag)) ok = false;
-                // the epilogue of tile k - NA has read accumulator a
-                if (ok && c == 0 && k >= NA && !mbar_wait(acce0 + 8 * a, (uint32_t)((k / NA - 1) & 1), abort_flag))
-                    ok = false;
-                if (!ok || *abort_flag) {
-                    ok = false;
-                    break;
-                }
-                fence_after();
-                const uint64_t da = smem_desc_sw<ROWB>(base + (uint32_t)s * A_STAGE);
-                const uint64_t db = smem_desc(b_base + (uint32_t)(c * KG * COUT * 16), COUT * 16, 128);
-                const uint32_t d = tmem + (uint32_t)(a * COUT);
-#pragma unroll
-                for (int t = 0; t < 9; ++t) {
-#pragma unroll
-                    for (int q = 0; q < KG / 2; ++q)
-                        mma_bf16(d, da + (uint64_t)(((t / 3) * TC_BOX + t % 3) * ROWB / 16 + 2 * q),
-                                 db + (uint64_t)((t * KGall + 2 * q) * COUT), IDESC,
-                                 (c > 0 || t > 0 || q > 0) ? 1u : 0u);
-                }
-                mma_commit(empty0 + 8 * s);
-                if (c == nch - 1) mma_commit(accf0 + 8 * a);
-                committed = j + 1;
-                // refill the stage of job j - 1, whose MMAs were issued before
-                if (j >= 1 && issued < jobs) {
-                    const long long jr = j - 1;
-                    if (!mbar_wait(empty0 + 8 * (uint32_t)(jr % NS), (uint32_t)((jr / NS) & 1), abort_flag)) {
+            Ring<NS> st;
+            int issued = 0;
+            for (; walk.left > 0 && ok; walk.next()) {
+                for (int c = 0; c < nch; ++c) {
+                    const uint32_t s = st.slot, fb = full0 + 8 * s;
+                    if (st.round > 0 && !mbar_wait(empty0 + 8 * s, (st.round - 1) & 1, abort_flag)) {
                         ok = false;
                         break;
                     }
-                    load(issued++);
+                    mbar_expect_tx(fb, A_STAGE);
+                    tma_load4(base + s * A_STAGE, &tin, c * CHUNK, walk.xb * TC_M - 1, walk.y - 1, walk.n, fb);
+                    st.next();
+                    ++issued;
                 }
             }
             if (!ok) {
                 *abort_flag = 1;
                 atomicExch(err, 1);
-                // the tensor copies and MMAs in flight finish before the CTA
-                // leaves: the last use of each stage, and the last commit
-                // (MMAs complete in order)
-                for (long long j = issued > NS ? issued - NS : 0; j < issued; ++j)
+                // the copies in flight land before the CTA leaves: the last
+                // use of each stage
+                for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
                     mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
+            }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        if (lane == 0) {
+            constexpr uint32_t IDESC = idesc_bf16(TC_M, COUT);
+            Ring<NS> st;
+            Ring<NA> ac;
+            const uint32_t tap_step = (uint32_t)(KGall * COUT);
+            int committed = 0;
+            for (int k = walk.left; k > 0 && ok; --k, ac.next()) {
+                // the epilogue of tile k - NA has read the accumulator
+                if (ac.round > 0 && !mbar_wait(acce0 + 8 * ac.slot, (ac.round - 1) & 1, abort_flag)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t d = tmem + ac.slot * COUT;
+                for (int c = 0; c < nch; ++c) {
+                    const uint32_t s = st.slot;
+                    if (!mbar_wait(full0 + 8 * s, st.round & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    fence_after();
+                    const Desc da(smem_desc_sw<ROWB>(base + s * A_STAGE));
+                    const Desc db(smem_desc(b_base + (uint32_t)(c * KG * COUT * 16), COUT * 16, 128));
+                    uint32_t bt = 0;
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) {
+#pragma unroll
+                        for (int q = 0; q < KG / 2; ++q)
+                            mma_bf16(d, da, (uint32_t)(((t / 3) * TC_BOX + t % 3) * ROWB / 16 + 2 * q), db,
+                                     bt + (uint32_t)(2 * q * COUT), IDESC, (c > 0 || t > 0 || q > 0) ? 1u : 0u);
+                        bt += tap_step;
+                    }
+                    mma_commit(empty0 + 8 * s);
+                    st.next();
+                    ++committed;
+                }
+                if (ok) mma_commit(accf0 + 8 * ac.slot);
+            }
+            if (!ok) {
+                *abort_flag = 1;
+                atomicExch(err, 1);
+                // MMAs complete in order: the last commit covers them all
                 if (committed > 0)
                     mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1));
             }
         }
         __syncwarp();
     } else {
-        // epilogue warps: tile k from accumulator k % NA
-        for (long long k = 0; k < my_tiles; ++k) {
-            const int a = (int)(k % NA);
-            const bool got = mbar_wait(accf0 + 8 * a, (uint32_t)((k / NA) & 1), abort_flag);
+        // epilogue warps: tile k from accumulator k % NA, 32 columns at a time
+        constexpr int CW = COUT < 32 ? COUT : 32;
+        Ring<NA> ac;
+        for (; walk.left > 0; walk.next(), ac.next()) {
+            const uint32_t a = ac.slot;
+            const bool got = mbar_wait(accf0 + 8 * a, ac.round & 1, abort_flag);
             if (!__all_sync(0xffffffffu, got)) {
                 ok = false;
                 break;
             }
             fence_after();
-            const long long tile = blockIdx.x + k * gridDim.x;
-            const int xb = (int)(tile % xt);
-            const long long ny = tile / xt;
-            const int y = (int)(ny % H), n = (int)(ny / H);
-            const int x = xb * TC_M + warp * 32 + lane;  // TMEM lane = GEMM row = pixel
-            const size_t pix = ((size_t)n * H + y) * W + x;
-            const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(a * COUT);
+            const int x = walk.xb * TC_M + warp * 32 + lane;  // TMEM lane = GEMM row = pixel
+            const size_t pix = ((size_t)walk.n * H + walk.y) * W + x;
+            const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + a * COUT;
 #pragma unroll 1
-            for (int c = 0; c < COUT; c += 16) {
-                float v[16];
-                tmem_ld16(acc + (uint32_t)c, v);
+            for (int c = 0; c < COUT; c += CW) {
+                uint32_t r[CW / 16][16];
+#pragma unroll
+                for (int i = 0; i < CW / 16; ++i) tmem_ld16_async(acc + (uint32_t)(c + 16 * i), r[i]);
+#pragma unroll
+                for (int i = 0; i < CW / 16; ++i) tmem_wait(r[i]);
+                if (c + CW == COUT) {
+                    // every column is in registers: the accumulator is free
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acce0 + 8 * a);
+                }
                 if (x < W) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        v[i] += sbias[c + i];
-                        if (relu) v[i] = fmaxf(v[i], 0.f);
-                    }
-                    if (out) {
-                        uint32_t pk[8];
+                    for (int q = 0; q < CW / 16; ++q) {
+                        float v[16];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                            pk[i] = *(const uint32_t *)&h2;
+                        for (int i = 0; i < 16; ++i) {
+                            v[i] = __uint_as_float(r[q][i]) + sbias[c + 16 * q + i];
+                            if (relu) v[i] = fmaxf(v[i], 0.f);
                         }
-                        uint4 *o = (uint4 *)(out + pix * out_cs + out_co + c);
-                        o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                        o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-                    }
-                    if (out32) {
-                        float4 *o = (float4 *)(out32 + pix * COUT + c);
+                        if (out) {
+                            uint32_t pk[8];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                            for (int i = 0; i < 8; ++i) {
+                                const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                                pk[i] = *(const uint32_t *)&h2;
+                            }
+                            store32(out + pix * out_cs + out_co + c + 16 * q, pk);
+                        }
+                        if (out32) {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                uint32_t pk[8];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) pk[j] = __float_as_uint(v[8 * i + j]);
+                                store32(out32 + pix * COUT + c + 16 * q + 8 * i, pk);
+                            }
+                        }
                     }
                 }
             }
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acce0 + 8 * a);
         }
         if (!ok) {
             *abort_flag = 1;
@@ -390,8 +480,8 @@ __device__ __forceinline__ void red_add4(float *dst, float a, float b, float c, 
 // memory across all of a CTA's jobs and are added to dw at the end with
 // 16-byte vector reductions (dw, cin and NC keep every group of four columns
 // aligned); a layer wider than NC input channels is split over gridDim.y.
-// One thread issues the copies (NS stages) and the MMAs; every wait is
-// bounded.
+// One thread of warp 0 issues the copies (NS stages), one of warp 1 the MMAs;
+// every wait is bounded.
 template <int CO, int NC, int NS>
 struct WgSmem {
     static constexpr int ROWB_A = CO * 2, ROWB_B = NC * 2;
@@ -440,9 +530,10 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
     uint64_t *bars = (uint64_t *)(smem + NS * STAGE + SM::TAIL);
     const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * NS;
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NS);
-    const int xt = (W + TC_M - 1) / TC_M;
-    const long long units = (long long)B * H * xt;
-    const long long jobs = units > blockIdx.x ? (units - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+    TileWalk walk(B, H, (W + TC_M - 1) / TC_M);
+    const int jobs = walk.left;
+    __shared__ volatile int abort_flag;  // a wait gave up
+    __shared__ int status;               // 1: every MMA committed and complete
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -455,6 +546,8 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
             mbar_init(full0 + 8 * k, 1);
             mbar_init(empty0 + 8 * k, 1);
         }
+        abort_flag = 0;
+        status = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     fence_before();
@@ -463,62 +556,63 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
     const uint32_t tmem = *tmem_slot;
     // kind::f16, BF16 operands, FP32 accumulator, A and B MN-major
     constexpr uint32_t IDESC = idesc_bf16(TC_M, NC) | (1u << 15) | (1u << 16);
-    __shared__ int status;  // 1: every MMA committed and complete
 
     if (tid == 0) {
         bool ok = true;
-        auto load = [&](long long j) {
-            const long long unit = blockIdx.x + j * gridDim.x;
-            const int xb = (int)(unit % xt);
-            const long long ny = unit / xt;
-            const int y = (int)(ny % H), n = (int)(ny / H);
-            const uint32_t s = (uint32_t)(j % NS), fb = full0 + 8 * s, dst = base + s * STAGE;
+        Ring<NS> st;
+        int issued = 0;
+        for (; walk.left > 0; walk.next(), st.next()) {
+            const uint32_t s = st.slot, fb = full0 + 8 * s, dst = base + s * STAGE;
+            if (st.round > 0 && !mbar_wait(empty0 + 8 * s, (st.round - 1) & 1, &abort_flag)) {
+                ok = false;
+                break;
+            }
             mbar_expect_tx(fb, SM::A_ROWS + SM::B_STAGE);
-            tma_load4(dst, &tdp, 0, xb * TC_M, y - 1, n, fb);
-            tma_load4(dst + A_STAGE, &tin, ci0, xb * TC_M - 1, y, n, fb);
-        };
-        long long issued = 0, committed = 0;
-        for (; issued < jobs && issued < NS; ++issued) load(issued);
-        for (long long j = 0; j < jobs; ++j) {
-            const uint32_t s = (uint32_t)(j % NS);
-            if (!mbar_wait(full0 + 8 * s, (uint32_t)((j / NS) & 1))) {
+            tma_load4(dst, &tdp, 0, walk.xb * TC_M, walk.y - 1, walk.n, fb);
+            tma_load4(dst + A_STAGE, &tin, ci0, walk.xb * TC_M - 1, walk.y, walk.n, fb);
+            ++issued;
+        }
+        if (!ok) {
+            abort_flag = 1;
+            atomicExch(err, 1);
+            // the copies in flight land before the CTA leaves
+            for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
+                mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
+        }
+    } else if (tid == 32) {
+        bool ok = true;
+        Ring<NS> st;
+        int committed = 0;
+        for (int j = 0; j < jobs; ++j, st.next()) {
+            const uint32_t s = st.slot;
+            if (!mbar_wait(full0 + 8 * s, st.round & 1, &abort_flag)) {
                 ok = false;
                 break;
             }
             fence_after();
             const uint32_t a0 = base + s * STAGE;
-            const uint64_t da = smem_desc_sw_mn<ROWB_A>(a0, TC_M * ROWB_A);
-            const uint64_t db = smem_desc_sw_mn<ROWB_B>(a0 + A_STAGE, TC_BOX * ROWB_B);
+            const Desc da(smem_desc_sw_mn<ROWB_A>(a0, TC_M * ROWB_A));
+            const Desc db(smem_desc_sw_mn<ROWB_B>(a0 + A_STAGE, TC_BOX * ROWB_B));
 #pragma unroll
             for (int ks = 0; ks < TC_M / 16; ++ks) {
 #pragma unroll
                 for (int b = 0; b < MB; ++b) {
 #pragma unroll
                     for (int kx = 0; kx < 3; ++kx)
-                        mma_bf16(tmem + (uint32_t)((b * 3 + kx) * NC),
-                                 da + (uint64_t)((b * 128 * TC_M * 2 + 16 * ks * ROWB_A) / 16),
-                                 db + (uint64_t)((16 * ks + kx) * ROWB_B / 16), IDESC, (j > 0 || ks > 0) ? 1u : 0u);
+                        mma_bf16(tmem + (uint32_t)((b * 3 + kx) * NC), da,
+                                 (uint32_t)((b * 128 * TC_M * 2 + 16 * ks * ROWB_A) / 16), db,
+                                 (uint32_t)((16 * ks + kx) * ROWB_B / 16), IDESC, (j > 0 || ks > 0) ? 1u : 0u);
                 }
             }
             mma_commit(empty0 + 8 * s);
-            committed = j + 1;
-            if (j >= 1 && issued < jobs) {
-                const long long jr = j - 1;
-                if (!mbar_wait(empty0 + 8 * (uint32_t)(jr % NS), (uint32_t)((jr / NS) & 1))) {
-                    ok = false;
-                    break;
-                }
-                load(issued++);
-            }
+            ++committed;
         }
-        // the last commit covers every MMA (they complete in order); copies
-        // still in flight after a failure land before the CTA leaves
+        // the last commit covers every MMA (they complete in order)
         if (committed > 0 &&
             !mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1)))
             ok = false;
         if (!ok) {
-            for (long long j = issued > NS ? issued - NS : 0; j < issued; ++j)
-                mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
+            abort_flag = 1;
             atomicExch(err, 1);
         }
         status = ok && committed == jobs ? 1 : 0;
