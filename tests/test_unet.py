@@ -190,3 +190,35 @@ def test_gpu_tcgen05_ragged_rows_match_mma_sync(monkeypatch):
         a, b = g1[s].astype(np.float64), g0[s].astype(np.float64)
         nb = np.linalg.norm(b)
         assert nb > 0 and np.linalg.norm(a - b) <= 3e-2 * nb, (k, np.linalg.norm(a - b) / nb)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,W,levels,base", [(1, 8, 8, 3, 16), (2, 16, 136, 3, 32), (5, 48, 272, 4, 16),
+                                               (1, 32, 32, 5, 32), (7, 24, 520, 3, 16)])
+def test_gpu_tcgen05_row_runs_match_mma_sync(monkeypatch, B, H, W, levels, base):
+    """Shapes around the row-ring convolutions' runs: images of one row or one
+    tile, fewer tiles than CTAs, runs that cross column segments and images
+    after a few rows, rows that end inside a warp's 32 pixels; with the masked
+    data gradients (16, 32 and 64 channels) and their bias sums.  Predictions
+    and every layer's parameter gradient agree with the mma.sync kernels to
+    the BF16 tolerance of the tests above."""
+    from thesis_gb300.warmstart import UNet
+    ic, oc = 4, 3
+    x, t, w = _problem(B, H, W, ic, oc, 31)
+    p = uo.init_params(ic, oc, 37, levels, base)
+    res = {}
+    for tc in ("1", "0"):
+        monkeypatch.setenv("THESIS_UNET_TC", tc)
+        with UNet(H, W, max_batch=B + 1, in_channels=ic, out_channels=oc, levels=levels, base_channels=base) as net:
+            net.set_params(p)
+            net.set_dataset(x, t, w)
+            net.gradients(list(range(B)))
+            g, loss = net.gradients(list(range(B)))
+            res[tc] = (net.predict(x), g, loss)
+    (p1, g1, l1), (p0, g0, l0) = res["1"], res["0"]
+    assert np.abs(p1 - p0).max() < 2e-2 * np.abs(p0).max() and abs(l1 - l0) <= 1e-3 * l0
+    for k, s in enumerate(_layer_slices(levels, base)):
+        a, b = g1[s].astype(np.float64), g0[s].astype(np.float64)
+        nb = np.linalg.norm(b)
+        if nb > 0:
+            assert np.linalg.norm(a - b) <= 3e-2 * nb, (k, np.linalg.norm(a - b) / nb)

@@ -250,30 +250,6 @@ __device__ __forceinline__ void st8(bf16 *p, const V8 &a) {
     *(uint4 *)p = r;
 }
 
-// db[co] += sum_p dpre[p][co]: thread t sums channel group t % G of pixels
-// t / G, t / G + 256 / G, ...; the block adds its partial sums per channel
-__global__ void __launch_bounds__(256) bias_grad_kernel(const bf16 *__restrict__ dpre, int cout, int npix,
-                                                        float *__restrict__ db) {
-    __shared__ float part[256][9];
-    const int G = cout / 8, t = threadIdx.x, v = t % G, sets = 256 / G;
-    V8 s;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) s.v[k] = 0.f;
-    for (int p = blockIdx.x * sets + t / G; p < npix; p += gridDim.x * sets) {
-        const V8 a = ld8(dpre + (size_t)p * cout + 8 * v);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) s.v[k] += a.v[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) part[t][k] = s.v[k];
-    __syncthreads();
-    if (t < cout) {
-        float a = 0.f;
-        for (int q = t / 8; q < 256; q += G) a += part[q][t % 8];
-        atomicAdd(db + t, a);
-    }
-}
-
 // 2x2 average pooling: out[n, y, x, c] = mean of in[n, 2y+i, 2x+j, c]
 __global__ void pool_kernel(const bf16 *in, int in_cs, int in_co, bf16 *out, int C, int B, int Ho, int Wo) {
     const int G = C / 8, total = B * Ho * Wo * G;
@@ -301,9 +277,62 @@ __global__ void up_kernel(const bf16 *in, int C, bf16 *out, int out_cs, int out_
     }
 }
 
+// Channel sums of the pre-activation gradients that a kernel writes, for the
+// bias gradient: a thread's channel group is the same in every round of its
+// grid-stride loop (256 threads and any grid are whole numbers of pixels), so
+// it adds up what it stores; the block's sums go to its own row of `part`,
+// which bias_final_kernel adds up.  (Adding them to the gradient with atomics
+// serialised at the one or two lines that hold it: 40 us for 600 warps.)
+struct BiasSum {
+    float s[8];
+    __device__ __forceinline__ BiasSum() {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] = 0.f;
+    }
+    __device__ __forceinline__ void add(const V8 &o) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] += __bfloat162float(__float2bfloat16(o.v[k]));
+    }
+    __device__ __forceinline__ void flush(int C, float *rows) {
+        __shared__ float part[256][9];
+        const int t = threadIdx.x, G = C / 8;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) part[t][k] = s[k];
+        __syncthreads();
+        if (t < C) {
+            float a = 0.f;
+            for (int q = t / 8; q < 256; q += G) a += part[q][t % 8];
+            rows[(size_t)blockIdx.x * unet_tc::BIAS_STRIDE + t] = a;
+        }
+    }
+};
+
+// Bias gradients: block k sums layer k's partial rows, in a fixed order.
+constexpr int MAX_LAYERS = 23;
+struct BiasPlan {
+    int rows[MAX_LAYERS], C[MAX_LAYERS];
+    long long off[MAX_LAYERS];
+};
+__global__ void __launch_bounds__(1024) bias_final_kernel(const __grid_constant__ BiasPlan plan, const float *part,
+                                                          float *grad) {
+    __shared__ float sh[1024];
+    const int k = blockIdx.x, C = plan.C[k], t = threadIdx.x, sets = 1024 / C;
+    const float *p = part + (size_t)k * unet_tc::BIAS_ROWS * unet_tc::BIAS_STRIDE;
+    float a = 0.f;
+#pragma unroll 8
+    for (int r = t / C; r < plan.rows[k]; r += sets) a += p[(size_t)r * unet_tc::BIAS_STRIDE + t % C];
+    sh[t] = a;
+    __syncthreads();
+    if (t < C) {
+        for (int q = 1; q < sets; ++q) a += sh[q * C + t];
+        grad[plan.off[k] + t] = a;
+    }
+}
+
 // dpre[p][c] = g[p][c] * (act[p][c] > 0)
-__global__ void relu_bwd_kernel(const bf16 *g, int g_cs, int g_co, const bf16 *act, int a_cs, int a_co, bf16 *dpre,
-                                int C, int npix) {
+__global__ void __launch_bounds__(256) relu_bwd_kernel(const bf16 *g, int g_cs, int g_co, const bf16 *act, int a_cs,
+                                                       int a_co, bf16 *dpre, int C, int npix, float *rows) {
+    BiasSum bs;
     const int G = C / 8, total = npix * G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int v = i % G, p = i / G;
@@ -312,12 +341,16 @@ __global__ void relu_bwd_kernel(const bf16 *g, int g_cs, int g_co, const bf16 *a
 #pragma unroll
         for (int k = 0; k < 8; ++k) o.v[k] = a.v[k] > 0.f ? o.v[k] : 0.f;
         st8(dpre + (size_t)i * 8, o);
+        bs.add(o);
     }
+    bs.flush(C, rows);
 }
 
 // dpre = (pool gradient + skip gradient) masked by ReLU, at full resolution
-__global__ void pool_skip_bwd_kernel(const bf16 *gpool, const bf16 *gskip, int s_cs, int s_co, const bf16 *act,
-                                     int a_cs, int a_co, bf16 *dpre, int C, int B, int H, int W) {
+__global__ void __launch_bounds__(256) pool_skip_bwd_kernel(const bf16 *gpool, const bf16 *gskip, int s_cs, int s_co,
+                                                            const bf16 *act, int a_cs, int a_co, bf16 *dpre, int C,
+                                                            int B, int H, int W, float *rows) {
+    BiasSum bs;
     const int G = C / 8, total = B * H * W * G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int v = i % G, p = i / G, x = p % W, ny = p / W, y = ny % H, n = ny / H;
@@ -328,12 +361,15 @@ __global__ void pool_skip_bwd_kernel(const bf16 *gpool, const bf16 *gskip, int s
 #pragma unroll
         for (int k = 0; k < 8; ++k) o.v[k] = a.v[k] > 0.f ? 0.25f * gp.v[k] + gs.v[k] : 0.f;
         st8(dpre + (size_t)i * 8, o);
+        bs.add(o);
     }
+    bs.flush(C, rows);
 }
 
 // dpre at low resolution = sum of the 2x2 upsampled gradient, masked by ReLU
-__global__ void up_bwd_kernel(const bf16 *gup, int g_cs, int g_co, const bf16 *act, bf16 *dpre, int C, int B, int H,
-                              int W) {
+__global__ void __launch_bounds__(256) up_bwd_kernel(const bf16 *gup, int g_cs, int g_co, const bf16 *act, bf16 *dpre,
+                                                     int C, int B, int H, int W, float *rows) {
+    BiasSum bs;
     const int G = C / 8, total = B * H * W * G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int v = i % G, p = i / G, x = p % W, ny = p / W, y = ny % H, n = ny / H;
@@ -346,12 +382,16 @@ __global__ void up_bwd_kernel(const bf16 *gup, int g_cs, int g_co, const bf16 *a
 #pragma unroll
         for (int k = 0; k < 8; ++k) o.v[k] = m.v[k] > 0.f ? a.v[k] + c.v[k] + d.v[k] + e.v[k] : 0.f;
         st8(dpre + (size_t)i * 8, o);
+        bs.add(o);
     }
+    bs.flush(C, rows);
 }
 
-// loss sums: sums[0] += sum_p w_p sum_{c<oc} (y - t)^2, sums[1] += sum_p w_p
-__global__ void loss_kernel(const float *pred, int pc, const float *tgt, int oc, const float *wt, long long npix,
-                            double *sums) {
+// loss sums: sums[0] += sum_p w_p sum_{c<oc} (y - t)^2, sums[1] += sum_p w_p;
+// one pair of atomics per block (two per warp took 120 us of a 150 us launch)
+__global__ void __launch_bounds__(256) loss_kernel(const float *pred, int pc, const float *tgt, int oc, const float *wt,
+                                                   long long npix, double *sums) {
+    __shared__ double sh[2][8];
     double a = 0, b = 0;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += (long long)gridDim.x * blockDim.x) {
         const float wp = wt[p];
@@ -368,14 +408,22 @@ __global__ void loss_kernel(const float *pred, int pc, const float *tgt, int oc,
         b += __shfl_down_sync(0xffffffffu, b, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(sums, a);
-        atomicAdd(sums + 1, b);
+        sh[0][threadIdx.x >> 5] = a;
+        sh[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double s = 0;
+        for (int k = 0; k < 8; ++k) s += sh[threadIdx.x][k];
+        atomicAdd(sums + threadIdx.x, s);
     }
 }
 
 // output gradient of the weighted MSE, BF16, pc channels (the unused ones 0)
-__global__ void loss_grad_kernel(const float *pred, int pc, const float *tgt, int oc, const float *wt,
-                                 int npix, const double *sums, bf16 *dout) {
+__global__ void __launch_bounds__(256) loss_grad_kernel(const float *pred, int pc, const float *tgt, int oc,
+                                                        const float *wt, int npix, const double *sums, bf16 *dout,
+                                                        float *rows) {
+    BiasSum bs;
     const float norm = sums[1] > 0 ? (float)(2.0 / (oc * sums[1])) : 0.f;
     const int G = pc / 8, total = npix * G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -388,7 +436,9 @@ __global__ void loss_grad_kernel(const float *pred, int pc, const float *tgt, in
             o.v[k] = c < oc ? wp * (pred[(size_t)i * 8 + k] - tgt[(size_t)p * oc + c]) : 0.f;
         }
         st8(dout + (size_t)i * 8, o);
+        bs.add(o);
     }
+    bs.flush(pc, rows);
 }
 
 __global__ void adam_kernel(float *p, const float *g, float *m, float *v, long long n, float lr, float c1, float c2) {
@@ -430,6 +480,12 @@ __global__ void unpack_output_kernel(const float *in, int pc, float *out, int oc
         out[i] = in[(i / oc) * pc + i % oc];
 }
 
+// blocks of an elementwise kernel that leaves a row of channel sums per block
+int sum_grid_for(long long n) {
+    const long long b = (n + 255) / 256;
+    return (int)std::max(1ll, std::min<long long>(b, unet_tc::BIAS_ROWS));
+}
+
 int grid_for(long long n, int block = 256) {
     long long b = (n + block - 1) / block;
     return (int)(b < 4096 ? (b > 0 ? b : 1) : 4096);
@@ -461,6 +517,7 @@ struct lbm_unet_s {
     // tensor-core configuration per layer shape (+-(cout * 4096 + cin) for
     // convolutions / weight gradients): instance index and CTAs per SM
     std::map<int, std::pair<int, int>> tc_choice;
+    std::map<int, std::pair<int, int>> rows_choice;  // row-ring convolutions: slots (0: none) and CTAs per SM
     int *tc_err = nullptr;     // set by a tensor-core kernel whose bounded wait gave up
     cudaStream_t stream = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -478,7 +535,8 @@ struct lbm_unet_s {
     std::vector<Act> e_a, cat, p, d_a, d_b, g_e_a, g_cat, g_p, g_d_a, g_d_b;
     float *out32 = nullptr;     // [B][H][W][16] FP32 output
     bf16 *dout = nullptr;       // its gradient
-    bf16 *dpre = nullptr;       // scratch: a layer's pre-activation gradient
+    float *bias_part = nullptr;  // [layer][BIAS_ROWS][BIAS_STRIDE] partial bias gradients
+    bf16 *dpre[2] = {nullptr, nullptr};  // pre-activation gradients of the layer at hand and of the one below
     float *fin = nullptr, *fout = nullptr;  // host-format staging
     float *tgt = nullptr, *wt = nullptr;    // batch targets and weights
     double *sums = nullptr;
@@ -576,12 +634,103 @@ bool nhwc_tensor_map(CUtensorMap *m, const bf16 *p, int C, int cs, int H, int W,
 }
 
 // the convolution's input rows: chunk channels x TC_BOX pixels x 3 rows
-bool act_tensor_map(CUtensorMap *m, const Act &a, int cin, int chunk, int H, int W, int B) {
-    return nhwc_tensor_map(m, a.p + a.co, cin, a.cs, H, W, B, chunk, unet_tc::TC_BOX, 3);
+bool act_tensor_map(CUtensorMap *m, const Act &a, int cin, int chunk, int H, int W, int B, int rows = 3) {
+    return nhwc_tensor_map(m, a.p + a.co, cin, a.cs, H, W, B, chunk, unet_tc::TC_BOX, rows);
 }
 
-void conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const float *bias, float *out32, int B,
-          int level, bool transposed) {
+// The row-ring convolution of a layer shape: ring slots and CTAs per SM, or
+// false where the weights and four rows do not fit an SM (cin 128 with cout
+// 64).  More CTAs hide an issuing thread's latency, more slots the copies':
+// CTAs x rows in flight beyond the three being read (at most four count).
+struct RowsChoice {
+    int nr = 0, occ = 0;
+};
+template <int COUT, int CHUNK, bool MASK>
+RowsChoice rows_choice(const lbm_unet_s *u, int cin) {
+    using SM = unet_tc::RowSmem<COUT, CHUNK>;
+    auto kern = unet_tc::conv3x3_rows_kernel<COUT, CHUNK, MASK>;
+    const int room = u->smem_optin - (MASK ? 1024 : 0);  // the masked form's own sums
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    const int regs = resident_by_registers((const void *)kern, unet_tc::CONV_THREADS);
+    RowsChoice best;
+    int best_score = 0;
+    for (int nr = unet_tc::ROW_MAX; nr >= 4; --nr) {
+        const size_t bytes = SM::bytes(cin, nr);
+        if (bytes > (size_t)room) continue;
+        const int occ = std::min(
+            std::min((int)(u->smem_per_sm / (bytes + (MASK ? 2048 : 1024))), 512 / std::max(32, SM::NA * COUT)), regs);
+        const int score = occ * std::min(nr - 3, 4) * 16 + occ;
+        if (occ >= 1 && score > best_score) {
+            best_score = score;
+            best.nr = nr;
+            best.occ = occ;
+        }
+    }
+    return best;
+}
+
+// A data gradient's mask: the activation whose ReLU it passes, and where the
+// channel sums of the masked gradient (a bias gradient's partial rows) go.
+struct ReluMask {
+    const Act *act;
+    float *rows;  // per CTA
+    int *nrows;
+};
+template <int COUT, int CHUNK, bool MASK>
+bool rows_run(lbm_unet_s *u, int cin, const CUtensorMap &map, const RowsChoice &c, const bf16 *w, const float *bias,
+              bf16 *op, const Act &out, float *out32, const ReluMask *mask, int B, int H, int W, int relu) {
+    const long long tiles = (long long)B * H * ((W + unet_tc::TC_M - 1) / unet_tc::TC_M);
+    const long long g = std::min(std::min((long long)u->sms * c.occ, tiles), (long long)unet_tc::BIAS_ROWS);
+    auto kern = unet_tc::conv3x3_rows_kernel<COUT, CHUNK, MASK>;
+    // outputs staged in shared memory leave by tensor copies of 32 pixels
+    CUtensorMap tout = map;
+    if (unet_tc::RowSmem<COUT, CHUNK>::STAGED &&
+        (!op || !nhwc_tensor_map(&tout, op + out.co, COUT, out.cs, H, W, B, COUT, 32, 1)))
+        return false;
+    kern<<<(unsigned)g, unet_tc::CONV_THREADS, unet_tc::RowSmem<COUT, CHUNK>::bytes(cin, c.nr), u->stream>>>(
+        map, tout, cin, c.nr, w, bias, op, out.cs, out.co, out32, mask ? mask->act->p + mask->act->co : nullptr,
+        mask ? mask->act->cs : 0, mask ? mask->rows : nullptr, B, H, W, relu, u->tc_err);
+    if (mask) *mask->nrows = (int)g;
+    return true;
+}
+
+#define ROWS_LIST(X)                                                                                      \
+    X(16, 16) X(16, 32) X(16, 64) X(32, 16) X(32, 32) X(32, 64) X(64, 16) X(64, 32) X(64, 64) X(128, 16)  \
+    X(128, 32)
+// data gradients through a ReLU: outputs of 16, 32 and 64 channels
+#define ROWS_MASK_LIST(X) X(16, 16) X(16, 32) X(16, 64) X(32, 16) X(32, 32) X(32, 64) X(64, 16) X(64, 32) X(64, 64)
+RowsChoice rows_choice_of(const lbm_unet_s *u, int cout, int chunk, int cin, bool mask) {
+#define ROWS_CHOICE(CO, CH) \
+    if (!mask && cout == CO && chunk == CH) return rows_choice<CO, CH, false>(u, cin);
+#define ROWS_MASK_CHOICE(CO, CH) \
+    if (mask && cout == CO && chunk == CH) return rows_choice<CO, CH, true>(u, cin);
+    ROWS_LIST(ROWS_CHOICE)
+    ROWS_MASK_LIST(ROWS_MASK_CHOICE)
+#undef ROWS_CHOICE
+#undef ROWS_MASK_CHOICE
+    return RowsChoice();
+}
+bool rows_run_of(lbm_unet_s *u, int cout, int chunk, int cin, const CUtensorMap &map, const RowsChoice &c, const bf16 *w,
+                 const float *bias, bf16 *op, const Act &out, float *out32, const ReluMask *mask, int B, int H, int W,
+                 int relu) {
+#define ROWS_RUN(CO, CH)                 \
+    if (!mask && cout == CO && chunk == CH) \
+        return rows_run<CO, CH, false>(u, cin, map, c, w, bias, op, out, out32, mask, B, H, W, relu);
+#define ROWS_MASK_RUN(CO, CH)           \
+    if (mask && cout == CO && chunk == CH) \
+        return rows_run<CO, CH, true>(u, cin, map, c, w, bias, op, out, out32, mask, B, H, W, relu);
+    ROWS_LIST(ROWS_RUN)
+    ROWS_MASK_LIST(ROWS_MASK_RUN)
+#undef ROWS_RUN
+#undef ROWS_MASK_RUN
+    return false;
+}
+
+// With `mask` (data gradients) the output is the masked gradient where a
+// kernel does that itself: the result then is true, and `out` holds it.
+bool conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const float *bias, float *out32, int B,
+          int level, bool transposed, const ReluMask *mask = nullptr) {
     const int H = H_of(u, level), W = W_of(u, level);
     dim3 grid((W + TILE_X - 1) / TILE_X, H, B);
     const bf16 *w = transposed ? l.wt : l.w;
@@ -664,10 +813,24 @@ void conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const fl
     }
             TC_LIST(TC_CHUNK)
             CUtensorMap map;
+            for (const ReluMask *m : {mask, (const ReluMask *)nullptr}) {
+                const int rkey = m ? -key : key;
+                if (!u->rows_choice.count(rkey)) {
+                    const RowsChoice rc = rows_choice_of(u, cout, chunk, cin, m != nullptr);
+                    u->rows_choice[rkey] = std::make_pair(rc.nr, rc.occ);
+                }
+                RowsChoice rc;
+                rc.nr = u->rows_choice[rkey].first;
+                rc.occ = u->rows_choice[rkey].second;
+                if (rc.nr && act_tensor_map(&map, in, cin, chunk, H, W, B, 1) &&
+                    rows_run_of(u, cout, chunk, cin, map, rc, w, bias, op, out, out32, m, B, H, W, relu))
+                    return m != nullptr;
+                if (!mask) break;
+            }
             if (act_tensor_map(&map, in, cin, chunk, H, W, B)) {
                 idx = 0;
                 TC_LIST(TC_RUN)
-                return;
+                return false;
             }
             fprintf(stderr, "thesis_unet: tensor map encoding failed; convolutions fall back to mma.sync\n");
             u->tc = false;
@@ -684,16 +847,17 @@ void conv(lbm_unet_s *u, const Layer &l, const Act &in, const Act &out, const fl
     case 128: conv3x3_kernel<128><<<grid, 128, 0, u->stream>>>(in.p, in.cs, in.co, cin, w, bias, op, out.cs, out.co, out32, H, W, relu); break;
     default: ufail(LBM_ERR_INVALID, "no convolution kernel for this width"); break;
     }
+    return false;
 }
 
 // persistent tensor-core weight gradient (unet_tc.cuh); false when the
 // layer's shape has no instance
-bool wgrad_tc(lbm_unet_s *u, const Layer &l, const Act &in, int B, int H, int W, float *dw) {
+bool wgrad_tc(lbm_unet_s *u, const Layer &l, const Act &in, const bf16 *dpre, int B, int H, int W, float *dw) {
     const int nc = l.cin < 64 ? l.cin : 64;
     if (l.cin % nc) return false;
     const long long units = (long long)B * H * ((W + unet_tc::TC_M - 1) / unet_tc::TC_M);
     CUtensorMap tdp, tin;
-    if (!nhwc_tensor_map(&tdp, u->dpre, l.cout, l.cout, H, W, B, l.cout, unet_tc::TC_M, 3) ||
+    if (!nhwc_tensor_map(&tdp, dpre, l.cout, l.cout, H, W, B, l.cout, unet_tc::TC_M, 3) ||
         !nhwc_tensor_map(&tin, in.p + in.co, l.cin, in.cs, H, W, B, nc, unet_tc::TC_BOX, 1)) {
         fprintf(stderr, "thesis_unet: tensor map encoding failed; weight gradients fall back to mma.sync\n");
         u->tc = false;
@@ -762,27 +926,21 @@ bool wgrad_tc(lbm_unet_s *u, const Layer &l, const Act &in, int B, int H, int W,
     return true;
 }
 
-void wgrad(lbm_unet_s *u, const Layer &l, const Act &in, int B, int level) {
+// the weight gradient; the kernel that made dpre has added the bias gradient
+void wgrad(lbm_unet_s *u, const Layer &l, const Act &in, const bf16 *dpre, int B, int level) {
     const int H = H_of(u, level), W = W_of(u, level);
     const long long rows = (long long)B * H * ((W + TILE_X - 1) / TILE_X);
     dim3 grid((unsigned)(rows < 64 ? rows : 64), 9);
     float *dw = u->grad + l.w_off;
-    const long long npix = (long long)B * H * W;
-    if (u->tc && l.cin % 16 == 0 && wgrad_tc(u, l, in, B, H, W, dw)) {
-        bias_grad_kernel<<<grid_for(npix * (l.cout / 8), 256), 256, 0, u->stream>>>(u->dpre, l.cout, (int)npix,
-                                                                                 u->grad + l.b_off);
-        return;
-    }
+    if (u->tc && l.cin % 16 == 0 && wgrad_tc(u, l, in, dpre, B, H, W, dw)) return;
 #define WG(CO, CI)                                                                                            \
     if (l.cout == CO && l.cin == CI) {                                                                        \
-        wgrad_kernel<CO, CI><<<grid, 128, 0, u->stream>>>(u->dpre, in.p, in.cs, in.co, dw, B, H, W);         \
+        wgrad_kernel<CO, CI><<<grid, 128, 0, u->stream>>>(dpre, in.p, in.cs, in.co, dw, B, H, W);            \
     } else
     WG(16, 16) WG(32, 16) WG(32, 32) WG(64, 32) WG(64, 64) WG(64, 128) WG(32, 64) WG(16, 32) {
         ufail(LBM_ERR_INVALID, "no weight-gradient kernel for this layer shape");
     }
 #undef WG
-    bias_grad_kernel<<<grid_for(npix * (l.cout / 8), 256), 256, 0, u->stream>>>(u->dpre, l.cout, (int)npix,
-                                                                                 u->grad + l.b_off);
 }
 
 void refresh_weights(lbm_unet_s *u) {
@@ -824,76 +982,102 @@ void forward(lbm_unet_s *u, int B) {
     cv(out_layer(u), u->d_b[0], none, 0, u->out32);
 }
 
-// backward pass from dout; parameter gradients accumulate into grad
+// Backward pass from dout; parameter gradients accumulate into grad.  cur is
+// the pre-activation gradient of the layer at hand; the one of the layer below
+// goes to the other of the two dpre buffers, from the data gradient's own
+// kernel where the layer below ends in a ReLU and nothing else (dgrad_relu),
+// else from the elementwise kernel that joins its gradients.
 void backward(lbm_unet_s *u, int B) {
     auto &L = u->L;
     const int NL = u->levels;
     auto npix = [&](int lev) { return (long long)B * H_of(u, lev) * W_of(u, lev); };
-    auto dgrad = [&](int k, const Act &gin, int lev) {
+    const bf16 *cur = u->dout;
+    auto other = [&]() { return cur == u->dpre[0] ? u->dpre[1] : u->dpre[0]; };
+    auto view_of = [&](const bf16 *p, int C) {
         Act d;
-        d.p = u->dpre;
-        d.cs = L[k].cout;
-        d.co = 0;
-        d.C = L[k].cout;
-        conv(u, L[k], d, gin, nullptr, nullptr, B, lev, true);
+        d.p = const_cast<bf16 *>(p);
+        d.cs = d.C = C;
+        return d;
     };
-    auto relu_bwd = [&](const Act &g, const Act &act, int C, int lev) {
-        const long long n = npix(lev) * C;
-        relu_bwd_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(g.p, g.cs, g.co, act.p, act.cs, act.co, u->dpre, C,
-                                                                  (int)npix(lev));
+    // layer k's partial rows of its bias gradient, and how many there are
+    auto rows = [&](int k) { return u->bias_part + (size_t)k * unet_tc::BIAS_ROWS * unet_tc::BIAS_STRIDE; };
+    BiasPlan plan;
+    for (int k = 0; k < (int)L.size(); ++k) {
+        plan.C[k] = L[k].cout;
+        plan.off[k] = (long long)L[k].b_off;
+    }
+    plan.rows[out_layer(u)] = sum_grid_for(npix(0) * 2);  // loss_grad_kernel's
+    auto wg = [&](int k, const Act &in, int lev) { wgrad(u, L[k], in, cur, B, lev); };
+    auto dgrad = [&](int k, const Act &gin, int lev) {
+        conv(u, L[k], view_of(cur, L[k].cout), gin, nullptr, nullptr, B, lev, true);
     };
-    auto pool_skip = [&](const Act &gpool, const Act &gskip, const Act &act, int C, int lev) {
-        const long long n = npix(lev) * C;
-        pool_skip_bwd_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(gpool.p, gskip.p, gskip.cs, gskip.co, act.p,
-                                                                   act.cs, act.co, u->dpre, C, B, H_of(u, lev),
-                                                                   W_of(u, lev));
+    // data gradient of layer k through the ReLU of layer below (its
+    // activation act); g is the gradient's own buffer for the two-kernel form
+    auto dgrad_relu = [&](int k, int below, const Act &g, const Act &act, int lev) {
+        const int C = L[k].cin;
+        bf16 *next = other();
+        const ReluMask mask{&act, rows(below), &plan.rows[below]};
+        const Act fused = view_of(next, C), in = view_of(cur, L[k].cout);
+        if (!conv(u, L[k], in, fused, nullptr, nullptr, B, lev, true, &mask)) {
+            // the convolution left the unmasked gradient in `next`
+            cudaMemcpyAsync(g.p, next, sizeof(bf16) * npix(lev) * C, cudaMemcpyDeviceToDevice, u->stream);
+            const int grid = plan.rows[below] = sum_grid_for(npix(lev) * C / 8);
+            relu_bwd_kernel<<<grid, 256, 0, u->stream>>>(g.p, C, 0, act.p, act.cs, act.co, next, C, (int)npix(lev),
+                                                         rows(below));
+        }
+        cur = next;
     };
-    auto up_bwd = [&](const Act &gup, const Act &act, int C, int lev) {
-        const long long n = npix(lev) * C;
-        up_bwd_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(gup.p, gup.cs, gup.co, act.p, u->dpre, C, B, H_of(u, lev),
-                                                            W_of(u, lev));
+    auto pool_skip = [&](int k, const Act &gpool, const Act &gskip, const Act &act, int C, int lev) {
+        bf16 *next = other();
+        const int grid = plan.rows[k] = sum_grid_for(npix(lev) * C / 8);
+        pool_skip_bwd_kernel<<<grid, 256, 0, u->stream>>>(gpool.p, gskip.p, gskip.cs, gskip.co, act.p, act.cs, act.co, next,
+                                                          C, B, H_of(u, lev), W_of(u, lev), rows(k));
+        cur = next;
     };
-    // output layer: dpre = dout
-    cudaMemcpyAsync(u->dpre, u->dout, sizeof(bf16) * npix(0) * 16, cudaMemcpyDeviceToDevice, u->stream);
-    wgrad(u, L[out_layer(u)], u->d_b[0], B, 0);
-    dgrad(out_layer(u), u->g_d_b[0], 0);
-    // decoder, from level 0 up
+    auto up_bwd = [&](int k, const Act &gup, const Act &act, int C, int lev) {
+        bf16 *next = other();
+        const int grid = plan.rows[k] = sum_grid_for(npix(lev) * C / 8);
+        up_bwd_kernel<<<grid, 256, 0, u->stream>>>(gup.p, gup.cs, gup.co, act.p, next, C, B, H_of(u, lev), W_of(u, lev),
+                                                   rows(k));
+        cur = next;
+    };
+    wg(out_layer(u), u->d_b[0], 0);
+    dgrad_relu(out_layer(u), dec_b(u, 0), u->g_d_b[0], u->d_b[0], 0);
+    // decoder, from level 0 up; d_b[l] was upsampled into the first channels of cat[l-1]
     for (int l = 0; l < NL; ++l) {
-        if (l == 0)
-            relu_bwd(u->g_d_b[0], u->d_b[0], ch_dec_b(u, 0), 0);
-        else  // d_b[l] was upsampled into the first channels of cat[l-1]
-            up_bwd(view(u->g_cat[l - 1], 0, ch_dec_b(u, l)), u->d_b[l], ch_dec_b(u, l), l);
-        wgrad(u, L[dec_b(u, l)], u->d_a[l], B, l);
-        dgrad(dec_b(u, l), u->g_d_a[l], l);
-        relu_bwd(u->g_d_a[l], u->d_a[l], ch(u, l), l);
-        wgrad(u, L[dec_a(u, l)], u->cat[l], B, l);
+        if (l > 0) up_bwd(dec_b(u, l), view(u->g_cat[l - 1], 0, ch_dec_b(u, l)), u->d_b[l], ch_dec_b(u, l), l);
+        wg(dec_b(u, l), u->d_a[l], l);
+        dgrad_relu(dec_b(u, l), dec_a(u, l), u->g_d_a[l], u->d_a[l], l);
+        wg(dec_a(u, l), u->cat[l], l);
         dgrad(dec_a(u, l), u->g_cat[l], l);
     }
     // bottleneck
-    up_bwd(view(u->g_cat[NL - 1], 0, ch(u, NL)), u->bb, ch(u, NL), NL);
-    wgrad(u, L[bott_b(u)], u->ba, B, NL);
-    dgrad(bott_b(u), u->g_ba, NL);
-    relu_bwd(u->g_ba, u->ba, ch(u, NL), NL);
-    wgrad(u, L[bott_a(u)], u->p[NL - 1], B, NL);
+    up_bwd(bott_b(u), view(u->g_cat[NL - 1], 0, ch(u, NL)), u->bb, ch(u, NL), NL);
+    wg(bott_b(u), u->ba, NL);
+    dgrad_relu(bott_b(u), bott_a(u), u->g_ba, u->ba, NL);
+    wg(bott_a(u), u->p[NL - 1], NL);
     dgrad(bott_a(u), u->g_p[NL - 1], NL);
     // encoder, from the deepest level down
     for (int l = NL - 1; l >= 0; --l) {
-        pool_skip(u->g_p[l], view(u->g_cat[l], ch_up(u, l), ch(u, l)), view(u->cat[l], ch_up(u, l), ch(u, l)), ch(u, l), l);
-        wgrad(u, L[enc_b(l)], u->e_a[l], B, l);
-        dgrad(enc_b(l), u->g_e_a[l], l);
-        relu_bwd(u->g_e_a[l], u->e_a[l], ch(u, l), l);
-        wgrad(u, L[enc_a(l)], l == 0 ? u->x0 : u->p[l - 1], B, l);
+        pool_skip(enc_b(l), u->g_p[l], view(u->g_cat[l], ch_up(u, l), ch(u, l)), view(u->cat[l], ch_up(u, l), ch(u, l)),
+                  ch(u, l), l);
+        wg(enc_b(l), u->e_a[l], l);
+        dgrad_relu(enc_b(l), enc_a(l), u->g_e_a[l], u->e_a[l], l);
+        wg(enc_a(l), l == 0 ? u->x0 : u->p[l - 1], l);
         if (l > 0) dgrad(enc_a(l), u->g_p[l - 1], l);
     }
+    bias_final_kernel<<<(unsigned)L.size(), 1024, 0, u->stream>>>(plan, u->bias_part, u->grad);
 }
 
 // loss and output gradient of the batch whose targets and weights are in tgt, wt
 void loss(lbm_unet_s *u, int B) {
     const long long np = (long long)B * u->cfg.height * u->cfg.width;
     cudaMemsetAsync(u->sums, 0, 2 * sizeof(double), u->stream);
-    loss_kernel<<<grid_for(np), 256, 0, u->stream>>>(u->out32, 16, u->tgt, u->cfg.out_channels, u->wt, np, u->sums);
-    loss_grad_kernel<<<grid_for(np * 2), 256, 0, u->stream>>>(u->out32, 16, u->tgt, u->cfg.out_channels, u->wt,
-                                                               (int)np, u->sums, u->dout);
+    loss_kernel<<<sum_grid_for(np), 256, 0, u->stream>>>(u->out32, 16, u->tgt, u->cfg.out_channels, u->wt, np, u->sums);
+    loss_grad_kernel<<<sum_grid_for(np * 2), 256, 0, u->stream>>>(u->out32, 16, u->tgt, u->cfg.out_channels, u->wt,
+                                                               (int)np, u->sums, u->dout,
+                                                               u->bias_part + (size_t)out_layer(u) * unet_tc::BIAS_ROWS *
+                                                                                    unet_tc::BIAS_STRIDE);
 }
 
 int gather_batch(lbm_unet_s *u, int batch, const int *idx) {
@@ -1044,7 +1228,8 @@ int lbm_unet_create(const lbm_unet_config *cfg, lbm_unet *out) {
     size_t dpre_elems = np * 16;
     for (int l = 0; l <= NL; ++l)
         dpre_elems = std::max(dpre_elems, (size_t)ch(u, l) * cfg->max_batch * H_of(u, l) * W_of(u, l));
-    rc = rc ? rc : alloc(u, (void **)&u->dpre, dpre_elems * sizeof(bf16));
+    rc = rc ? rc : alloc(u, (void **)&u->bias_part, sizeof(float) * u->L.size() * unet_tc::BIAS_ROWS * unet_tc::BIAS_STRIDE);
+    for (bf16 *&d : u->dpre) rc = rc ? rc : alloc(u, (void **)&d, dpre_elems * sizeof(bf16));
     rc = rc ? rc : alloc(u, (void **)&u->fin, np * 16 * sizeof(float));
     rc = rc ? rc : alloc(u, (void **)&u->fout, np * 16 * sizeof(float));
     rc = rc ? rc : alloc(u, (void **)&u->tgt, np * 16 * sizeof(float));

@@ -145,6 +145,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, volati
     return false;
 }
 
+// One lane of a converged warp.  The issuing warps run their loops with all
+// lanes and elect the one that issues: control flow and operands then stay
+// uniform in the compiler's eyes, and the descriptors reach the tensor core's
+// uniform registers without a move per operand and instruction.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+// mbar_wait by a whole warp, the answer uniform
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity, volatile int *stop) {
+    return __all_sync(0xffffffffu, mbar_wait(mbar, parity, stop));
+}
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -227,6 +241,17 @@ __device__ __forceinline__ void tma_load4(uint32_t dst, const void *tmap, int c,
         : "memory");
 }
 
+// Tiled tensor copy of a 4-D box from shared memory; elements outside the
+// tensor are not written.  The issuing thread groups and awaits its copies.
+__device__ __forceinline__ void tma_store4(const void *tmap, int c, int x, int y, int n, uint32_t src) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(tmap),
+                 "r"(c), "r"(x), "r"(y), "r"(n), "r"(src)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_read_wait() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 constexpr int TC_BOX = 136;  // staged pixels per row: x0 - 1 .. x0 + 134, a whole number of swizzle atoms
 
 template <int COUT, int CHUNK, int NS>
@@ -241,6 +266,153 @@ struct TcSmem {
         return 1024 + NS * (size_t)A_STAGE + 18 * (size_t)cin * COUT + 4 * COUT + 8 * (2 * NS + 2 * NA) + 16;
     }
 };
+
+// One finished tile of an epilogue warp: its 32 lanes of accumulator a to
+// registers, 32 columns at a time, the accumulator released (barrier
+// `release`) once all are read, then bias, ReLU and the stores.
+// STAGED: the warp's 32 pixels go through `stage` (its own swizzled 32 x COUT
+// tile in shared memory) and leave by one tensor copy: a thread's own stores
+// are one sector in each of 32 lines, and their L1 wavefronts (512 of a
+// 64-channel tile's 860) bound the level-0 layers with 32 and 64 outputs.
+// MASK (data gradients): the output is the gradient before the layer below's
+// ReLU, so it is zeroed where that layer's activation `act` (channels from
+// act, stride act_cs) is not positive, and bsum gathers each channel's sum of
+// the stored values over this lane's pixels, the bias gradient's share.
+template <int COUT, bool MASK>
+struct EpilogueMask {
+    const __nv_bfloat16 *act = nullptr;
+    int act_cs = 0;
+    float bsum[MASK ? COUT : 1];
+    // the tile's activations, and the next tile's on their way: a load takes
+    // about a tile's time to arrive
+    uint32_t m[MASK ? COUT / 16 : 1][8], ahead[MASK ? COUT / 16 : 1][8];
+    __device__ __forceinline__ void take() {
+        if constexpr (MASK) {
+#pragma unroll
+            for (int i = 0; i < COUT / 16; ++i)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) m[i][k] = ahead[i][k];
+        }
+    }
+    __device__ __forceinline__ void load(bool in, size_t pix) {
+        if constexpr (MASK) {
+#pragma unroll
+            for (int i = 0; i < COUT / 16; ++i) {
+                const void *p = act + pix * act_cs + 16 * i;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ahead[i][k] = 0u;
+                if (in)
+                    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                 : "=r"(ahead[i][0]), "=r"(ahead[i][1]), "=r"(ahead[i][2]), "=r"(ahead[i][3]),
+                                   "=r"(ahead[i][4]), "=r"(ahead[i][5]), "=r"(ahead[i][6]), "=r"(ahead[i][7])
+                                 : "l"(p));
+            }
+        }
+    }
+};
+template <int COUT, bool STAGED, bool MASK = false>
+__device__ __forceinline__ void conv_epilogue(uint32_t tmem, uint32_t a, uint32_t release, const float *sbias,
+                                              const CUtensorMap *tout, uint32_t stage, __nv_bfloat16 *out, int out_cs,
+                                              int out_co, float *out32, int n, int y, int xb, int H, int W, int relu,
+                                              EpilogueMask<COUT, MASK> *mask = nullptr) {
+    constexpr int CW = COUT < 32 ? COUT : 32, RB = COUT * 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    fence_after();
+    const int x = xb * TC_M + warp * 32 + lane;  // TMEM lane = GEMM row = pixel
+    const size_t pix = ((size_t)n * H + y) * W + x;
+    const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + a * COUT;
+    if (STAGED) {
+        if (lane == 0) tma_store_read_wait();  // the tile before has left the stage
+        __syncwarp();
+    }
+#pragma unroll(MASK ? COUT / CW : 1)
+    for (int c = 0; c < COUT; c += CW) {
+        uint32_t r[CW / 16][16];
+#pragma unroll
+        for (int i = 0; i < CW / 16; ++i) tmem_ld16_async(acc + (uint32_t)(c + 16 * i), r[i]);
+#pragma unroll
+        for (int i = 0; i < CW / 16; ++i) tmem_wait(r[i]);
+        if (c + CW == COUT) {
+            // every column is in registers: the accumulator is free
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(release);
+        }
+#pragma unroll
+        for (int q = 0; q < CW / 16; ++q) {
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 b4 = *(const float4 *)(sbias + c + 16 * q + 4 * i);
+                v[4 * i] = __uint_as_float(r[q][4 * i]) + b4.x;
+                v[4 * i + 1] = __uint_as_float(r[q][4 * i + 1]) + b4.y;
+                v[4 * i + 2] = __uint_as_float(r[q][4 * i + 2]) + b4.z;
+                v[4 * i + 3] = __uint_as_float(r[q][4 * i + 3]) + b4.w;
+            }
+            if (relu) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
+            }
+            if (STAGED || out) {
+                uint32_t pk[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                    pk[i] = *(const uint32_t *)&h2;
+                }
+                if constexpr (MASK) {
+                    // positive: sign clear and not zero (zero beyond the image)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t m = mask->m[c / 16 + q][i];
+                        const __nv_bfloat162 mv = *(const __nv_bfloat162 *)&m;
+                        const float2 mf = __bfloat1622float2(mv);
+                        const __nv_bfloat162 pv = *(const __nv_bfloat162 *)&pk[i];
+                        float2 pf = __bfloat1622float2(pv);
+                        if (!(mf.x > 0.f)) {
+                            pk[i] &= 0xFFFF0000u;
+                            pf.x = 0.f;
+                        }
+                        if (!(mf.y > 0.f)) {
+                            pk[i] &= 0x0000FFFFu;
+                            pf.y = 0.f;
+                        }
+                        mask->bsum[c + 16 * q + 2 * i] += pf.x;
+                        mask->bsum[c + 16 * q + 2 * i + 1] += pf.y;
+                    }
+                }
+                if (STAGED) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        // the tensor copy's swizzle: 16-byte chunk index xor 128-byte line index
+                        uint32_t off = (uint32_t)(lane * RB + 2 * (c + 16 * q) + 16 * k);
+                        off ^= ((off >> 7) & (RB / 16 - 1)) << 4;
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + off), "r"(pk[4 * k]),
+                                     "r"(pk[4 * k + 1]), "r"(pk[4 * k + 2]), "r"(pk[4 * k + 3])
+                                     : "memory");
+                    }
+                } else if (x < W) {
+                    store32(out + pix * out_cs + out_co + c + 16 * q, pk);
+                }
+            }
+            if (!STAGED && out32 && x < W) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) pk[j] = __float_as_uint(v[8 * i + j]);
+                    store32(out32 + pix * COUT + c + 16 * q + 8 * i, pk);
+                }
+            }
+        }
+    }
+    if (STAGED) {
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0 && xb * TC_M + warp * 32 < W)
+            tma_store4(tout, 0, xb * TC_M + warp * 32, y, n, stage);
+    }
+}
 
 // Warp roles: warps 0-3 read the accumulators (each its 32 TMEM lanes) and
 // store the outputs; one thread of warp 4 issues the tensor copies, one of
@@ -336,55 +508,55 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
         }
         __syncwarp();
     } else if (warp == 5) {
-        if (lane == 0) {
-            constexpr uint32_t IDESC = idesc_bf16(TC_M, COUT);
-            Ring<NS> st;
-            Ring<NA> ac;
-            const uint32_t tap_step = (uint32_t)(KGall * COUT);
-            int committed = 0;
-            for (int k = walk.left; k > 0 && ok; --k, ac.next()) {
-                // the epilogue of tile k - NA has read the accumulator
-                if (ac.round > 0 && !mbar_wait(acce0 + 8 * ac.slot, (ac.round - 1) & 1, abort_flag)) {
+        constexpr uint32_t IDESC = idesc_bf16(TC_M, COUT);
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        Ring<NS> st;
+        Ring<NA> ac;
+        const uint32_t tap_step = (uint32_t)(KGall * COUT);
+        int committed = 0;
+        for (int k = walk.left; k > 0 && ok; --k, ac.next()) {
+            // the epilogue of tile k - NA has read the accumulator
+            if (ac.round > 0 && !mbar_wait_warp(acce0 + 8 * ac.slot, (ac.round - 1) & 1, abort_flag)) {
+                ok = false;
+                break;
+            }
+            const uint32_t d = tm + ac.slot * COUT;
+            for (int c = 0; c < nch; ++c) {
+                const uint32_t s = st.slot;
+                if (!mbar_wait_warp(full0 + 8 * s, st.round & 1, abort_flag)) {
                     ok = false;
                     break;
                 }
-                const uint32_t d = tmem + ac.slot * COUT;
-                for (int c = 0; c < nch; ++c) {
-                    const uint32_t s = st.slot;
-                    if (!mbar_wait(full0 + 8 * s, st.round & 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    fence_after();
-                    const Desc da(smem_desc_sw<ROWB>(base + s * A_STAGE));
-                    const Desc db(smem_desc(b_base + (uint32_t)(c * KG * COUT * 16), COUT * 16, 128));
-                    uint32_t bt = 0;
+                fence_after();
+                const Desc da(smem_desc_sw<ROWB>(base + s * A_STAGE));
+                const Desc db(smem_desc(b_base + (uint32_t)(c * KG * COUT * 16), COUT * 16, 128));
+                if (leader) {
 #pragma unroll
                     for (int t = 0; t < 9; ++t) {
 #pragma unroll
                         for (int q = 0; q < KG / 2; ++q)
                             mma_bf16(d, da, (uint32_t)(((t / 3) * TC_BOX + t % 3) * ROWB / 16 + 2 * q), db,
-                                     bt + (uint32_t)(2 * q * COUT), IDESC, (c > 0 || t > 0 || q > 0) ? 1u : 0u);
-                        bt += tap_step;
+                                     (uint32_t)t * tap_step + (uint32_t)(2 * q * COUT), IDESC,
+                                     (c > 0 || t > 0 || q > 0) ? 1u : 0u);
                     }
                     mma_commit(empty0 + 8 * s);
-                    st.next();
-                    ++committed;
+                    if (c == nch - 1) mma_commit(accf0 + 8 * ac.slot);
                 }
-                if (ok) mma_commit(accf0 + 8 * ac.slot);
+                st.next();
+                ++committed;
             }
-            if (!ok) {
-                *abort_flag = 1;
-                atomicExch(err, 1);
-                // MMAs complete in order: the last commit covers them all
-                if (committed > 0)
-                    mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1));
-            }
+        }
+        if (!ok) {
+            *abort_flag = 1;
+            if (leader) atomicExch(err, 1);
+            // MMAs complete in order: the last commit covers them all
+            if (committed > 0)
+                mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1));
         }
         __syncwarp();
     } else {
         // epilogue warps: tile k from accumulator k % NA, 32 columns at a time
-        constexpr int CW = COUT < 32 ? COUT : 32;
         Ring<NA> ac;
         for (; walk.left > 0; walk.next(), ac.next()) {
             const uint32_t a = ac.slot;
@@ -393,52 +565,278 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
                 ok = false;
                 break;
             }
-            fence_after();
-            const int x = walk.xb * TC_M + warp * 32 + lane;  // TMEM lane = GEMM row = pixel
-            const size_t pix = ((size_t)walk.n * H + walk.y) * W + x;
-            const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + a * COUT;
-#pragma unroll 1
-            for (int c = 0; c < COUT; c += CW) {
-                uint32_t r[CW / 16][16];
-#pragma unroll
-                for (int i = 0; i < CW / 16; ++i) tmem_ld16_async(acc + (uint32_t)(c + 16 * i), r[i]);
-#pragma unroll
-                for (int i = 0; i < CW / 16; ++i) tmem_wait(r[i]);
-                if (c + CW == COUT) {
-                    // every column is in registers: the accumulator is free
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acce0 + 8 * a);
+            conv_epilogue<COUT, false>(tmem, a, acce0 + 8 * a, sbias, nullptr, 0, out, out_cs, out_co, out32, walk.n,
+                                       walk.y, walk.xb, H, W, relu);
+        }
+        if (!ok) {
+            *abort_flag = 1;
+            if (lane == 0) atomicExch(err, 1);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+}
+
+// The same convolution with a ring of input rows: a CTA takes a contiguous run
+// of tiles in the order (image, row segment, y), y fastest, and keeps whole
+// input rows (all cin channels, TC_BOX pixels) in NR ring slots, so a tile
+// brings one new row where conv3x3_tc_kernel's stage brings three, and the
+// tiles divide evenly over the CTAs.  A run crosses a few column segments; each
+// costs two extra rows.  Chunks of CHUNK channels lie one after another in a
+// slot, each a swizzled K-major tile of its own, and the MMAs run chunk, tap,
+// K = 16, the order of conv3x3_tc_kernel, so the sums are the same.
+// Barriers as there, with one full and empty barrier per slot: a slot is
+// released by the commit of the last tile that reads its row.
+template <int COUT, int CHUNK>
+struct RowSmem {
+    static constexpr int NA = 4 * COUT <= 512 ? 4 : 2;
+    static constexpr int ROWB = CHUNK * 2, SUB = TC_BOX * ROWB;  // a chunk of a row; a whole number of swizzle atoms
+    // outputs of 32 and 64 channels leave through shared memory (conv_epilogue)
+    static constexpr bool STAGED = COUT == 32 || COUT == 64;
+    static constexpr int STAGE = STAGED ? TC_M * COUT * 2 : 0;
+    static constexpr size_t row_bytes(int cin) { return (size_t)TC_BOX * 2 * cin; }
+    static constexpr size_t bytes(int cin, int nr) {
+        return 1024 + STAGE + nr * row_bytes(cin) + 18 * (size_t)cin * COUT + 4 * COUT + 8 * (2 * nr + 2 * NA) + 16;
+    }
+};
+constexpr int ROW_MAX = 8;  // most ring slots
+// rows of partial bias gradients a kernel may leave, one per block, and their pitch
+constexpr int BIAS_ROWS = 1216, BIAS_STRIDE = 64;
+
+// A run of tiles in the order (n, xb, y), y fastest.
+struct RunWalk {
+    int y, xb, n, left, xt, H;
+    __device__ __forceinline__ RunWalk(int B, int H_, int xt_) : xt(xt_), H(H_) {
+        const long long total = (long long)B * H * xt;
+        const int t0 = (int)(total * blockIdx.x / gridDim.x), t1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
+        left = t1 - t0;
+        y = t0 % H;
+        xb = t0 / H % xt;
+        n = t0 / H / xt;
+    }
+    // tiles left in this column segment
+    __device__ __forceinline__ int segment() const { return left < H - y ? left : H - y; }
+    __device__ __forceinline__ void advance(int k) {
+        left -= k;
+        y += k;
+        if (y == H) {
+            y = 0;
+            if (++xb == xt) {
+                xb = 0;
+                ++n;
+            }
+        }
+    }
+};
+// Ring position with a run-time number of slots.
+struct RowRing {
+    int slot = 0, nr;
+    uint32_t round = 0;
+    __device__ __forceinline__ explicit RowRing(int n) : nr(n) {}
+    __device__ __forceinline__ void next() {
+        if (++slot == nr) {
+            slot = 0;
+            ++round;
+        }
+    }
+};
+
+template <int COUT, int CHUNK, bool MASK>
+__global__ void __launch_bounds__(CONV_THREADS, 1)
+conv3x3_rows_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout, int cin, int nr, const __nv_bfloat16 *__restrict__ w,
+                    const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out, int out_cs, int out_co,
+                    float *__restrict__ out32, const __nv_bfloat16 *__restrict__ act, int act_cs, float *__restrict__ db_rows,
+                    int B, int H, int W, int relu, int *err) {
+    static_assert(COUT % 16 == 0 && COUT <= 128 && (CHUNK == 16 || CHUNK == 32 || CHUNK == 64), "N, K chunk");
+    using SM = RowSmem<COUT, CHUNK>;
+    constexpr int ROWB = SM::ROWB, SUB = SM::SUB, KG = CHUNK / 8, NA = SM::NA;
+    constexpr uint32_t COLS = NA * COUT < 32 ? 32 : NA * COUT;  // a power of two >= 32
+    __shared__ float db_sum[MASK ? 4 : 1][MASK ? COUT : 1];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw), stage0 = (raw + 1023u) & ~1023u, base = stage0 + SM::STAGE;
+    unsigned char *smem = smem_raw + (base - raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int KGall = cin / 8, nch = cin / CHUNK;
+    const uint32_t row = (uint32_t)(TC_BOX * 2 * cin), b_base = base + (uint32_t)nr * row;
+    float *sbias = (float *)(smem + (size_t)nr * row + (size_t)18 * cin * COUT);
+    uint64_t *bars = (uint64_t *)(sbias + COUT);
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * nr, accf0 = empty0 + 8 * nr, acce0 = accf0 + 8 * NA;
+    uint32_t *tmem_slot = (uint32_t *)(bars + 2 * nr + 2 * NA);
+    volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+    RunWalk walk(B, H, (W + TC_M - 1) / TC_M);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < nr; ++k) {
+            mbar_init(full0 + 8 * k, 1);
+            mbar_init(empty0 + 8 * k, 1);
+        }
+        for (int a = 0; a < NA; ++a) {
+            mbar_init(accf0 + 8 * a, 1);
+            mbar_init(acce0 + 8 * a, 4);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < COUT) sbias[tid] = bias ? bias[tid] : 0.f;
+    // every weight of the layer, as in conv3x3_tc_kernel
+    for (int i = tid; i < 9 * KGall * COUT; i += CONV_THREADS) {
+        const int tc = i / KGall, j = i % KGall, t = tc / COUT, co = tc % COUT;
+        cp_async16(b_base + (uint32_t)(((t * KGall + j) * COUT + co) * 16), w + (size_t)i * 8, 16);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    fence_proxy_async();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tmem_slot;
+    bool ok = true;
+
+    if (warp == 4) {
+        if (lane == 0) {
+            RowRing st(nr);
+            int issued = 0;
+            while (walk.left > 0 && ok) {
+                const int seg = walk.segment();
+                for (int r = -1; r <= seg; ++r, st.next(), ++issued) {
+                    const uint32_t s = (uint32_t)st.slot, fb = full0 + 8 * s;
+                    if (st.round > 0 && !mbar_wait(empty0 + 8 * s, (st.round - 1) & 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(fb, row);
+                    for (int c = 0; c < nch; ++c)
+                        tma_load4(base + s * row + (uint32_t)(c * SUB), &tin, c * CHUNK, walk.xb * TC_M - 1,
+                                  walk.y + r, walk.n, fb);
                 }
-                if (x < W) {
+                walk.advance(seg);
+            }
+            if (!ok) {
+                *abort_flag = 1;
+                atomicExch(err, 1);
+                // the copies in flight land before the CTA leaves: the last
+                // use of each slot
+                for (int j = issued > nr ? issued - nr : 0; j < issued; ++j)
+                    mbar_wait(full0 + 8 * (uint32_t)(j % nr), (uint32_t)((j / nr) & 1));
+            }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        constexpr uint32_t IDESC = idesc_bf16(TC_M, COUT);
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        RowRing st(nr);
+        Ring<NA> ac;
+        const uint32_t tap_step = (uint32_t)(KGall * COUT);
+        int w0 = 0, w1 = 0, w2 = 0;  // slots of the tile's rows y - 1, y, y + 1
+        int last_slot = -1;          // the last commit's barrier and phase
+        uint32_t last_round = 0;
+        auto take = [&]() -> bool {  // the next row of the ring becomes w2
+            w0 = w1;
+            w1 = w2;
+            w2 = st.slot;
+            const bool got = mbar_wait_warp(full0 + 8 * (uint32_t)st.slot, st.round & 1, abort_flag);
+            st.next();
+            return got;
+        };
+        while (walk.left > 0 && ok) {
+            const int seg = walk.segment();
+            ok = take() && take();
+            for (int k = 0; k < seg && ok; ++k, ac.next()) {
+                if (!take() ||
+                    (ac.round > 0 && !mbar_wait_warp(acce0 + 8 * ac.slot, (ac.round - 1) & 1, abort_flag))) {
+                    ok = false;
+                    break;
+                }
+                fence_after();
+                const uint32_t d = tm + ac.slot * COUT;
+                for (int c = 0; c < nch; ++c) {
+                    const uint32_t sub = (uint32_t)(c * SUB);
+                    const Desc r0(smem_desc_sw<ROWB>(base + (uint32_t)w0 * row + sub)),
+                        r1(smem_desc_sw<ROWB>(base + (uint32_t)w1 * row + sub)),
+                        r2(smem_desc_sw<ROWB>(base + (uint32_t)w2 * row + sub));
+                    const Desc db(smem_desc(b_base + (uint32_t)(c * KG * COUT * 16), COUT * 16, 128));
+                    if (leader) {
 #pragma unroll
-                    for (int q = 0; q < CW / 16; ++q) {
-                        float v[16];
+                        for (int t = 0; t < 9; ++t) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            v[i] = __uint_as_float(r[q][i]) + sbias[c + 16 * q + i];
-                            if (relu) v[i] = fmaxf(v[i], 0.f);
-                        }
-                        if (out) {
-                            uint32_t pk[8];
-#pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                                pk[i] = *(const uint32_t *)&h2;
-                            }
-                            store32(out + pix * out_cs + out_co + c + 16 * q, pk);
-                        }
-                        if (out32) {
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                uint32_t pk[8];
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) pk[j] = __float_as_uint(v[8 * i + j]);
-                                store32(out32 + pix * COUT + c + 16 * q + 8 * i, pk);
-                            }
+                            for (int q = 0; q < KG / 2; ++q)
+                                mma_bf16(d, t < 3 ? r0 : (t < 6 ? r1 : r2), (uint32_t)((t % 3) * ROWB / 16 + 2 * q), db,
+                                         (uint32_t)t * tap_step + (uint32_t)(2 * q * COUT), IDESC,
+                                         (c > 0 || t > 0 || q > 0) ? 1u : 0u);
                         }
                     }
                 }
+                // row y - 1 has served; at a segment's end so have the others
+                if (leader) {
+                    mma_commit(empty0 + 8 * (uint32_t)w0);
+                    if (k == seg - 1) {
+                        mma_commit(empty0 + 8 * (uint32_t)w1);
+                        mma_commit(empty0 + 8 * (uint32_t)w2);
+                    }
+                    mma_commit(accf0 + 8 * ac.slot);
+                }
+                last_slot = w0;
+                last_round = st.round - (w0 >= st.slot ? 1u : 0u);
+            }
+            walk.advance(seg);
+        }
+        if (!ok) {
+            *abort_flag = 1;
+            if (leader) atomicExch(err, 1);
+            // MMAs complete in order: the last commit covers them all
+            if (last_slot >= 0) mbar_wait(empty0 + 8 * (uint32_t)last_slot, last_round & 1);
+        }
+        __syncwarp();
+    } else {
+        // epilogue warps: tile k from accumulator k % NA, 32 columns at a time
+        Ring<NA> ac;
+        EpilogueMask<COUT, MASK> mask;
+        if constexpr (MASK) {
+            mask.act = act;
+            mask.act_cs = act_cs;
+#pragma unroll
+            for (int i = 0; i < COUT; ++i) mask.bsum[i] = 0.f;
+        }
+        RunWalk next = walk;
+        auto load_next = [&]() {
+            if constexpr (MASK) {
+                const int x = next.xb * TC_M + warp * 32 + lane;
+                mask.load(next.left > 0 && x < W, ((size_t)next.n * H + next.y) * W + x);
+                if (next.left > 0) next.advance(1);
+            }
+        };
+        load_next();
+        for (; walk.left > 0; walk.advance(1), ac.next()) {
+            mask.take();
+            load_next();
+            const bool got = mbar_wait(accf0 + 8 * ac.slot, ac.round & 1, abort_flag);
+            if (!__all_sync(0xffffffffu, got)) {
+                ok = false;
+                break;
+            }
+            conv_epilogue<COUT, SM::STAGED, MASK>(tmem, ac.slot, acce0 + 8 * ac.slot, sbias, &tout,
+                                                  stage0 + (uint32_t)warp * 64 * COUT, out, out_cs, out_co, out32, walk.n,
+                                                  walk.y, walk.xb, H, W, relu, &mask);
+        }
+        if (SM::STAGED && lane == 0) tma_store_wait();
+        if constexpr (MASK) {
+            // channel sums of the warp's pixels, then (below) of the CTA's
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < COUT; ++i) {
+                float v = mask.bsum[i];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == i % 32) db_sum[warp][i] = v;
             }
         }
         if (!ok) {
@@ -448,6 +846,11 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
     }
     fence_before();
     __syncthreads();
+    if constexpr (MASK) {
+        if (tid < COUT)
+            db_rows[(size_t)blockIdx.x * BIAS_STRIDE + tid] =
+                (db_sum[0][tid] + db_sum[1][tid]) + (db_sum[2][tid] + db_sum[3][tid]);
+    }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
 }
@@ -579,13 +982,15 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
             for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
                 mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
         }
-    } else if (tid == 32) {
+    } else if (warp == 1) {
         bool ok = true;
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         Ring<NS> st;
         int committed = 0;
         for (int j = 0; j < jobs; ++j, st.next()) {
             const uint32_t s = st.slot;
-            if (!mbar_wait(full0 + 8 * s, st.round & 1, &abort_flag)) {
+            if (!mbar_wait_warp(full0 + 8 * s, st.round & 1, &abort_flag)) {
                 ok = false;
                 break;
             }
@@ -593,29 +998,33 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
             const uint32_t a0 = base + s * STAGE;
             const Desc da(smem_desc_sw_mn<ROWB_A>(a0, TC_M * ROWB_A));
             const Desc db(smem_desc_sw_mn<ROWB_B>(a0 + A_STAGE, TC_BOX * ROWB_B));
+            if (leader) {
 #pragma unroll
-            for (int ks = 0; ks < TC_M / 16; ++ks) {
+                for (int ks = 0; ks < TC_M / 16; ++ks) {
 #pragma unroll
-                for (int b = 0; b < MB; ++b) {
+                    for (int b = 0; b < MB; ++b) {
 #pragma unroll
-                    for (int kx = 0; kx < 3; ++kx)
-                        mma_bf16(tmem + (uint32_t)((b * 3 + kx) * NC), da,
-                                 (uint32_t)((b * 128 * TC_M * 2 + 16 * ks * ROWB_A) / 16), db,
-                                 (uint32_t)((16 * ks + kx) * ROWB_B / 16), IDESC, (j > 0 || ks > 0) ? 1u : 0u);
+                        for (int kx = 0; kx < 3; ++kx)
+                            mma_bf16(tm + (uint32_t)((b * 3 + kx) * NC), da,
+                                     (uint32_t)((b * 128 * TC_M * 2 + 16 * ks * ROWB_A) / 16), db,
+                                     (uint32_t)((16 * ks + kx) * ROWB_B / 16), IDESC, (j > 0 || ks > 0) ? 1u : 0u);
+                    }
                 }
+                mma_commit(empty0 + 8 * s);
             }
-            mma_commit(empty0 + 8 * s);
             ++committed;
         }
         // the last commit covers every MMA (they complete in order)
         if (committed > 0 &&
-            !mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1)))
+            !mbar_wait_warp(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1), nullptr))
             ok = false;
-        if (!ok) {
-            abort_flag = 1;
-            atomicExch(err, 1);
+        if (leader) {
+            if (!ok) {
+                abort_flag = 1;
+                atomicExch(err, 1);
+            }
+            status = ok && committed == jobs ? 1 : 0;
         }
-        status = ok && committed == jobs ? 1 : 0;
     }
     __syncthreads();
     if (status && jobs > 0) {
