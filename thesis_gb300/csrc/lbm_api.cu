@@ -129,7 +129,7 @@ struct lbm_handle_s {
     const void *res_kern = nullptr;
     ResidentPlan res_plan;
     unsigned long long *res_mail = nullptr;
-    unsigned *res_err = nullptr;
+    unsigned *res_err = nullptr, *res_err_d = nullptr;  // host word and its device address
     unsigned res_tag = 0;
     double omega = 1, omega_m = 1, gshift = 0;
     float scale = 1024.f;
@@ -190,9 +190,10 @@ static void free_handle(lbm_handle_s *H) {
     void *ptrs[] = {H->fbuf[0], H->fbuf[1], H->word, H->slot, H->mask, H->kind, H->uvw,
                     H->rho, H->ux, H->uy, H->uz, H->pux, H->puy, H->puz, H->partial, H->norms,
                     H->tma_row, H->tma_lmask, H->tma_omask, H->tma_err, H->mdiff_prev, H->fd_snap,
-                    H->bcq, H->bc_macro, H->res_mail, H->res_err};
+                    H->bcq, H->bc_macro, H->res_mail};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (H->res_err) cudaFreeHost(H->res_err);
     if (H->stepped) cudaEventDestroy(H->stepped);
     if (H->stream) cudaStreamDestroy(H->stream);
     delete H;
@@ -401,13 +402,16 @@ static int setup_resident(lbm_handle_s *H) {
     if (!kern) return LBM_OK;
     const size_t bytes = sizeof(unsigned long long) * 16 * (size_t)H->N;
     cudaError_t e = cudaMalloc((void **)&H->res_mail, bytes);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&H->res_err, sizeof(unsigned));
+    // the error word lies in host memory: only a wait that gives up writes it,
+    // and the host reads it without a copy
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&H->res_err, sizeof(unsigned), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&H->res_err_d, (void *)H->res_err, 0);
     if (e == cudaSuccess) e = cudaMemset(H->res_mail, 0, bytes);
-    if (e == cudaSuccess) e = cudaMemset(H->res_err, 0, sizeof(unsigned));
     if (e != cudaSuccess) {
         cudaGetLastError();  // no room for the messages: a launch per step
         return LBM_OK;
     }
+    *(volatile unsigned *)H->res_err = 0;
     H->res_kern = kern;
     return LBM_OK;
 }
@@ -415,13 +419,9 @@ static int setup_resident(lbm_handle_s *H) {
 // A bounded wait inside the row-staged or the on-chip kernel that gave up
 // leaves a code on the device; report it once the stream is idle.
 static int check_tma(lbm_handle_s *H) {
-    if (H->res_kern) {
-        unsigned int err = 0;
-        CUDA_TRY(cudaMemcpy(&err, H->res_err, sizeof(err), cudaMemcpyDeviceToHost));
-        if (err) {
-            H->status = LBM_ERR_CUDA;
-            return fail(LBM_ERR_CUDA, "on-chip steps: a wait for a neighbouring tile gave up");
-        }
+    if (H->res_kern && *(volatile unsigned *)H->res_err) {
+        H->status = LBM_ERR_CUDA;
+        return fail(LBM_ERR_CUDA, "on-chip steps: a wait for a neighbouring tile gave up");
     }
     if (!H->tma_kernel) return LBM_OK;
     unsigned int err = 0;
@@ -884,7 +884,7 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
         a.wrap = H->jit_key.wrap;
         a.tag = H->res_tag;
         a.mail = H->res_mail;
-        a.err = H->res_err;
+        a.err = H->res_err_d;
         const int e = resident_launch(H->res_kern, H->res_plan, a, s);
         if (e != cudaSuccess) {
             H->status = LBM_ERR_CUDA;
@@ -938,10 +938,12 @@ int lbm_get_macro(lbm_handle H, float *rho, float *u, float *v, float *w) {
     CUDA_TRY(cudaDeviceSynchronize());
     if (int rc = check_tma(H)) return rc;
     const size_t b = sizeof(float) * H->N;
-    if (rho) CUDA_TRY(cudaMemcpy(rho, H->rho, b, cudaMemcpyDeviceToHost));
-    if (u) CUDA_TRY(cudaMemcpy(u, H->ux, b, cudaMemcpyDeviceToHost));
-    if (v) CUDA_TRY(cudaMemcpy(v, H->uy, b, cudaMemcpyDeviceToHost));
-    if (w) CUDA_TRY(cudaMemcpy(w, H->uz, b, cudaMemcpyDeviceToHost));
+    // queued together and awaited once
+    if (rho) CUDA_TRY(cudaMemcpyAsync(rho, H->rho, b, cudaMemcpyDeviceToHost, H->stream));
+    if (u) CUDA_TRY(cudaMemcpyAsync(u, H->ux, b, cudaMemcpyDeviceToHost, H->stream));
+    if (v) CUDA_TRY(cudaMemcpyAsync(v, H->uy, b, cudaMemcpyDeviceToHost, H->stream));
+    if (w) CUDA_TRY(cudaMemcpyAsync(w, H->uz, b, cudaMemcpyDeviceToHost, H->stream));
+    CUDA_TRY(cudaStreamSynchronize(H->stream));
     return LBM_OK;
 }
 

@@ -43,7 +43,7 @@ namespace lbm {
 namespace {
 
 constexpr int PLANE = 2944;              // halo'd tile nodes a buffer holds per direction (desc packs t in 12 bits)
-constexpr int MAX_COMPUTE = 512, MAX_COMM = 256, MSGS = 4;  // threads; messages per comm thread
+constexpr int MAX_COMPUTE = 512, MAX_COMM = 128, MSGS = 8;  // threads; messages per comm thread
 constexpr unsigned RES_SPIN = 1u << 22;  // polls of a wait, seconds
 
 __device__ __forceinline__ unsigned long long mail_load(const unsigned long long *q) {
@@ -153,28 +153,40 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
     const int bar_threads = edge_threads + (int)blockDim.x - a.compute;
 
     if (tid < a.compute) {
+        // the boundary record of this thread's first node, which it updates in
+        // every step: three dependent loads and the conversions of its FP64
+        // velocity off the steps' critical path
+        SlotInfo slot;
+        if (tid < nt && (desc[tid] & W_SPECIAL)) {
+            const int t = desc[tid] >> 20;
+            slot = load_slot<PHYS>(a.p, x0 - 1 + t % pitch + nx * (y0 - 1 + t / pitch));
+        }
+        // A node's streamed populations: pulled, or its own across a blocked link.
+        auto gather = [&](const T *c, uint32_t w, T (&raw)[9]) {
+            const T *lo = c - pitch, *hi = c + pitch;
+            raw[0] = c[0];
+            raw[1] = c[PLANE - 1];
+            raw[2] = lo[2 * PLANE];
+            raw[3] = c[3 * PLANE + 1];
+            raw[4] = hi[4 * PLANE];
+            raw[5] = lo[5 * PLANE - 1];
+            raw[6] = lo[6 * PLANE + 1];
+            raw[7] = hi[7 * PLANE + 1];
+            raw[8] = hi[8 * PLANE - 1];
+            if (w & 0x1FEu) {
+#pragma unroll
+                for (int d = 1; d < 9; ++d)
+                    if ((w >> d) & 1u) raw[d] = c[(PHYS ? L::opp(d) : d) * PLANE];
+            }
+        };
         // One step of this thread's nodes; LAST writes to global memory.
         auto nodes = [&](const StepParams &p, const T *in, T *out, auto last_tag) {
             constexpr bool LAST = decltype(last_tag)::value;
-            auto node_step = [&](int i) {
+            auto node_step = [&](int i, const SlotInfo *pre) {
                 const uint32_t u = desc[i], w = u & 0xFFFFFu;
                 const int t = u >> 20;
-                const T *c = in + t, *lo = c - pitch, *hi = c + pitch;
                 T raw[9];
-                raw[0] = c[0];
-                raw[1] = c[PLANE - 1];
-                raw[2] = lo[2 * PLANE];
-                raw[3] = c[3 * PLANE + 1];
-                raw[4] = hi[4 * PLANE];
-                raw[5] = lo[5 * PLANE - 1];
-                raw[6] = lo[6 * PLANE + 1];
-                raw[7] = hi[7 * PLANE + 1];
-                raw[8] = hi[8 * PLANE - 1];
-                if (w & 0x1FEu) {
-#pragma unroll
-                    for (int d = 1; d < 9; ++d)
-                        if ((w >> d) & 1u) raw[d] = c[(PHYS ? L::opp(d) : d) * PLANE];
-                }
+                gather(in + t, w, raw);
                 int node = 0;
                 if (LAST || (w & W_SPECIAL)) node = x0 - 1 + t % pitch + nx * (y0 - 1 + t / pitch);
                 T res[9];
@@ -183,14 +195,14 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
                         f1 h[9];
 #pragma unroll
                         for (int d = 0; d < 9; ++d) h[d] = f1(pop_value(raw[d]));
-                        h_finish<9, COLL, ST, true, true, DynGeom>(p, g, node, w, h);
+                        h_finish<9, COLL, ST, true, true, DynGeom>(p, g, node, w, h, pre);
 #pragma unroll
                         for (int d = 0; d < 9; ++d) h_put<ST>(&res[d], h[d].v);
                     } else {
                         float f[9];
 #pragma unroll
                         for (int d = 0; d < 9; ++d) f[d] = S::decode(raw[d], p.shift[d], p.inv_scale);
-                        update_node<9, COLL, ST, false, true, DynGeom>(f, w, node, p, g);
+                        update_node<9, COLL, ST, false, true, DynGeom>(f, w, node, p, g, pre);
 #pragma unroll
                         for (int d = 0; d < 9; ++d) res[d] = S::encode(f[d], p.shift[d], p.scale);
                     }
@@ -208,7 +220,7 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
                     for (int d = 0; d < 9; ++d) out[d * PLANE + t] = res[d];
                 }
             };
-            if (tid < nt) node_step(tid);
+            if (tid < nt) node_step(tid, &slot);
             if constexpr (!LAST) {
                 // the perimeter lies in the first round: hand it over
                 if (tid < edge_threads) {
@@ -216,8 +228,38 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
                     bar_arrive(1, bar_threads);
                 }
             }
+            int i = tid + a.compute;
+            if constexpr (PHYS && !LAST) {
+                // the inner rounds two at a time on packed FP32x2
 #pragma unroll 1
-            for (int i = tid + a.compute; i < nt; i += a.compute) node_step(i);
+                for (; i + a.compute < nt; i += 2 * a.compute) {
+                    const uint32_t ua = desc[i], ub = desc[i + a.compute];
+                    if ((ua | ub) & W_SPECIAL) {
+                        node_step(i, nullptr);
+                        node_step(i + a.compute, nullptr);
+                        continue;
+                    }
+                    const bool fa = ua & W_FLUID, fb = ub & W_FLUID;
+                    const int ta = ua >> 20, tb = ub >> 20;
+                    const T *ca = in + ta, *cb = in + tb;
+                    T ra[9], rb[9];
+                    gather(ca, ua, ra);
+                    gather(cb, ub, rb);
+                    f2 h[9];
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) h[d] = f2(fa ? pop_value(ra[d]) : 0.f, fb ? pop_value(rb[d]) : 0.f);
+                    h_pair_relax<9, COLL, ST, true>(p, 0, 0, fa, fb, h);
+                    const float S0 = ST == LBM_STORE_F16S ? p.scale : 1.f;
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) {
+                        const float zero = -p.sigma * p.shift[d] * S0;
+                        h_put<ST>(out + d * PLANE + ta, fa ? h[d].v.x : zero);
+                        h_put<ST>(out + d * PLANE + tb, fb ? h[d].v.y : zero);
+                    }
+                }
+            }
+#pragma unroll 1
+            for (; i < nt; i += a.compute) node_step(i, nullptr);
         };
 #pragma unroll 1
         for (int s = 0; s < a.steps - 1; ++s) {
@@ -297,7 +339,7 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
                     break;
                 }
             }
-            if (bad) atomicExch(a.err, 1u);
+            if (bad) *(volatile unsigned *)a.err = 1u;
             if (__syncthreads_or(bad)) return;
         }
     }

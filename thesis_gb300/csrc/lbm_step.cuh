@@ -331,23 +331,42 @@ __device__ __forceinline__ void phys_open_outlet(V (&f)[Q], int kind, int sl, in
     }
 }
 
+// A boundary slot's record, for a thread that keeps one node over many steps
+// (FP32 arithmetic); the step kernels read what they need of it as they go.
+struct SlotInfo {
+    int sl = 0, kind = 0;
+    unsigned long long mask = 0;
+    float u = 0.f, v = 0.f, w = 0.f;
+};
+template <bool PHYS>
+__device__ __forceinline__ SlotInfo load_slot(const StepParams &p, int node) {
+    SlotInfo s;
+    s.sl = __ldg(p.slot + node);
+    if (PHYS) s.kind = __ldg(p.bc_kind + s.sl);
+    s.mask = __ldg(p.bc_mask + s.sl);
+    s.u = (float)__ldg(p.bc_uvw + 3 * s.sl);
+    s.v = (float)__ldg(p.bc_uvw + 3 * s.sl + 1);
+    s.w = (float)__ldg(p.bc_uvw + 3 * s.sl + 2);
+    return s;
+}
+
 // Boundary conditions of a fluid node whose populations are gathered
 // (pulled, bounced back): Zou-He faces, moving walls, the reference's wall,
 // periodic and symmetry copies.  keep_macro / zero_v report the reference's
 // 3D inlet and 2D outlet special cases.
 template <int Q, int ST, bool PHYS, bool WRAP, class G>
 __device__ __forceinline__ void apply_bc(typename Store<ST>::R (&f)[Q], uint32_t w, int node, const StepParams &p,
-                                         const G &g, bool &keep_macro, bool &zero_v) {
+                                         const G &g, bool &keep_macro, bool &zero_v, const SlotInfo *pre = nullptr) {
     using R = typename Store<ST>::R;
     using L = Lat<Q>;
     keep_macro = false;
     zero_v = false;
     if (w & W_SPECIAL) {
-        const int sl = __ldg(p.slot + node);
-        const R u0 = (R)__ldg(p.bc_uvw + 3 * sl), v0 = (R)__ldg(p.bc_uvw + 3 * sl + 1),
-                w0 = (R)__ldg(p.bc_uvw + 3 * sl + 2);
+        const int sl = pre ? pre->sl : __ldg(p.slot + node);
+        const R u0 = pre ? (R)pre->u : (R)__ldg(p.bc_uvw + 3 * sl), v0 = pre ? (R)pre->v : (R)__ldg(p.bc_uvw + 3 * sl + 1),
+                w0 = pre ? (R)pre->w : (R)__ldg(p.bc_uvw + 3 * sl + 2);
         if constexpr (!PHYS) {
-            const unsigned long long mk = __ldg(p.bc_mask + sl);
+            const unsigned long long mk = pre ? pre->mask : __ldg(p.bc_mask + sl);
             // curved walls: the interpolated values come from the read buffer
             // only, so they are formed before any condition changes f
             R cv[Q];
@@ -401,11 +420,11 @@ __device__ __forceinline__ void apply_bc(typename Store<ST>::R (&f)[Q], uint32_t
 
 template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G>
 __device__ __forceinline__ void update_node(typename Store<ST>::R (&f)[Q], uint32_t w, int node,
-                                            const StepParams &p, const G &g) {
+                                            const StepParams &p, const G &g, const SlotInfo *pre = nullptr) {
     using R = typename Store<ST>::R;
     using L = Lat<Q>;
     bool keep_macro, zero_v;
-    apply_bc<Q, ST, PHYS, WRAP, G>(f, w, node, p, g, keep_macro, zero_v);
+    apply_bc<Q, ST, PHYS, WRAP, G>(f, w, node, p, g, keep_macro, zero_v, pre);
 
     R rho = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll

@@ -515,7 +515,8 @@ __device__ __forceinline__ void h_gather(const G &g, uint32_t w, const typename 
 // Boundary closures, moments, the macroscopic store and the collision of a
 // fluid node whose streamed populations are in h (storage units).
 template <int Q, int COLL, int ST, bool PHYS, bool WRAP, class G>
-__device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int node, uint32_t w, f1 (&h)[Q]) {
+__device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int node, uint32_t w, f1 (&h)[Q],
+                                         const SlotInfo *pre = nullptr) {
     using L = Lat<Q>;
     using T = typename Store<ST>::T;
     constexpr bool F16 = ST == LBM_STORE_F16S || ST == LBM_STORE_F16C;
@@ -528,16 +529,17 @@ __device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int no
         // deviations keep their digits (an f-space detour rounds every
         // population to FP32 near w_d, 1e-4 of a slow flow's velocity)
         if (w & W_SPECIAL) {
-            const int sl = __ldg(p.slot + node);
-            const int kind = __ldg(p.bc_kind + sl);
+            const int sl = pre ? pre->sl : __ldg(p.slot + node);
+            const int kind = pre ? pre->kind : __ldg(p.bc_kind + sl);
             if (kind & (BCK_MOVING | BCK_ACTIVE)) {
-                const float u0 = (float)__ldg(p.bc_uvw + 3 * sl), v0 = (float)__ldg(p.bc_uvw + 3 * sl + 1),
-                            w0 = (float)__ldg(p.bc_uvw + 3 * sl + 2);
+                const float u0 = pre ? pre->u : (float)__ldg(p.bc_uvw + 3 * sl),
+                            v0 = pre ? pre->v : (float)__ldg(p.bc_uvw + 3 * sl + 1),
+                            w0 = pre ? pre->w : (float)__ldg(p.bc_uvw + 3 * sl + 2);
                 float hv[Q];
 #pragma unroll
                 for (int d = 0; d < Q; ++d) hv[d] = h[d].v;
                 if (kind & BCK_MOVING) {
-                    bc_moving_wall_h<Q>(hv, __ldg(p.bc_mask + sl), (float)p.rho0, S, u0, v0, w0);
+                    bc_moving_wall_h<Q>(hv, pre ? pre->mask : __ldg(p.bc_mask + sl), (float)p.rho0, S, u0, v0, w0);
                 } else if (kind & (BCK_EXTRAP1 | BCK_EXTRAP2 | BCK_HE)) {
                     phys_open_outlet<Q, ST, WRAP, G, float>(
                         hv, kind, sl, node, p, g, [](const T *q, int) { return h_raw<ST>(q); },
@@ -560,7 +562,7 @@ __device__ __forceinline__ void h_finish(const StepParams &p, const G &g, int no
             float f[Q];
 #pragma unroll
             for (int d = 0; d < Q; ++d) f[d] = fmaf(h[d].v, invS, sigma * p.shift[d]);
-            apply_bc<Q, ST, PHYS, WRAP, G>(f, w, node, p, g, keep, zv);
+            apply_bc<Q, ST, PHYS, WRAP, G>(f, w, node, p, g, keep, zv, pre);
 #pragma unroll
             for (int d = 0; d < Q; ++d) h[d] = f1((f[d] - sigma * p.shift[d]) * S);
         }
@@ -707,6 +709,49 @@ __device__ __forceinline__ void h_node_w(const StepParams &p, const G &g, int x,
 
 
 
+// Moments, the macroscopic store and the collision of two nodes' streamed
+// populations on packed lanes; neither is a boundary-slot node, a solid one's
+// lane carries zeros.
+template <int Q, int COLL, int ST, bool PHYS>
+__device__ __forceinline__ void h_pair_relax(const StepParams &p, int node0, int node1, bool fl0, bool fl1,
+                                             f2 (&h)[Q]) {
+    using L = Lat<Q>;
+    constexpr bool F16 = ST == LBM_STORE_F16S || ST == LBM_STORE_F16C;
+    const float sigma = p.sigma;
+    const float S = F16 ? p.scale : 1.f;
+    const float invS = F16 ? p.inv_scale : 1.f;
+    f2 sum = h[0], jx = 0.f, jy = 0.f, jz = 0.f;
+#pragma unroll
+    for (int d = 1; d < Q; ++d) {
+        sum += h[d];
+        if (L::cx(d) == 1) jx += h[d]; else if (L::cx(d) == -1) jx -= h[d];
+        if (L::cy(d) == 1) jy += h[d]; else if (L::cy(d) == -1) jy -= h[d];
+        if (L::cz(d) == 1) jz += h[d]; else if (L::cz(d) == -1) jz -= h[d];
+    }
+    const f2 rms = F16 ? sum * f2(invS) : sum;
+    const f2 rho = rms + f2(sigma);
+    // a solid lane's rho is sigma + 0 = 1 (F16S/F32 shifted) or 0 (unshifted);
+    // guard the reciprocal, its results are discarded
+    const float r0 = fl0 ? rho.v.x : 1.f, r1 = fl1 ? rho.v.y : 1.f;
+    const f2 sc(invS / r0, invS / r1);
+    const f2 ux = fma2(jx, sc, f2(p.gshift_f)), uy = jy * sc, uz = jz * sc;
+    if (p.write_macro) {
+        if (fl0) {
+            p.rho[node0] = rho.v.x;
+            p.ux[node0] = ux.v.x;
+            p.uy[node0] = uy.v.x;
+            p.uz[node0] = uz.v.x;
+        }
+        if (fl1) {
+            p.rho[node1] = rho.v.y;
+            p.ux[node1] = ux.v.y;
+            p.uy[node1] = uy.v.y;
+            p.uz[node1] = uz.v.y;
+        }
+    }
+    collide_x2<Q, COLL, ST, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
+}
+
 // Two nodes updated together, the second dn nodes and dp elements after the
 // first: each gathers by its own flag word (pull, or its own opposite
 // population across a blocked link), then moments and collision run on packed
@@ -766,36 +811,7 @@ __device__ __forceinline__ void h_pair_w(const StepParams &p, const G &g, bool i
         }
         h[d] = f2(a0, a1);
     }
-    f2 sum = h[0], jx = 0.f, jy = 0.f, jz = 0.f;
-#pragma unroll
-    for (int d = 1; d < Q; ++d) {
-        sum += h[d];
-        if (L::cx(d) == 1) jx += h[d]; else if (L::cx(d) == -1) jx -= h[d];
-        if (L::cy(d) == 1) jy += h[d]; else if (L::cy(d) == -1) jy -= h[d];
-        if (L::cz(d) == 1) jz += h[d]; else if (L::cz(d) == -1) jz -= h[d];
-    }
-    const f2 rms = F16 ? sum * f2(invS) : sum;
-    const f2 rho = rms + f2(sigma);
-    // a solid lane's rho is sigma + 0 = 1 (F16S/F32 shifted) or 0 (unshifted);
-    // guard the reciprocal, its results are discarded
-    const float r0 = fl0 ? rho.v.x : 1.f, r1 = fl1 ? rho.v.y : 1.f;
-    const f2 sc(invS / r0, invS / r1);
-    const f2 ux = fma2(jx, sc, f2(p.gshift_f)), uy = jy * sc, uz = jz * sc;
-    if (p.write_macro) {
-        if (fl0) {
-            p.rho[node0] = rho.v.x;
-            p.ux[node0] = ux.v.x;
-            p.uy[node0] = uy.v.x;
-            p.uz[node0] = uz.v.x;
-        }
-        if (fl1) {
-            p.rho[node1] = rho.v.y;
-            p.ux[node1] = ux.v.y;
-            p.uy[node1] = uy.v.y;
-            p.uz[node1] = uz.v.y;
-        }
-    }
-    collide_x2<Q, COLL, ST, PHYS>(h, rho, rms, ux, uy, uz, p, sigma, S);
+    h_pair_relax<Q, COLL, ST, PHYS>(p, node0, node1, fl0, fl1, h);
     if (in_row) {
 #pragma unroll
         for (int d = 0; d < Q; ++d) {
