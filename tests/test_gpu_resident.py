@@ -84,3 +84,32 @@ def test_calls_of_several_lengths(monkeypatch, storage):
     assert np.abs(f - f1).max() <= tol
     for a, b in zip(mac[:3], mac1[:3]):
         assert np.abs(a - b).max() <= 9 * tol
+
+
+def test_handles_of_two_threads():
+    """Two threads step their own lattices at the same time, each lattice as
+    wide as the GPU: every launch runs to its end and gives the state of a run
+    alone."""
+    import threading
+    cases = [cavity(512, 300, N.MRT, N.MODE_PHYSICS, N.STORE_F32), cavity(300, 400, N.BGKW, N.MODE_REFERENCE, N.STORE_F32)]
+    out = {}
+
+    def run(k, tag):
+        lat, args = cases[k]
+        with Solver(lat, args) as s:
+            s.init(*rest(lat.num_nodes))
+            for _ in range(20):
+                s.step(50)
+            s.step(10, write_macro=True)
+            out[tag, k] = s.get_state(), s.macro()
+    for k in range(2):
+        run(k, "alone")
+    threads = [threading.Thread(target=run, args=(k, "together")) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        assert np.array_equal(out["alone", k][0], out["together", k][0])
+        for a, b in zip(out["alone", k][1], out["together", k][1]):
+            assert np.array_equal(a, b)
