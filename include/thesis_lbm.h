@@ -340,7 +340,10 @@ const char *lbm_kernel_warning(lbm_handle h);
  * from deviations from the rest state).  This function has no
  * counterpart in the reference. */
 int lbm_autotune(lbm_handle h, int trial_steps, int *block, int *hint, int *pred);
-/* The knobs of the handle's step kernel (defaults 128, 0, 0). */
+/* The knobs of the handle's step kernel: 128, 0, 0 unless tuned, requested or
+ * set by the rule for physics-mode 3D lattices of 200,000 nodes and more (the
+ * block that fits a row, 36 warps per SM, three nodes along z with 16-bit
+ * storage of a million nodes and more). */
 int lbm_kernel_config(lbm_handle h, int *block, int *hint, int *pred);
 
 /* Compile (no GPU needed, nothing is loaded) the run-time specialised step

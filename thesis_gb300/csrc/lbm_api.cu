@@ -1245,7 +1245,10 @@ int lbm_autotune(lbm_handle H, int trial_steps, int *block, int *hint, int *pred
                         {128, 0, 0, 1, 6, 0, 1}};
         vs.insert(vs.end(), pv, pv + 4);
     }
+    // first the kernel in place: its block may be one fitted to the row, which
+    // the list does not hold
     std::vector<JitStepKey> cand;
+    if (fspace_ok || H->jit_key.hspace || H->jit_key.pair) cand.push_back(H->jit_key);
     for (const V &v : vs) {
         JitStepKey k = H->jit_key;
         k.block = v.block;
