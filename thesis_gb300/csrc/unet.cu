@@ -230,8 +230,7 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const bf16 *__restrict__ dpr
 struct V8 {
     float v[8];
 };
-__device__ __forceinline__ V8 ld8(const bf16 *p) {
-    const uint4 r = __ldg((const uint4 *)p);
+__device__ __forceinline__ V8 unpack8(const uint4 &r) {
     const __nv_bfloat162 *h = (const __nv_bfloat162 *)&r;
     V8 o;
 #pragma unroll
@@ -242,6 +241,7 @@ __device__ __forceinline__ V8 ld8(const bf16 *p) {
     }
     return o;
 }
+__device__ __forceinline__ V8 ld8(const bf16 *p) { return unpack8(__ldg((const uint4 *)p)); }
 __device__ __forceinline__ void st8(bf16 *p, const V8 &a) {
     uint4 r;
     __nv_bfloat162 *h = (__nv_bfloat162 *)&r;
@@ -250,15 +250,35 @@ __device__ __forceinline__ void st8(bf16 *p, const V8 &a) {
     *(uint4 *)p = r;
 }
 
-// 2x2 average pooling: out[n, y, x, c] = mean of in[n, 2y+i, 2x+j, c]
-__global__ void pool_kernel(const bf16 *in, int in_cs, int in_co, bf16 *out, int C, int B, int Ho, int Wo) {
-    const int G = C / 8, total = B * Ho * Wo * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int g = i % G, p = i / G, x = p % Wo, ny = p / Wo, y = ny % Ho, n = ny / Ho;
-        const int Wi = 2 * Wo;
-        const size_t b = (((size_t)n * 2 * Ho + 2 * y) * Wi + 2 * x) * in_cs + in_co + 8 * g;
-        const V8 a = ld8(in + b), c = ld8(in + b + in_cs), d = ld8(in + b + (size_t)Wi * in_cs),
-                 e = ld8(in + b + (size_t)Wi * in_cs + in_cs);
+// The resampling kernels below walk the items (8 channels of one node) of the
+// smaller of their two images, 2^lg channel groups to a pixel: item i is pixel
+// i >> lg, at row (n, y) and column x, and its 2x2 pixels of the larger image
+// start at row 2 (n, y), column 2x, as an image's height is even.  That leaves
+// one division per four pixels where the groups, image, row and column of each
+// pixel were divided out.  16 x 256 x 1024, all levels of a step: upsampling
+// 119 -> 91 us, the pooling and skip gradient 313 -> 293, the upsampling's
+// gradient 149 -> 147: what is left is DRAM at 0.6 of its copy rate, as the
+// joined tensors are read and written half a line at a time.
+struct Quad {
+    size_t p;  // the first of the four pixels of the larger image
+    int g;     // the item's channel group
+    __device__ __forceinline__ Quad(unsigned i, int lg, unsigned W) {
+        const unsigned q = i >> lg, ny = q / W, x = q - ny * W;
+        p = (size_t)(2 * ny) * (2 * W) + 2 * x;
+        g = (int)(i & ((1u << lg) - 1));
+    }
+    // pixel k = 0..3: left and right of the upper row, then of the lower
+    __device__ __forceinline__ size_t at(int k, unsigned W) const { return p + (k & 1) + (k >> 1) * (size_t)(2 * W); }
+};
+
+// 2x2 average pooling of in (its pixels in_cs channels apart) to Ho x Wo;
+// total = items of the output
+__global__ void pool_kernel(const bf16 *in, int in_cs, int in_co, bf16 *out, int lg, unsigned total, unsigned Wo) {
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const Quad q(i, lg, Wo);
+        const bf16 *b = in + in_co + 8 * q.g;
+        const V8 a = ld8(b + q.at(0, Wo) * in_cs), c = ld8(b + q.at(1, Wo) * in_cs), d = ld8(b + q.at(2, Wo) * in_cs),
+                 e = ld8(b + q.at(3, Wo) * in_cs);
         V8 o;
 #pragma unroll
         for (int k = 0; k < 8; ++k) o.v[k] = 0.25f * (a.v[k] + c.v[k] + d.v[k] + e.v[k]);
@@ -266,14 +286,14 @@ __global__ void pool_kernel(const bf16 *in, int in_cs, int in_co, bf16 *out, int
     }
 }
 
-// nearest x2 upsampling into channels [out_co, out_co + C) of out
-__global__ void up_kernel(const bf16 *in, int C, bf16 *out, int out_cs, int out_co, int B, int Ho, int Wo) {
-    const int G = C / 8, total = B * Ho * Wo * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int g = i % G, p = i / G, x = p % Wo, ny = p / Wo, y = ny % Ho, n = ny / Ho;
-        const int Hi = Ho / 2, Wi = Wo / 2;
-        *(uint4 *)(out + (size_t)p * out_cs + out_co + 8 * g) =
-            __ldg((const uint4 *)(in + (((size_t)n * Hi + y / 2) * Wi + x / 2) * C + 8 * g));
+// nearest x2 upsampling into channels [out_co, out_co + C) of out; total =
+// items of the input, W its width
+__global__ void up_kernel(const bf16 *in, bf16 *out, int out_cs, int out_co, int lg, unsigned total, unsigned W) {
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const Quad q(i, lg, W);
+        const uint4 v = __ldg((const uint4 *)(in + (size_t)i * 8));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *(uint4 *)(out + q.at(k, W) * out_cs + out_co + 8 * q.g) = v;
     }
 }
 
@@ -346,37 +366,43 @@ __global__ void __launch_bounds__(256) relu_bwd_kernel(const bf16 *g, int g_cs, 
     bs.flush(C, rows);
 }
 
-// dpre = (pool gradient + skip gradient) masked by ReLU, at full resolution
+// dpre = (pool gradient + skip gradient) masked by ReLU, at full resolution;
+// total = items of the pooled gradient, W its width
 __global__ void __launch_bounds__(256) pool_skip_bwd_kernel(const bf16 *gpool, const bf16 *gskip, int s_cs, int s_co,
                                                             const bf16 *act, int a_cs, int a_co, bf16 *dpre, int C,
-                                                            int B, int H, int W, float *rows) {
+                                                            int lg, unsigned total, unsigned W, float *rows) {
     BiasSum bs;
-    const int G = C / 8, total = B * H * W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int v = i % G, p = i / G, x = p % W, ny = p / W, y = ny % H, n = ny / H;
-        const V8 gp = ld8(gpool + (((size_t)n * (H / 2) + y / 2) * (W / 2) + x / 2) * C + 8 * v);
-        const V8 gs = ld8(gskip + (size_t)p * s_cs + s_co + 8 * v);
-        const V8 a = ld8(act + (size_t)p * a_cs + a_co + 8 * v);
-        V8 o;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const Quad q(i, lg, W);
+        const V8 gp = ld8(gpool + (size_t)i * 8);
+        uint4 gs[4], a[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o.v[k] = a.v[k] > 0.f ? 0.25f * gp.v[k] + gs.v[k] : 0.f;
-        st8(dpre + (size_t)i * 8, o);
-        bs.add(o);
+        for (int k = 0; k < 4; ++k) gs[k] = __ldg((const uint4 *)(gskip + q.at(k, W) * s_cs + s_co + 8 * q.g));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = __ldg((const uint4 *)(act + q.at(k, W) * a_cs + a_co + 8 * q.g));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const V8 s = unpack8(gs[k]), m = unpack8(a[k]);
+            V8 o;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) o.v[c] = m.v[c] > 0.f ? 0.25f * gp.v[c] + s.v[c] : 0.f;
+            st8(dpre + q.at(k, W) * C + 8 * q.g, o);
+            bs.add(o);
+        }
     }
     bs.flush(C, rows);
 }
 
-// dpre at low resolution = sum of the 2x2 upsampled gradient, masked by ReLU
+// dpre at low resolution = sum of the 2x2 upsampled gradient, masked by ReLU;
+// total = items of dpre, W its width
 __global__ void __launch_bounds__(256) up_bwd_kernel(const bf16 *gup, int g_cs, int g_co, const bf16 *act, bf16 *dpre,
-                                                     int C, int B, int H, int W, float *rows) {
+                                                     int C, int lg, unsigned total, unsigned W, float *rows) {
     BiasSum bs;
-    const int G = C / 8, total = B * H * W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int v = i % G, p = i / G, x = p % W, ny = p / W, y = ny % H, n = ny / H;
-        const int W2 = 2 * W;
-        const size_t b = (((size_t)n * 2 * H + 2 * y) * W2 + 2 * x) * g_cs + g_co + 8 * v;
-        const V8 a = ld8(gup + b), c = ld8(gup + b + g_cs), d = ld8(gup + b + (size_t)W2 * g_cs),
-                 e = ld8(gup + b + (size_t)W2 * g_cs + g_cs);
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const Quad q(i, lg, W);
+        const bf16 *b = gup + g_co + 8 * q.g;
+        const V8 a = ld8(b + q.at(0, W) * g_cs), c = ld8(b + q.at(1, W) * g_cs), d = ld8(b + q.at(2, W) * g_cs),
+                 e = ld8(b + q.at(3, W) * g_cs);
         const V8 m = ld8(act + (size_t)i * 8);
         V8 o;
 #pragma unroll
@@ -452,10 +478,20 @@ __global__ void adam_kernel(float *p, const float *g, float *m, float *v, long l
     }
 }
 
-// BF16 copies of one layer's FP32 weights [9][cout][cin]: w and the data-
-// gradient form wt[tap'][ci][co] = w[8 - tap'][co][ci]
-__global__ void weights_kernel(const float *p, bf16 *w, bf16 *wt, int cout, int cin) {
-    const int total = 9 * cout * cin;
+// BF16 copies of the FP32 weights [9][cout][cin] of every layer (row blockIdx.y
+// of the grid): w and the data-gradient form wt[tap'][ci][co] =
+// w[8 - tap'][co][ci].  One launch: a launch per layer was 3 us each, 59 us for
+// the 19 layers of the 4-level network (a training step of 8 images of
+// 64 x 256, 3 levels, base 16: 952 -> 897 us).
+struct WeightPlan {
+    bf16 *w[MAX_LAYERS], *wt[MAX_LAYERS];
+    int cout[MAX_LAYERS], cin[MAX_LAYERS];
+    long long off[MAX_LAYERS];
+};
+__global__ void weights_kernel(const __grid_constant__ WeightPlan plan, const float *params) {
+    const int k = blockIdx.y, cout = plan.cout[k], cin = plan.cin[k], total = 9 * cout * cin;
+    const float *p = params + plan.off[k];
+    bf16 *w = plan.w[k], *wt = plan.wt[k];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int ci = i % cin, co = (i / cin) % cout, tap = i / (cin * cout);
         const bf16 b = __float2bfloat16(p[i]);
@@ -485,6 +521,9 @@ int sum_grid_for(long long n) {
     const long long b = (n + 255) / 256;
     return (int)std::max(1ll, std::min<long long>(b, unet_tc::BIAS_ROWS));
 }
+
+// log2 of the channel groups of C = 16, 32 or 64 channels
+int log2_groups(int C) { return C == 16 ? 1 : C == 32 ? 2 : 3; }
 
 int grid_for(long long n, int block = 256) {
     long long b = (n + block - 1) / block;
@@ -944,9 +983,19 @@ void wgrad(lbm_unet_s *u, const Layer &l, const Act &in, const bf16 *dpre, int B
 }
 
 void refresh_weights(lbm_unet_s *u) {
-    for (const Layer &l : u->L)
-        weights_kernel<<<grid_for(9LL * l.cout * l.cin), 256, 0, u->stream>>>(u->params + l.w_off, l.w, l.wt, l.cout,
-                                                                               l.cin);
+    WeightPlan plan;
+    int most = 0;
+    for (int k = 0; k < (int)u->L.size(); ++k) {
+        const Layer &l = u->L[k];
+        plan.w[k] = l.w;
+        plan.wt[k] = l.wt;
+        plan.cout[k] = l.cout;
+        plan.cin[k] = l.cin;
+        plan.off[k] = (long long)l.w_off;
+        most = std::max(most, 9 * l.cout * l.cin);
+    }
+    const dim3 grid((unsigned)std::min((most + 255) / 256, 96), (unsigned)u->L.size());
+    weights_kernel<<<grid, 256, 0, u->stream>>>(plan, u->params);
 }
 
 // forward pass on the batch in x0; FP32 output in out32
@@ -963,17 +1012,17 @@ void forward(lbm_unet_s *u, int B) {
         const Act skip = view(u->cat[l], ch_up(u, l), ch(u, l));
         cv(enc_b(l), u->e_a[l], skip, l);
         const long long n = (long long)B * H_of(u, l + 1) * W_of(u, l + 1) * ch(u, l);
-        pool_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(skip.p, skip.cs, skip.co, u->p[l].p, ch(u, l), B,
-                                                          H_of(u, l + 1), W_of(u, l + 1));
+        pool_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(skip.p, skip.cs, skip.co, u->p[l].p, log2_groups(ch(u, l)),
+                                                          (unsigned)(n / 8), W_of(u, l + 1));
         x = u->p[l];
     }
     cv(bott_a(u), x, u->ba, NL);
     cv(bott_b(u), u->ba, u->bb, NL);
     Act prev = u->bb;
     for (int l = NL - 1; l >= 0; --l) {
-        const long long n = (long long)B * H_of(u, l) * W_of(u, l) * prev.C;
-        up_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(prev.p, prev.C, u->cat[l].p, u->cat[l].cs, 0, B, H_of(u, l),
-                                                        W_of(u, l));
+        const long long n = (long long)B * H_of(u, l + 1) * W_of(u, l + 1) * prev.C;
+        up_kernel<<<grid_for(n / 8), 256, 0, u->stream>>>(prev.p, u->cat[l].p, u->cat[l].cs, 0, log2_groups(prev.C),
+                                                        (unsigned)(n / 8), W_of(u, l + 1));
         cv(dec_a(u, l), u->cat[l], u->d_a[l], l);
         cv(dec_b(u, l), u->d_a[l], u->d_b[l], l);
         prev = u->d_b[l];
@@ -1029,16 +1078,18 @@ void backward(lbm_unet_s *u, int B) {
     };
     auto pool_skip = [&](int k, const Act &gpool, const Act &gskip, const Act &act, int C, int lev) {
         bf16 *next = other();
-        const int grid = plan.rows[k] = sum_grid_for(npix(lev) * C / 8);
+        const long long items = npix(lev + 1) * C / 8;
+        const int grid = plan.rows[k] = sum_grid_for(items);
         pool_skip_bwd_kernel<<<grid, 256, 0, u->stream>>>(gpool.p, gskip.p, gskip.cs, gskip.co, act.p, act.cs, act.co, next,
-                                                          C, B, H_of(u, lev), W_of(u, lev), rows(k));
+                                                          C, log2_groups(C), (unsigned)items, W_of(u, lev + 1), rows(k));
         cur = next;
     };
     auto up_bwd = [&](int k, const Act &gup, const Act &act, int C, int lev) {
         bf16 *next = other();
-        const int grid = plan.rows[k] = sum_grid_for(npix(lev) * C / 8);
-        up_bwd_kernel<<<grid, 256, 0, u->stream>>>(gup.p, gup.cs, gup.co, act.p, next, C, B, H_of(u, lev), W_of(u, lev),
-                                                   rows(k));
+        const long long items = npix(lev) * C / 8;
+        const int grid = plan.rows[k] = sum_grid_for(items);
+        up_bwd_kernel<<<grid, 256, 0, u->stream>>>(gup.p, gup.cs, gup.co, act.p, next, C, log2_groups(C), (unsigned)items,
+                                                   W_of(u, lev), rows(k));
         cur = next;
     };
     wg(out_layer(u), u->d_b[0], 0);
