@@ -321,7 +321,8 @@ int lbm_kernel_variant(lbm_handle h);
  * instead (LBM_ERR_CUDA).  No counterpart in the reference. */
 const char *lbm_kernel_warning(lbm_handle h);
 
-/* Autotuner of the run-time specialised kernel: builds its variants (one
+/* Autotuner of the run-time specialised kernel: takes the kernel in place and
+ * builds its variants (one
  * node per thread with blocks of 128 or 256 threads along x, plain or
  * L2-256-byte-prefetching loads, bounce-back by selected address or by
  * predicated loads; and, for even n with F32/F16S storage, two nodes per
