@@ -406,7 +406,9 @@ static int setup_resident(lbm_handle_s *H) {
     // and the host reads it without a copy
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&H->res_err, sizeof(unsigned), cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&H->res_err_d, (void *)H->res_err, 0);
-    if (e == cudaSuccess) e = cudaMemset(H->res_mail, 0, bytes);
+    // awaited on the handle's stream: a clearing that runs after the first messages would lose them
+    if (e == cudaSuccess) e = cudaMemsetAsync(H->res_mail, 0, bytes, H->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();  // no room for the messages: a launch per step
         return LBM_OK;
@@ -633,9 +635,11 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
         std::vector<double> qt((size_t)q * H->nslots, 0.5);
         if (H->nslots) e = cudaMemcpy(H->bcq, qt.data(), sizeof(double) * qt.size(), cudaMemcpyHostToDevice);
     }
-    if (e == cudaSuccess) e = cudaMemset(H->pux, 0, sizeof(float) * N);
-    if (e == cudaSuccess) e = cudaMemset(H->puy, 0, sizeof(float) * N);
-    if (e == cudaSuccess) e = cudaMemset(H->puz, 0, sizeof(float) * N);
+    // on the handle's stream, and awaited: the default stream may hold work of
+    // others, and a clearing that runs after the first use would undo it
+    for (float *f : {H->pux, H->puy, H->puz})
+        if (e == cudaSuccess) e = cudaMemsetAsync(f, 0, sizeof(float) * N, H->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) {
         free_handle(H);
         return fail(LBM_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
