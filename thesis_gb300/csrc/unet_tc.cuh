@@ -500,11 +500,11 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
             if (!ok) {
                 *abort_flag = 1;
                 atomicExch(err, 1);
-                // the copies in flight land before the CTA leaves: the last
-                // use of each stage
-                for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
-                    mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
             }
+            // the copies in flight land before the CTA leaves, whichever role
+            // gave up: the last use of each stage
+            for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
+                mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -550,10 +550,14 @@ conv3x3_tc_kernel(const __grid_constant__ CUtensorMap tin, int cin, const __nv_b
         if (!ok) {
             *abort_flag = 1;
             if (leader) atomicExch(err, 1);
-            // MMAs complete in order: the last commit covers them all
-            if (committed > 0)
-                mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1));
         }
+        // no MMA or commit is in flight when the tensor memory is freed,
+        // whichever role gave up: they complete in order, so the last commits
+        // cover them all
+        if (committed > 0)
+            mbar_wait(empty0 + 8 * (uint32_t)((committed - 1) % NS), (uint32_t)(((committed - 1) / NS) & 1));
+        const int done = committed / nch;  // finished tiles
+        if (done > 0) mbar_wait(accf0 + 8 * (uint32_t)((done - 1) % NA), (uint32_t)(((done - 1) / NA) & 1));
         __syncwarp();
     } else {
         // epilogue warps: tile k from accumulator k % NA, 32 columns at a time
@@ -722,11 +726,10 @@ conv3x3_rows_kernel(const __grid_constant__ CUtensorMap tin, const __grid_consta
             if (!ok) {
                 *abort_flag = 1;
                 atomicExch(err, 1);
-                // the copies in flight land before the CTA leaves: the last
-                // use of each slot
-                for (int j = issued > nr ? issued - nr : 0; j < issued; ++j)
-                    mbar_wait(full0 + 8 * (uint32_t)(j % nr), (uint32_t)((j / nr) & 1));
             }
+            // as in conv3x3_tc_kernel: the last use of each slot
+            for (int j = issued > nr ? issued - nr : 0; j < issued; ++j)
+                mbar_wait(full0 + 8 * (uint32_t)(j % nr), (uint32_t)((j / nr) & 1));
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -737,8 +740,7 @@ conv3x3_rows_kernel(const __grid_constant__ CUtensorMap tin, const __grid_consta
         Ring<NA> ac;
         const uint32_t tap_step = (uint32_t)(KGall * COUT);
         int w0 = 0, w1 = 0, w2 = 0;  // slots of the tile's rows y - 1, y, y + 1
-        int last_slot = -1;          // the last commit's barrier and phase
-        uint32_t last_round = 0;
+        int tiles = 0;               // tiles issued and committed
         auto take = [&]() -> bool {  // the next row of the ring becomes w2
             w0 = w1;
             w1 = w2;
@@ -784,17 +786,16 @@ conv3x3_rows_kernel(const __grid_constant__ CUtensorMap tin, const __grid_consta
                     }
                     mma_commit(accf0 + 8 * ac.slot);
                 }
-                last_slot = w0;
-                last_round = st.round - (w0 >= st.slot ? 1u : 0u);
+                ++tiles;
             }
             walk.advance(seg);
         }
         if (!ok) {
             *abort_flag = 1;
             if (leader) atomicExch(err, 1);
-            // MMAs complete in order: the last commit covers them all
-            if (last_slot >= 0) mbar_wait(empty0 + 8 * (uint32_t)last_slot, last_round & 1);
         }
+        // as in conv3x3_tc_kernel; a tile's last commit is its accumulator's
+        if (tiles > 0) mbar_wait(accf0 + 8 * (uint32_t)((tiles - 1) % NA), (uint32_t)(((tiles - 1) / NA) & 1));
         __syncwarp();
     } else {
         // epilogue warps: tile k from accumulator k % NA, 32 columns at a time
@@ -978,10 +979,10 @@ wgrad_tc_kernel(const __grid_constant__ CUtensorMap tdp, const __grid_constant__
         if (!ok) {
             abort_flag = 1;
             atomicExch(err, 1);
-            // the copies in flight land before the CTA leaves
-            for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
-                mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
         }
+        // the copies in flight land before the CTA leaves, whichever role gave up
+        for (int j = issued > NS ? issued - NS : 0; j < issued; ++j)
+            mbar_wait(full0 + 8 * (uint32_t)(j % NS), (uint32_t)((j / NS) & 1));
     } else if (warp == 1) {
         bool ok = true;
         const bool leader = elect_one();
