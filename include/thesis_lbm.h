@@ -312,6 +312,17 @@ long long lbm_fluid_nodes(lbm_handle h);
  * per step. */
 int lbm_kernel_variant(lbm_handle h);
 
+/* 1 where calls of several steps run on chip (see above), else 0.  A wait of
+ * that kernel for a neighbouring tile's message is bounded; if one gives up,
+ * the state is lost: lbm_step and every function that reads the state or the
+ * fields return LBM_ERR_CUDA until lbm_init, lbm_set_state or
+ * lbm_set_populations brings a new one. */
+int lbm_on_chip(lbm_handle h);
+
+/* For tests: `polls` of a message after the first, before its wait gives up
+ * (negative: the default, seconds). */
+int lbm_test_on_chip(lbm_handle h, int polls);
+
 /* Empty when the handle runs the kernel lbm_create meant to use; otherwise
  * why it fell back (the run-time specialised kernel could not be built, for
  * example without NVRTC or the toolkit headers it compiles against), in

@@ -50,3 +50,36 @@ def test_default_stream_busy():
     finally:
         stop.set()
         t.join()
+
+
+def test_wait_that_gives_up():
+    """A wait that runs out (one poll allowed) leaves the kernel at once; every
+    reader and the next step report it, and a new state ends it."""
+    lat, args = cavity(256, 200)
+    nn = lat.num_nodes
+    box = (0, 10, 0, 10, 0, 1)
+    with Solver(lat, args) as s:
+        assert s.on_chip
+        s.init(*rest(nn))
+        s.step(20)
+        good = s.get_state()
+        s.step(30)
+        later = s.get_state()
+        readers = [s.get_state, s.populations, s.macro, s.norms, s.residual, s.macro_diff, s.residual_l2,
+                   s.residual_fd_rel_diff, lambda: s.momentum_exchange(box), lambda: s.step(1), lambda: s.step(20)]
+        if (np.asarray(lat.bc[:, 5]) > 0).any():
+            readers.append(lambda: s.reference_drag_lift(int(lat.bc[:, 5].max()), np.zeros(nn), np.zeros(nn)))
+        for renew in (lambda: s.set_state(good), lambda: (s.init(*rest(nn)), s.step(20))):
+            N.check(s._lib.lbm_test_on_chip(s._h, 0))
+            s.step(30)
+            for read in readers:
+                with pytest.raises(N.LbmError) as e:
+                    read()
+                assert e.value.code == N.LBM_ERR_CUDA
+            assert s.status == N.LBM_ERR_CUDA
+            N.check(s._lib.lbm_test_on_chip(s._h, -1))
+            renew()
+            assert s.status == N.LBM_OK
+            assert np.array_equal(s.get_state(), good)
+            s.step(30)
+            assert np.array_equal(s.get_state(), later)

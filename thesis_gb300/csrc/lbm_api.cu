@@ -130,7 +130,7 @@ struct lbm_handle_s {
     ResidentPlan res_plan;
     unsigned long long *res_mail = nullptr;
     unsigned *res_err = nullptr, *res_err_d = nullptr;  // host word and its device address
-    unsigned res_tag = 0;
+    unsigned res_tag = 0, res_polls = RESIDENT_POLLS;
     double omega = 1, omega_m = 1, gshift = 0;
     float scale = 1024.f;
 };
@@ -418,13 +418,20 @@ static int setup_resident(lbm_handle_s *H) {
     return LBM_OK;
 }
 
-// A bounded wait inside the row-staged or the on-chip kernel that gave up
-// leaves a code on the device; report it once the stream is idle.
-static int check_tma(lbm_handle_s *H) {
-    if (H->res_kern && *(volatile unsigned *)H->res_err) {
-        H->status = LBM_ERR_CUDA;
-        return fail(LBM_ERR_CUDA, "on-chip steps: a wait for a neighbouring tile gave up");
-    }
+// A bounded wait inside the on-chip or the row-staged kernel that gave up
+// leaves a code: the state is unfinished and no reader may pass it off as the
+// result.  The on-chip kernel's lies in host memory and says all there is to
+// know once the steps are over; before, that they have failed already.
+static int check_on_chip(lbm_handle_s *H) {
+    if (!H->res_err || !*(volatile unsigned *)H->res_err) return LBM_OK;
+    H->status = LBM_ERR_CUDA;
+    return fail(LBM_ERR_CUDA, "on-chip steps: a wait for a neighbouring tile gave up; the state is lost until "
+                              "lbm_init, lbm_set_state or lbm_set_populations");
+}
+
+// Both codes, for readers, once the steps are over.
+static int check_waits(lbm_handle_s *H) {
+    if (int rc = check_on_chip(H)) return rc;
     if (!H->tma_kernel) return LBM_OK;
     unsigned int err = 0;
     CUDA_TRY(cudaMemcpy(&err, H->tma_err, sizeof(err), cudaMemcpyDeviceToHost));
@@ -433,6 +440,17 @@ static int check_tma(lbm_handle_s *H) {
         return fail(LBM_ERR_CUDA, "row-staged step: a shared-memory pipeline wait timed out (code " +
                                       std::to_string(err) + ")");
     }
+    return LBM_OK;
+}
+
+// A new state ends a failure: called by the functions that bring one.
+static int clear_waits(lbm_handle_s *H) {
+    const bool on_chip = H->res_err && *(volatile unsigned *)H->res_err;
+    if (!on_chip && !H->tma_kernel) return LBM_OK;
+    CUDA_TRY(cudaDeviceSynchronize());  // the failed steps may have been queued on any stream
+    if (on_chip) *(volatile unsigned *)H->res_err = 0;
+    if (H->tma_kernel) CUDA_TRY(cudaMemset(H->tma_err, 0, sizeof(unsigned int)));
+    if (H->status == LBM_ERR_CUDA) H->status = LBM_OK;
     return LBM_OK;
 }
 
@@ -710,6 +728,7 @@ int lbm_reference_drag_lift(lbm_handle H, int boundary_id, const float *node_x, 
     std::vector<float> rho((size_t)H->N);
     CUDA_TRY(cudaMemcpyAsync(rho.data(), H->rho, sizeof(float) * H->N, cudaMemcpyDeviceToHost, H->stream));
     CUDA_TRY(cudaStreamSynchronize(H->stream));
+    if (int rc = check_waits(H)) return rc;
     // per node as gpuUpdateMacro2D stores it (FLOAT_TYPE of a double
     // product), summed in FP64
     for (size_t k = 0; k < H->id_nodes.size(); ++k) {
@@ -785,6 +804,7 @@ static int init_bc_macro(lbm_handle_s *H) {
 int lbm_init(lbm_handle H, const float *rho, const float *u, const float *v, const float *w) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     int rc;
+    if ((rc = clear_waits(H))) return rc;
     if ((rc = upload_or_fill(H->rho, rho, (float)H->P.rho, H->N, H->stream))) return rc;
     if ((rc = upload_or_fill(H->ux, u, (float)H->P.u, H->N, H->stream))) return rc;
     if ((rc = upload_or_fill(H->uy, v, (float)H->P.v, H->N, H->stream))) return rc;
@@ -888,6 +908,7 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
         a.wrap = H->jit_key.wrap;
         a.tag = H->res_tag;
         a.mail = H->res_mail;
+        a.polls = H->res_polls;
         a.err = H->res_err_d;
         const int e = resident_launch(H->res_kern, H->res_plan, a, s);
         if (e != cudaSuccess) {
@@ -906,6 +927,7 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     if (!H->initialised) return fail(LBM_ERR_INVALID, "lbm_init has not been called");
     if (nsteps < 0) return fail(LBM_ERR_INVALID, "negative step count");
+    if (int rc = check_on_chip(H)) return rc;
     cudaStream_t s = stream ? (cudaStream_t)stream : H->stream;
     if (H->res_kern && nsteps >= RESIDENT_MIN_STEPS) {
         // a stream under capture records plain launches, as it always did
@@ -940,7 +962,7 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
 int lbm_get_macro(lbm_handle H, float *rho, float *u, float *v, float *w) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     CUDA_TRY(cudaDeviceSynchronize());
-    if (int rc = check_tma(H)) return rc;
+    if (int rc = check_waits(H)) return rc;
     const size_t b = sizeof(float) * H->N;
     // queued together and awaited once
     if (rho) CUDA_TRY(cudaMemcpyAsync(rho, H->rho, b, cudaMemcpyDeviceToHost, H->stream));
@@ -954,7 +976,7 @@ int lbm_get_macro(lbm_handle H, float *rho, float *u, float *v, float *w) {
 int lbm_get_populations(lbm_handle H, double *f) {
     if (!H || !f) return fail(LBM_ERR_INVALID, "null argument");
     CUDA_TRY(cudaDeviceSynchronize());
-    if (int rc = check_tma(H)) return rc;
+    if (int rc = check_waits(H)) return rc;
     double *tmp = nullptr;
     const size_t bytes = sizeof(double) * (size_t)H->q * H->N;
     CUDA_TRY(cudaMalloc((void **)&tmp, bytes));
@@ -973,6 +995,7 @@ int lbm_get_populations(lbm_handle H, double *f) {
 
 int lbm_set_populations(lbm_handle H, const double *f) {
     if (!H || !f) return fail(LBM_ERR_INVALID, "null argument");
+    if (int rc = clear_waits(H)) return rc;
     CUDA_TRY(cudaStreamWaitEvent(H->stream, H->stepped, 0));
     // macroscopic fields as lbm_init leaves them (the params' constants);
     // the fluid nodes' values are rewritten by the next step that stores them
@@ -1033,12 +1056,14 @@ static int state_copy(lbm_handle H, void *host, bool to_host) {
 int lbm_get_state(lbm_handle H, void *state) {
     if (!H || !state) return fail(LBM_ERR_INVALID, "null argument");
     if (!H->initialised) return fail(LBM_ERR_INVALID, "lbm_init has not been called");
-    return state_copy(H, state, true);
+    const int rc = state_copy(H, state, true);
+    return rc ? rc : check_waits(H);
 }
 
 int lbm_set_state(lbm_handle H, const void *state) {
     if (!H || !state) return fail(LBM_ERR_INVALID, "null argument");
     int rc;
+    if ((rc = clear_waits(H))) return rc;
     if ((rc = upload_or_fill(H->rho, nullptr, (float)H->P.rho, H->N, H->stream))) return rc;
     if ((rc = upload_or_fill(H->ux, nullptr, (float)H->P.u, H->N, H->stream))) return rc;
     if ((rc = upload_or_fill(H->uy, nullptr, (float)H->P.v, H->N, H->stream))) return rc;
@@ -1063,7 +1088,7 @@ int lbm_macro_norms(lbm_handle H, double *out) {
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(out, H->norms, sizeof(double) * LBM_NORMS, cudaMemcpyDeviceToHost, H->stream));
     CUDA_TRY(cudaStreamSynchronize(H->stream));
-    if (int rc = check_tma(H)) return rc;
+    if (int rc = check_waits(H)) return rc;
     for (int k = 0; k < LBM_NORMS; ++k)
         if (!isfinite(out[k])) {
             H->status = LBM_DIVERGED;
@@ -1088,6 +1113,7 @@ int lbm_residual_l2(lbm_handle H, double *out) {
     cudaFreeAsync(partial, H->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("L2 residual: ") + cudaGetErrorString(e));
+    if (int rc = check_waits(H)) return rc;
     *out = sqrt(s);
     if (!(*out == *out)) {
         H->status = LBM_DIVERGED;
@@ -1120,6 +1146,7 @@ int lbm_residual_fd_rel_diff(lbm_handle H, double *out) {
     cudaFreeAsync(partial, H->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("FdRelDiff residual: ") + cudaGetErrorString(e));
+    if (int rc = check_waits(H)) return rc;
     H->fd_recorded = true;
     *out = first ? 0.0 : r[0];
     if (r[1] > 0) {
@@ -1147,6 +1174,7 @@ int lbm_momentum_exchange(lbm_handle H, const int *box, double *force) {
     cudaFreeAsync(partial, H->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("momentum exchange: ") + cudaGetErrorString(e));
+    if (int rc = check_waits(H)) return rc;
     return LBM_OK;
 }
 
@@ -1159,7 +1187,7 @@ int lbm_macro_diff(lbm_handle H, double *out) {
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(out, H->norms, sizeof(double) * 5, cudaMemcpyDeviceToHost, H->stream));
     CUDA_TRY(cudaStreamSynchronize(H->stream));
-    if (int rc = check_tma(H)) return rc;
+    if (int rc = check_waits(H)) return rc;
     if (out[4] != 0.0) {
         H->status = LBM_DIVERGED;
         return fail(LBM_DIVERGED, "non-finite macroscopic field (divergence)");
@@ -1194,6 +1222,14 @@ long long lbm_fluid_nodes(lbm_handle H) { return H ? H->fluid : -1; }
 
 int lbm_kernel_variant(lbm_handle H) {
     return H ? (H->jit_kernel ? 4 : (H->tma_kernel ? 3 : (H->pair_kernel ? 2 : 1))) : -1;
+}
+
+int lbm_on_chip(lbm_handle H) { return H ? (H->res_kern ? 1 : 0) : -1; }
+
+int lbm_test_on_chip(lbm_handle H, int polls) {
+    if (!H) return fail(LBM_ERR_INVALID, "null handle");
+    H->res_polls = polls < 0 ? RESIDENT_POLLS : (unsigned)polls;
+    return LBM_OK;
 }
 
 const char *lbm_kernel_warning(lbm_handle H) { return H ? H->kernel_warning.c_str() : ""; }

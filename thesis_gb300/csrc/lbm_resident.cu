@@ -44,7 +44,6 @@ namespace {
 
 constexpr int PLANE = 2944;              // halo'd tile nodes a buffer holds per direction (desc packs t in 12 bits)
 constexpr int MAX_COMPUTE = 512, MAX_COMM = 128, MSGS = 8;  // threads; messages per comm thread
-constexpr unsigned RES_SPIN = 1u << 22;  // polls of a wait, seconds
 
 __device__ __forceinline__ unsigned long long mail_load(const unsigned long long *q) {
     unsigned long long v;
@@ -322,6 +321,7 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
 #pragma unroll
             for (int k = 0; k < MSGS; ++k) need |= in_s[k] >= 0 ? 1u << k : 0u;
             bool bad = false;
+            unsigned look = min(a.polls, 1023u);  // the next poll after which to look at the limit and at *err
 #pragma unroll 1
             for (unsigned spin = 0; need; ++spin) {
                 unsigned long long v[MSGS];
@@ -334,9 +334,13 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
                         need &= ~(1u << k);
                         pop_from((unsigned)v[k], out[in_s[k]]);
                     }
-                if ((spin & 1023u) == 1023u && (spin >= RES_SPIN || *(volatile unsigned *)a.err)) {
-                    bad = true;
-                    break;
+                if (spin >= look) {
+                    if (!need) break;
+                    look += 1024u;
+                    if (spin >= a.polls || *(volatile unsigned *)a.err) {
+                        bad = true;
+                        break;
+                    }
                 }
             }
             if (bad) *(volatile unsigned *)a.err = 1u;

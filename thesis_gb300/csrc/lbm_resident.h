@@ -20,8 +20,11 @@ struct ResidentArgs {
     int wrap;                 // links leave the lattice by wrapping round
     unsigned tag;             // messages of this launch carry tag + 1 .. tag + steps - 1
     unsigned long long *mail; // [2][8][nx * ny] messages
-    unsigned *err;            // set when a bounded wait gave up
+    unsigned polls;           // of a message after the first, before its wait gives up
+    unsigned *err;            // set when a wait gave up
 };
+
+constexpr unsigned RESIDENT_POLLS = 1u << 22;  // seconds
 
 // A plan for an nx x ny lattice of `elem`-byte populations, or false where
 // the lattice does not fit on chip.

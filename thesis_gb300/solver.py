@@ -173,6 +173,11 @@ class Solver:
         N.check(self._lib.lbm_kernel_config(self._h, C.byref(b), C.byref(h), C.byref(p)))
         return b.value, h.value, p.value
 
+    @property
+    def on_chip(self):
+        """Whether calls of several steps run on chip (lbm_on_chip)."""
+        return self._lib.lbm_on_chip(self._h) == 1
+
     def init(self, rho=None, u=None, v=None, w=None):
         arrs = [None if a is None else np.ascontiguousarray(a, np.float32).reshape(-1) for a in (rho, u, v, w)]
         N.check(self._lib.lbm_init(self._h, *[_fptr(a) for a in arrs]))
