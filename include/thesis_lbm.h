@@ -309,7 +309,7 @@ long long lbm_fluid_nodes(lbm_handle h);
  * 440,000 nodes; F32, or F16S in physics mode; boundaries that touch only
  * the node's own populations) run in one cooperative launch with the same
  * node arithmetic (lbm_resident.cu); a stream under capture records a launch
- * per step. */
+ * per step, and so does a call whose cooperative launch the driver refuses. */
 int lbm_kernel_variant(lbm_handle h);
 
 /* 1 where calls of several steps run on chip (see above), else 0.  A wait of
@@ -320,8 +320,9 @@ int lbm_kernel_variant(lbm_handle h);
 int lbm_on_chip(lbm_handle h);
 
 /* For tests: `polls` of a message after the first, before its wait gives up
- * (negative: the default, seconds). */
-int lbm_test_on_chip(lbm_handle h, int polls);
+ * (negative: the default, seconds), and the number of launches to come that
+ * are taken as refused by the driver. */
+int lbm_test_on_chip(lbm_handle h, int polls, int refuse);
 
 /* Empty when the handle runs the kernel lbm_create meant to use; otherwise
  * why it fell back (the run-time specialised kernel could not be built, for

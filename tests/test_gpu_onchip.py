@@ -70,16 +70,33 @@ def test_wait_that_gives_up():
         if (np.asarray(lat.bc[:, 5]) > 0).any():
             readers.append(lambda: s.reference_drag_lift(int(lat.bc[:, 5].max()), np.zeros(nn), np.zeros(nn)))
         for renew in (lambda: s.set_state(good), lambda: (s.init(*rest(nn)), s.step(20))):
-            N.check(s._lib.lbm_test_on_chip(s._h, 0))
+            N.check(s._lib.lbm_test_on_chip(s._h, 0, 0))
             s.step(30)
             for read in readers:
                 with pytest.raises(N.LbmError) as e:
                     read()
                 assert e.value.code == N.LBM_ERR_CUDA
             assert s.status == N.LBM_ERR_CUDA
-            N.check(s._lib.lbm_test_on_chip(s._h, -1))
+            N.check(s._lib.lbm_test_on_chip(s._h, -1, 0))
             renew()
             assert s.status == N.LBM_OK
             assert np.array_equal(s.get_state(), good)
             s.step(30)
             assert np.array_equal(s.get_state(), later)
+
+
+def test_refused_launch():
+    """A launch that the driver refuses (here: taken as refused) leaves the
+    call to the launch-per-step kernel, with the same state and fields; the
+    next call runs on chip again."""
+    lat, args = cavity(256, 200)
+
+    def run(refuse):
+        with Solver(lat, args) as s:
+            s.init(*rest(lat.num_nodes))
+            for k in (20, 41, 7):
+                N.check(s._lib.lbm_test_on_chip(s._h, -1, refuse))
+                s.step(k, write_macro=True)
+            return [s.get_state()] + list(s.macro()) + [s.status]
+    for a, b in zip(run(0), run(1)):
+        assert np.array_equal(a, b)

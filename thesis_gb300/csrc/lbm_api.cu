@@ -131,6 +131,7 @@ struct lbm_handle_s {
     unsigned long long *res_mail = nullptr;
     unsigned *res_err = nullptr, *res_err_d = nullptr;  // host word and its device address
     unsigned res_tag = 0, res_polls = RESIDENT_POLLS;
+    int res_refuse = 0;  // launches to take as refused (lbm_test_on_chip)
     double omega = 1, omega_m = 1, gshift = 0;
     float scale = 1024.f;
 };
@@ -895,8 +896,12 @@ static int step_graph(lbm_handle_s *H, int c) {
 constexpr int RESIDENT_MIN_STEPS = 4;
 constexpr int RESIDENT_CHUNK = 8192;  // steps per launch, tens of milliseconds
 
+// Runs up to nsteps steps and returns how many: where the driver refuses a
+// launch (a stream whose context holds fewer SMs than the device, another
+// process's share), the rest of the call is the caller's, a launch per step.
 static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cudaStream_t s) {
-    for (int done = 0; done < nsteps;) {
+    int done = 0;
+    while (done < nsteps) {
         const int k = std::min(nsteps - done, RESIDENT_CHUNK);
         ResidentArgs a;
         a.p = make_params(H, H->cur, 0);
@@ -910,17 +915,19 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
         a.mail = H->res_mail;
         a.polls = H->res_polls;
         a.err = H->res_err_d;
-        const int e = resident_launch(H->res_kern, H->res_plan, a, s);
-        if (e != cudaSuccess) {
-            H->status = LBM_ERR_CUDA;
-            return fail(LBM_ERR_CUDA, std::string("on-chip step launch: ") + cudaGetErrorString((cudaError_t)e));
+        if (H->res_refuse > 0) {
+            --H->res_refuse;
+            break;
+        }
+        if (resident_launch(H->res_kern, H->res_plan, a, s) != cudaSuccess) {
+            cudaGetLastError();  // an error that lasts is the next launch's too
+            break;
         }
         H->res_tag += (unsigned)k;
         H->cur ^= 1;
         done += k;
     }
-    CUDA_TRY(cudaEventRecord(H->stepped, s));
-    return LBM_OK;
+    return done;
 }
 
 int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
@@ -933,7 +940,13 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
         // a stream under capture records plain launches, as it always did
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (stream && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-        if (cap == cudaStreamCaptureStatusNone) return resident_steps(H, nsteps, write_macro_last, s);
+        if (cap == cudaStreamCaptureStatusNone) {
+            nsteps -= resident_steps(H, nsteps, write_macro_last, s);
+            if (nsteps == 0) {
+                CUDA_TRY(cudaEventRecord(H->stepped, s));
+                return LBM_OK;
+            }
+        }
     }
     int plain = nsteps - (write_macro_last && nsteps > 0 ? 1 : 0);
     int rc;
@@ -1226,9 +1239,10 @@ int lbm_kernel_variant(lbm_handle H) {
 
 int lbm_on_chip(lbm_handle H) { return H ? (H->res_kern ? 1 : 0) : -1; }
 
-int lbm_test_on_chip(lbm_handle H, int polls) {
+int lbm_test_on_chip(lbm_handle H, int polls, int refuse) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     H->res_polls = polls < 0 ? RESIDENT_POLLS : (unsigned)polls;
+    H->res_refuse = refuse;
     return LBM_OK;
 }
 
