@@ -320,9 +320,11 @@ int lbm_kernel_variant(lbm_handle h);
 int lbm_on_chip(lbm_handle h);
 
 /* For tests: `polls` of a message after the first, before its wait gives up
- * (negative: the default, seconds), and the number of launches to come that
- * are taken as refused by the driver. */
-int lbm_test_on_chip(lbm_handle h, int polls, int refuse);
+ * (negative: the default, seconds); the number of launches to come that are
+ * taken as refused by the driver; and the part of the SMs to take (1, 2, 4, 8:
+ * one part of so many; 0: by the handles at work).  A part too small for the
+ * lattice falls back to the next larger. */
+int lbm_test_on_chip(lbm_handle h, int polls, int refuse, int parts);
 
 /* Empty when the handle runs the kernel lbm_create meant to use; otherwise
  * why it fell back (the run-time specialised kernel could not be built, for

@@ -70,14 +70,14 @@ def test_wait_that_gives_up():
         if (np.asarray(lat.bc[:, 5]) > 0).any():
             readers.append(lambda: s.reference_drag_lift(int(lat.bc[:, 5].max()), np.zeros(nn), np.zeros(nn)))
         for renew in (lambda: s.set_state(good), lambda: (s.init(*rest(nn)), s.step(20))):
-            N.check(s._lib.lbm_test_on_chip(s._h, 0, 0))
+            N.check(s._lib.lbm_test_on_chip(s._h, 0, 0, 0))
             s.step(30)
             for read in readers:
                 with pytest.raises(N.LbmError) as e:
                     read()
                 assert e.value.code == N.LBM_ERR_CUDA
             assert s.status == N.LBM_ERR_CUDA
-            N.check(s._lib.lbm_test_on_chip(s._h, -1, 0))
+            N.check(s._lib.lbm_test_on_chip(s._h, -1, 0, 0))
             renew()
             assert s.status == N.LBM_OK
             assert np.array_equal(s.get_state(), good)
@@ -95,8 +95,56 @@ def test_refused_launch():
         with Solver(lat, args) as s:
             s.init(*rest(lat.num_nodes))
             for k in (20, 41, 7):
-                N.check(s._lib.lbm_test_on_chip(s._h, -1, refuse))
+                N.check(s._lib.lbm_test_on_chip(s._h, -1, refuse, 0))
                 s.step(k, write_macro=True)
             return [s.get_state()] + list(s.macro()) + [s.status]
     for a, b in zip(run(0), run(1)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,m", [(13, 200), (61, 47), (203, 131), (400, 350)])
+@pytest.mark.parametrize("storage", [N.STORE_F32, N.STORE_F16S])
+def test_parts_of_the_chip(n, m, storage):
+    """The cuts for a half, a quarter and an eighth of the SMs give the state
+    of the cut for all of them (the last size fits no eighth)."""
+    lat, args = cavity(n, m, storage=storage)
+
+    def run(parts):
+        with Solver(lat, args) as s:
+            s.init(*rest(lat.num_nodes))
+            N.check(s._lib.lbm_test_on_chip(s._h, -1, 0, parts))
+            s.step(25)
+            s.step(12, write_macro=True)
+            return [s.get_state()] + list(s.macro())
+    ref = run(1)
+    for parts in (2, 4, 8):
+        for a, b in zip(ref, run(parts)):
+            assert np.array_equal(a, b)
+
+
+def test_handles_side_by_side():
+    """Six handles stepped by six threads on streams of their own, call after
+    call, so that launches meet in flight: each ends as it does alone."""
+    import torch
+    cases = [cavity(128 + 8 * k, 96 + 40 * k, (N.BGKW, N.TRT, N.MRT)[k % 3]) for k in range(6)]
+
+    def run(k, out):
+        lat, args = cases[k]
+        stream = torch.cuda.Stream()
+        with Solver(lat, args) as s:
+            s.init(*rest(lat.num_nodes))
+            for _ in range(30):
+                s.step(40, write_macro=False, stream=stream.cuda_stream)
+            s.step(10, write_macro=True, stream=stream.cuda_stream)
+            out[k] = [s.get_state()] + list(s.macro())
+    alone, together = {}, {}
+    for k in range(6):
+        run(k, alone)
+    threads = [threading.Thread(target=run, args=(k, together)) for k in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(6):
+        for a, b in zip(alone[k], together[k]):
+            assert np.array_equal(a, b)

@@ -127,11 +127,12 @@ struct lbm_handle_s {
     size_t tma_smem = 0;
     // many steps per launch with the populations on chip (2D lattices that fit)
     const void *res_kern = nullptr;
-    ResidentPlan res_plan;
+    ResidentPlan res_plan[RESIDENT_PLANS];  // for the whole chip, a half, a quarter, an eighth; empty where none fits
+    int res_sms = 0, res_dev = 0;
     unsigned long long *res_mail = nullptr;
     unsigned *res_err = nullptr, *res_err_d = nullptr;  // host word and its device address
     unsigned res_tag = 0, res_polls = RESIDENT_POLLS;
-    int res_refuse = 0;  // launches to take as refused (lbm_test_on_chip)
+    int res_refuse = 0, res_parts = 0;  // lbm_test_on_chip
     double omega = 1, omega_m = 1, gshift = 0;
     float scale = 1024.f;
 };
@@ -184,8 +185,77 @@ static StepParams make_params(const lbm_handle_s *H, int from, int write_macro) 
     return p;
 }
 
+// The handles whose on-chip steps may be in flight, each with its stream and
+// the SMs of its last launch.
+struct OnChip {
+    const lbm_handle_s *H;
+    cudaStream_t stream;
+    int tiles;
+};
+static std::mutex g_on_chip_mutex;
+static std::vector<OnChip> g_on_chip;
+
+static void on_chip_remove(const lbm_handle_s *H) {
+    std::lock_guard<std::mutex> lock(g_on_chip_mutex);
+    for (size_t i = 0; i < g_on_chip.size(); ++i)
+        if (g_on_chip[i].H == H) g_on_chip.erase(g_on_chip.begin() + i--);
+}
+// After the launches and the record of H->stepped that follows them.
+static void on_chip_add(const lbm_handle_s *H, cudaStream_t s, int tiles) {
+    on_chip_remove(H);
+    std::lock_guard<std::mutex> lock(g_on_chip_mutex);
+    g_on_chip.push_back({H, s, tiles});
+}
+
+// The plan for a call on stream s.  A tile takes an SM's shared memory whole,
+// so the launches of several handles run side by side only where their tiles
+// fit the SMs together.  While other handles' launches are in flight on other
+// streams and a whole-chip launch does not fit beside them, a handle takes a
+// half, a quarter or an eighth of the SMs, as many parts as there are handles
+// at work: a step of a small lattice is mostly one message flight, whatever the
+// tile.  Handles on streams of their own, 100 steps a call, us for a step of all
+// of them (whole-chip launches one after another; a launch per step):
+//   128^2  x 4: 2.5 (7.3; 4.3)   x 8: 2.8 (14.6; 5.4)
+//   256^2  x 4: 3.2 (8.4; 5.3)   x 8: 6.3 (16.8; 6.5)
+//   400^2  x 4: 5.3 (9.3; 7.0)   x 8: 10.6 (19.2; 13.6)
+// 512^2 and larger fit no part; there the launches take turns (x 4: 9.7, against
+// 9.4 with a launch per step; x 8: 19.6 and 25.7).  Eight of 320^2 fit by fours
+// and are the case left slower than a launch per step: 9.0 and 7.2.
+static const ResidentPlan &on_chip_plan(const lbm_handle_s *H, cudaStream_t s) {
+    int others = 0, used = 0;
+    {
+        std::lock_guard<std::mutex> lock(g_on_chip_mutex);
+        // a query is no business of a stream capture that this or another
+        // thread may have begun
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        bool relaxed = false;
+        for (size_t i = 0; i < g_on_chip.size(); ++i) {
+            const OnChip e = g_on_chip[i];
+            if (e.H == H || e.H->res_dev != H->res_dev || e.stream == s) continue;
+            if (!relaxed) relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+            if (cudaEventQuery(e.H->stepped) != cudaErrorNotReady) {
+                g_on_chip.erase(g_on_chip.begin() + i--);
+            } else {
+                ++others;
+                used += e.tiles;
+            }
+        }
+        if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    int k = 0;
+    if (H->res_parts > 0) {
+        while ((1 << k) < H->res_parts) ++k;
+    } else if (others && used + H->res_plan[0].tiles() > H->res_sms) {
+        while ((1 << k) < others + 1) ++k;
+    }
+    k = std::min(k, RESIDENT_PLANS - 1);
+    while (k > 0 && !H->res_plan[k].tiles()) --k;
+    return H->res_plan[k];
+}
+
 static void free_handle(lbm_handle_s *H) {
     if (!H) return;
+    on_chip_remove(H);
     for (int c = 0; c < 2; ++c)
         if (H->graph[c]) cudaGraphExecDestroy(H->graph[c]);
     void *ptrs[] = {H->fbuf[0], H->fbuf[1], H->word, H->slot, H->mask, H->kind, H->uvw,
@@ -398,9 +468,15 @@ static int setup_resident(lbm_handle_s *H) {
     CUDA_TRY(cudaGetDevice(&dev));
     CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop || !resident_plan(H->n, H->m, (int)H->elem, sms, &H->res_plan)) return LBM_OK;
-    const void *kern = resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan);
+    if (!coop || !resident_plan(H->n, H->m, (int)H->elem, sms, &H->res_plan[0])) return LBM_OK;
+    const void *kern = resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan[0]);
     if (!kern) return LBM_OK;
+    for (int k = 1; k < RESIDENT_PLANS; ++k)
+        if (!resident_plan(H->n, H->m, (int)H->elem, sms >> k, &H->res_plan[k]) ||
+            !resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan[k]))
+            H->res_plan[k] = ResidentPlan();
+    H->res_sms = sms;
+    H->res_dev = dev;
     const size_t bytes = sizeof(unsigned long long) * 16 * (size_t)H->N;
     cudaError_t e = cudaMalloc((void **)&H->res_mail, bytes);
     // the error word lies in host memory: only a wait that gives up writes it,
@@ -899,7 +975,7 @@ constexpr int RESIDENT_CHUNK = 8192;  // steps per launch, tens of milliseconds
 // Runs up to nsteps steps and returns how many: where the driver refuses a
 // launch (a stream whose context holds fewer SMs than the device, another
 // process's share), the rest of the call is the caller's, a launch per step.
-static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cudaStream_t s) {
+static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cudaStream_t s, const ResidentPlan &plan) {
     int done = 0;
     while (done < nsteps) {
         const int k = std::min(nsteps - done, RESIDENT_CHUNK);
@@ -907,9 +983,9 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
         a.p = make_params(H, H->cur, 0);
         a.last = make_params(H, H->cur, write_macro_last && done + k == nsteps);
         a.steps = k;
-        a.gx = H->res_plan.gx;
-        a.gy = H->res_plan.gy;
-        a.compute = H->res_plan.compute;
+        a.gx = plan.gx;
+        a.gy = plan.gy;
+        a.compute = plan.compute;
         a.wrap = H->jit_key.wrap;
         a.tag = H->res_tag;
         a.mail = H->res_mail;
@@ -919,7 +995,7 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
             --H->res_refuse;
             break;
         }
-        if (resident_launch(H->res_kern, H->res_plan, a, s) != cudaSuccess) {
+        if (resident_launch(H->res_kern, plan, a, s) != cudaSuccess) {
             cudaGetLastError();  // an error that lasts is the next launch's too
             break;
         }
@@ -941,9 +1017,11 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (stream && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
         if (cap == cudaStreamCaptureStatusNone) {
-            nsteps -= resident_steps(H, nsteps, write_macro_last, s);
+            const ResidentPlan &plan = on_chip_plan(H, s);
+            nsteps -= resident_steps(H, nsteps, write_macro_last, s, plan);
             if (nsteps == 0) {
                 CUDA_TRY(cudaEventRecord(H->stepped, s));
+                on_chip_add(H, s, plan.tiles());
                 return LBM_OK;
             }
         }
@@ -1239,10 +1317,11 @@ int lbm_kernel_variant(lbm_handle H) {
 
 int lbm_on_chip(lbm_handle H) { return H ? (H->res_kern ? 1 : 0) : -1; }
 
-int lbm_test_on_chip(lbm_handle H, int polls, int refuse) {
+int lbm_test_on_chip(lbm_handle H, int polls, int refuse, int parts) {
     if (!H) return fail(LBM_ERR_INVALID, "null handle");
     H->res_polls = polls < 0 ? RESIDENT_POLLS : (unsigned)polls;
     H->res_refuse = refuse;
+    H->res_parts = parts;
     return LBM_OK;
 }
 

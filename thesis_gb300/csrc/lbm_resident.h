@@ -12,7 +12,9 @@ namespace lbm {
 struct ResidentPlan {
     int gx = 0, gy = 0, compute = 0, comm = 0;
     size_t smem = 0;
+    int tiles() const { return gx * gy; }
 };
+constexpr int RESIDENT_PLANS = 4;
 
 struct ResidentArgs {
     StepParams p, last;       // fin: the state at entry, fout: where it goes; last: with write_macro as asked

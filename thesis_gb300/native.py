@@ -111,7 +111,7 @@ def lib():
         "lbm_bytes_per_update": (C.c_int, [vp]),
         "lbm_kernel_variant": (C.c_int, [vp]),
         "lbm_on_chip": (C.c_int, [vp]),
-        "lbm_test_on_chip": (C.c_int, [vp, C.c_int, C.c_int]),
+        "lbm_test_on_chip": (C.c_int, [vp, C.c_int, C.c_int, C.c_int]),
         "lbm_kernel_warning": (C.c_char_p, [vp]),
         "lbm_jit_check": (C.c_int, [C.c_int] * 11),
         "lbm_autotune": (C.c_int, [vp, C.c_int, _IP, _IP, _IP]),
