@@ -148,3 +148,28 @@ def test_handles_side_by_side():
     for k in range(6):
         for a, b in zip(alone[k], together[k]):
             assert np.array_equal(a, b)
+
+
+def test_error_words_of_many_handles():
+    """More handles at once than a page of error words holds: a wait that gives
+    up in one is reported by that one alone, also after words were given back."""
+    lat, args = cavity(24, 24)
+    ss = [Solver(lat, args) for _ in range(1030)]
+    try:
+        for s in ss[::2]:
+            s.close()
+        ss = ss[1::2] + [Solver(lat, args) for _ in range(40)]
+        for s in ss:
+            s.init(*rest(lat.num_nodes))
+        N.check(ss[7]._lib.lbm_test_on_chip(ss[7]._h, 0, 0, 0))
+        for s in ss:
+            s.step(10)
+        for k, s in enumerate(ss):
+            if k == 7:
+                with pytest.raises(N.LbmError):
+                    s.get_state()
+            else:
+                s.get_state()
+    finally:
+        for s in ss:
+            s.close()

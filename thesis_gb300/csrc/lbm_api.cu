@@ -130,6 +130,7 @@ struct lbm_handle_s {
     ResidentPlan res_plan[RESIDENT_PLANS];  // for the whole chip, a half, a quarter, an eighth; empty where none fits
     int res_sms = 0, res_dev = 0;
     unsigned long long *res_mail = nullptr;
+    size_t res_mail_bytes = 0;
     unsigned *res_err = nullptr, *res_err_d = nullptr;  // host word and its device address
     unsigned res_tag = 0, res_polls = RESIDENT_POLLS;
     int res_refuse = 0, res_parts = 0;  // lbm_test_on_chip
@@ -183,6 +184,56 @@ static StepParams make_params(const lbm_handle_s *H, int from, int write_macro) 
     p.outlet_profile = H->P.outlet_profile;
     p.update_inlet_outlet = H->P.update_inlet_outlet;
     return p;
+}
+
+// Error words of the on-chip kernels: in host memory, as only a wait that gives
+// up writes one and the host reads it without a copy.  Pages of mapped memory
+// are dealt out by the word, since making and freeing one costs more than the
+// rest of a small handle (128^2, made, initialised and destroyed: 1020 us with a
+// page each and messages by node, 740 now; 605 without the on-chip kernel).
+// The last page is kept.
+struct ErrorPage {
+    static constexpr int WORDS = 1024;
+    unsigned *host = nullptr, *dev = nullptr;
+    std::vector<int> free;
+};
+static std::mutex g_error_mutex;
+static std::vector<ErrorPage> g_error_pages;
+
+static cudaError_t error_word_take(unsigned **host, unsigned **dev) {
+    std::lock_guard<std::mutex> lock(g_error_mutex);
+    auto page = std::find_if(g_error_pages.begin(), g_error_pages.end(), [](const ErrorPage &p) { return !p.free.empty(); });
+    if (page == g_error_pages.end()) {
+        ErrorPage p;
+        cudaError_t e = cudaHostAlloc((void **)&p.host, sizeof(unsigned) * ErrorPage::WORDS,
+                                      cudaHostAllocMapped | cudaHostAllocPortable);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&p.dev, (void *)p.host, 0);
+        if (e != cudaSuccess) {
+            if (p.host) cudaFreeHost(p.host);
+            return e;
+        }
+        for (int i = ErrorPage::WORDS; i-- > 0;) p.free.push_back(i);
+        page = g_error_pages.insert(g_error_pages.end(), p);
+    }
+    const int i = page->free.back();
+    page->free.pop_back();
+    *host = page->host + i;
+    *dev = page->dev + i;
+    *(volatile unsigned *)*host = 0;
+    return cudaSuccess;
+}
+static void error_word_give(unsigned *host) {
+    std::lock_guard<std::mutex> lock(g_error_mutex);
+    for (size_t k = 0; k < g_error_pages.size(); ++k) {
+        ErrorPage &p = g_error_pages[k];
+        if (host < p.host || host >= p.host + ErrorPage::WORDS) continue;
+        p.free.push_back((int)(host - p.host));
+        if ((int)p.free.size() == ErrorPage::WORDS && g_error_pages.size() > 1) {
+            cudaFreeHost(p.host);
+            g_error_pages.erase(g_error_pages.begin() + k);
+        }
+        return;
+    }
 }
 
 // The handles whose on-chip steps may be in flight, each with its stream and
@@ -264,7 +315,7 @@ static void free_handle(lbm_handle_s *H) {
                     H->bcq, H->bc_macro, H->res_mail};
     for (void *p : ptrs)
         if (p) cudaFree(p);
-    if (H->res_err) cudaFreeHost(H->res_err);
+    if (H->res_err) error_word_give(H->res_err);
     if (H->stepped) cudaEventDestroy(H->stepped);
     if (H->stream) cudaStreamDestroy(H->stream);
     delete H;
@@ -460,39 +511,31 @@ static int setup_jit(lbm_handle_s *H, const HostArray<uint32_t> &word, bool pair
 // own populations: open outlets and curved walls read neighbours from the
 // read buffer, which that kernel does not keep.  F16S in reference mode and
 // F64 keep the launch per step.
-static int setup_resident(lbm_handle_s *H) {
-    if (H->q != 9 || !H->jit_kernel || H->jit_key.pair || one_node_boundaries(H->P, H->q) || H->bc_macro) return LBM_OK;
+static void setup_resident(lbm_handle_s *H) {
+    if (H->q != 9 || !H->jit_kernel || H->jit_key.pair || one_node_boundaries(H->P, H->q)) return;
     const bool phys = H->P.mode == LBM_MODE_PHYSICS;
-    if (H->P.storage != LBM_STORE_F32 && !(H->P.storage == LBM_STORE_F16S && phys)) return LBM_OK;
+    if (H->P.storage != LBM_STORE_F32 && !(H->P.storage == LBM_STORE_F16S && phys)) return;
     int dev = 0, sms = 0, coop = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop || !resident_plan(H->n, H->m, (int)H->elem, sms, &H->res_plan[0])) return LBM_OK;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (e != cudaSuccess || !coop || !resident_plan(H->n, H->m, (int)H->elem, sms, &H->res_plan[0])) return;
     const void *kern = resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan[0]);
-    if (!kern) return LBM_OK;
+    if (!kern) return;
+    // blocks of the other plans are no larger than the kernel's launch bounds
     for (int k = 1; k < RESIDENT_PLANS; ++k)
-        if (!resident_plan(H->n, H->m, (int)H->elem, sms >> k, &H->res_plan[k]) ||
-            !resident_prepare(H->P.collision_model, H->P.storage, phys, H->res_plan[k]))
-            H->res_plan[k] = ResidentPlan();
-    H->res_sms = sms;
-    H->res_dev = dev;
-    const size_t bytes = sizeof(unsigned long long) * 16 * (size_t)H->N;
-    cudaError_t e = cudaMalloc((void **)&H->res_mail, bytes);
-    // the error word lies in host memory: only a wait that gives up writes it,
-    // and the host reads it without a copy
-    if (e == cudaSuccess) e = cudaHostAlloc((void **)&H->res_err, sizeof(unsigned), cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&H->res_err_d, (void *)H->res_err, 0);
-    // awaited on the handle's stream: a clearing that runs after the first messages would lose them
-    if (e == cudaSuccess) e = cudaMemsetAsync(H->res_mail, 0, bytes, H->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
+        if (!resident_plan(H->n, H->m, (int)H->elem, sms >> k, &H->res_plan[k])) H->res_plan[k] = ResidentPlan();
+    for (const ResidentPlan &p : H->res_plan)
+        H->res_mail_bytes = std::max(H->res_mail_bytes, sizeof(unsigned long long) * p.messages());
+    e = cudaMalloc((void **)&H->res_mail, H->res_mail_bytes);
+    if (e == cudaSuccess) e = error_word_take(&H->res_err, &H->res_err_d);
     if (e != cudaSuccess) {
         cudaGetLastError();  // no room for the messages: a launch per step
-        return LBM_OK;
+        return;
     }
-    *(volatile unsigned *)H->res_err = 0;
     H->res_kern = kern;
-    return LBM_OK;
+    H->res_sms = sms;
+    H->res_dev = dev;
 }
 
 // A bounded wait inside the on-chip or the row-staged kernel that gave up
@@ -698,6 +741,7 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
     ALLOC(H->mdiff_prev, sizeof(float) * 4 * N);
     ALLOC(H->norms, sizeof(double) * LBM_NORMS);
 #undef ALLOC
+    if (!kernel_chosen) setup_resident(H);
     cudaError_t e = cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&H->stepped, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemcpy(H->word, flags.word.data(), sizeof(uint32_t) * N, cudaMemcpyHostToDevice);
@@ -730,21 +774,15 @@ int lbm_create(const lbm_lattice_desc *L, const lbm_params *P, lbm_handle *out) 
         std::vector<double> qt((size_t)q * H->nslots, 0.5);
         if (H->nslots) e = cudaMemcpy(H->bcq, qt.data(), sizeof(double) * qt.size(), cudaMemcpyHostToDevice);
     }
-    // on the handle's stream, and awaited: the default stream may hold work of
-    // others, and a clearing that runs after the first use would undo it
+    // clearing on the handle's stream, and awaited: the default stream may hold
+    // work of others, and a clearing that runs after the first use would undo it
     for (float *f : {H->pux, H->puy, H->puz})
         if (e == cudaSuccess) e = cudaMemsetAsync(f, 0, sizeof(float) * N, H->stream);
+    if (e == cudaSuccess && H->res_kern) e = cudaMemsetAsync(H->res_mail, 0, H->res_mail_bytes, H->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(H->stream);
     if (e != cudaSuccess) {
         free_handle(H);
         return fail(LBM_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
-    }
-    if (!kernel_chosen) {
-        rc = setup_resident(H);
-        if (rc) {
-            free_handle(H);
-            return rc;
-        }
     }
     *out = H;
     return LBM_OK;
@@ -986,6 +1024,7 @@ static int resident_steps(lbm_handle_s *H, int nsteps, int write_macro_last, cud
         a.gx = plan.gx;
         a.gy = plan.gy;
         a.compute = plan.compute;
+        a.links = plan.links;
         a.wrap = H->jit_key.wrap;
         a.tag = H->res_tag;
         a.mail = H->res_mail;

@@ -14,8 +14,9 @@
 // message is one 8-byte word {population bits, tag} written and read with
 // single relaxed accesses, so its arrival needs no fence and no flag: the
 // reader polls the word itself until it carries the tag of the state it
-// wants.  Messages are indexed by destination node and direction
-// (mail[parity][d - 1][node]).  Every link that crosses a tile edge is sent
+// wants.  A tile reads its messages from slots of its own
+// (mail[parity][tile][link], numbered by tile_link), side by side for the lanes
+// that poll them.  Every link that crosses a tile edge is sent
 // and awaited in both directions, blocked or not: neighbouring tiles then
 // advance in lockstep, neither can be two states ahead of the other, and two
 // parities of the mailbox suffice.  The first step takes its halo from the
@@ -109,6 +110,16 @@ __device__ __forceinline__ int lattice_o2(int d) { return d <= 4 ? (d + 1) % 4 +
 // cut g ways.
 __device__ __forceinline__ int axis_begin(int i, int n, int g) { return (int)((long long)i * n / g); }
 
+// The number of the link in direction d that leaves a tw x th tile from (lx,
+// ly), among 6 (tw + th): three directions per node of each side, top, bottom,
+// right, left; a corner's diagonal belongs to its row.
+__host__ __device__ __forceinline__ int tile_link(int lx, int ly, int d, int cx, int cy, int tw, int th) {
+    if (ly + cy >= th) return (d == 2 ? 0 : d - 4) * tw + lx;                      // 2 5 6
+    if (ly + cy < 0) return (3 + (d == 4 ? 0 : d - 6)) * tw + lx;                  // 4 7 8
+    const int q = cx > 0 ? (d == 1 ? 0 : (d == 5 ? 1 : 2)) : 3 + (d == 3 ? 0 : d - 5);  // 1 5 8, 3 6 7
+    return 6 * tw + q * th + ly;
+}
+
 template <int COLL, int ST, bool PHYS>
 __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(const __grid_constant__ ResidentArgs a) {
     using L = Lat<9>;
@@ -117,7 +128,7 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tid = threadIdx.x;
     const DynGeom g{a.p.nx, a.p.ny, a.p.nz, a.p.pitch};
-    const int nx = g.nx, ny = g.ny, N = nx * ny;
+    const int nx = g.nx, ny = g.ny;
     const int bx = blockIdx.x % a.gx, by = blockIdx.x / a.gx;
     const int x0 = axis_begin(bx, nx, a.gx), y0 = axis_begin(by, ny, a.gy);
     const int tw = axis_begin(bx + 1, nx, a.gx) - x0, th = axis_begin(by + 1, ny, a.gy) - y0;
@@ -272,12 +283,11 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
         int out_s[MSGS], out_m[MSGS], in_s[MSGS], in_m[MSGS];
 #pragma unroll
         for (int k = 0; k < MSGS; ++k) out_s[k] = in_s[k] = -1;
-        // 6 (tw + th) candidates: three directions per node of each side, top,
-        // bottom, right, left; a corner's diagonal belongs to its row
+        // the links by number (tile_link)
 #pragma unroll
         for (int k = 0; k < MSGS; ++k) {
-            int m = tid - a.compute + k * ((int)blockDim.x - a.compute);
-            int lx, ly, d;
+            const int link = tid - a.compute + k * ((int)blockDim.x - a.compute);
+            int m = link, lx, ly, d;
             if (m < 6 * tw) {
                 const bool top = m < 3 * tw;
                 const int j = top ? m : m - 3 * tw, q = j / tw;
@@ -301,16 +311,23 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
             int x = x0 + lx + cx, y = y0 + ly + cy;
             if (!inside(x, y)) continue;
             out_s[k] = d * PLANE + lx + 1 + pitch * (ly + 1);
-            out_m[k] = (d - 1) * N + x + nx * y;
-            // in: the opposite direction over the same link, from the halo
+            // the tile it lies in, and the link's number there, where it leaves in the
+            // opposite direction
             const int o = lattice_o2(d);
+            const int ox = lx + cx < 0 ? (bx + a.gx - 1) % a.gx : (lx + cx >= tw ? (bx + 1) % a.gx : bx);
+            const int oy = ly + cy < 0 ? (by + a.gy - 1) % a.gy : (ly + cy >= th ? (by + 1) % a.gy : by);
+            const int ox0 = axis_begin(ox, nx, a.gx), oy0 = axis_begin(oy, ny, a.gy);
+            out_m[k] = (ox + a.gx * oy) * a.links + tile_link(x - ox0, y - oy0, o, -cx, -cy,
+                                                              axis_begin(ox + 1, nx, a.gx) - ox0,
+                                                              axis_begin(oy + 1, ny, a.gy) - oy0);
+            // in: that direction over the same link, from the halo
             in_s[k] = o * PLANE + lx + cx + 1 + pitch * (ly + cy + 1);
-            in_m[k] = (o - 1) * N + x0 + lx + nx * (y0 + ly);
+            in_m[k] = (int)blockIdx.x * a.links + link;
         }
 #pragma unroll 1
         for (int s = 0; s < a.steps - 1; ++s) {
             T *out = s & 1 ? buf0 : buf1;
-            unsigned long long *mail = a.mail + (size_t)((s + 1) & 1) * 8 * N;
+            unsigned long long *mail = a.mail + (size_t)((s + 1) & 1) * (gridDim.x * a.links);
             const unsigned tag = a.tag + (unsigned)s + 1u;
             bar_sync(1, bar_threads);
 #pragma unroll
@@ -384,7 +401,8 @@ bool resident_plan(int nx, int ny, int elem, int sms, ResidentPlan *out) {
             out->gy = gy;
             nt = tw * th;
             edges = tile_edges(tw, th);
-            out->comm = std::min(MAX_COMM, (6 * (tw + th) + 31) / 32 * 32);
+            out->links = 6 * (tw + th);
+            out->comm = std::min(MAX_COMM, (out->links + 31) / 32 * 32);
         }
     }
     if (best < 0) return false;

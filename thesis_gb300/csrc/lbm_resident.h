@@ -8,20 +8,22 @@
 namespace lbm {
 
 // How a 2D lattice is cut into one tile per block: gx x gy tiles, `compute`
-// threads that update nodes and `comm` threads that exchange tile edges.
+// threads that update nodes and `comm` threads that exchange tile edges, over
+// at most `links` links out of a tile.
 struct ResidentPlan {
-    int gx = 0, gy = 0, compute = 0, comm = 0;
+    int gx = 0, gy = 0, compute = 0, comm = 0, links = 0;
     size_t smem = 0;
     int tiles() const { return gx * gy; }
+    size_t messages() const { return (size_t)2 * tiles() * links; }
 };
 constexpr int RESIDENT_PLANS = 4;
 
 struct ResidentArgs {
     StepParams p, last;       // fin: the state at entry, fout: where it goes; last: with write_macro as asked
-    int steps, gx, gy, compute;
+    int steps, gx, gy, compute, links;
     int wrap;                 // links leave the lattice by wrapping round
     unsigned tag;             // messages of this launch carry tag + 1 .. tag + steps - 1
-    unsigned long long *mail; // [2][8][nx * ny] messages
+    unsigned long long *mail; // [2][tile][links] messages
     unsigned polls;           // of a message after the first, before its wait gives up
     unsigned *err;            // set when a wait gave up
 };
