@@ -353,7 +353,10 @@ const char *lbm_kernel_warning(lbm_handle h);
  * may be NULL.  In physics mode with
  * F32 storage only storage-unit variants are candidates (their moments come
  * from deviations from the rest state).  This function has no
- * counterpart in the reference. */
+ * counterpart in the reference.  Where calls of several steps run on chip
+ * (lbm_on_chip), they still do, and the choice, which lbm_kernel_config and
+ * lbm_kernel_variant describe, serves calls of fewer than four steps and calls
+ * recorded by a stream under capture. */
 int lbm_autotune(lbm_handle h, int trial_steps, int *block, int *hint, int *pred);
 /* The knobs of the handle's step kernel: 128, 0, 0 unless tuned, requested or
  * set by the rule for physics-mode 3D lattices of 200,000 nodes and more (the

@@ -173,3 +173,22 @@ def test_error_words_of_many_handles():
     finally:
         for s in ss:
             s.close()
+
+
+@pytest.mark.parametrize("n,m", [(96, 64), (250, 130)])
+def test_tuning_keeps_steps_on_chip(n, m):
+    """Handles of a tuned shape run on chip whatever kernel the tuning chose for
+    a launch per step, and give the same state."""
+    lat, args = cavity(n, m)
+
+    def run(tune):
+        with Solver(lat, args) as s:
+            if tune:
+                s.autotune(4)
+            assert s.on_chip
+            s.init(*rest(lat.num_nodes))
+            s.step(30)
+            return s.get_state()
+    first = run(False)
+    assert np.array_equal(first, run(True))
+    assert np.array_equal(first, run(False))

@@ -510,9 +510,10 @@ static int setup_jit(lbm_handle_s *H, const HostArray<uint32_t> &word, bool pair
 // that fits (resident_plan), whose boundary conditions touch only the node's
 // own populations: open outlets and curved walls read neighbours from the
 // read buffer, which that kernel does not keep.  F16S in reference mode and
-// F64 keep the launch per step.
+// F64 keep the launch per step.  What tuning chose for the launch per step
+// (two nodes per thread, say) is no matter.
 static void setup_resident(lbm_handle_s *H) {
-    if (H->q != 9 || !H->jit_kernel || H->jit_key.pair || one_node_boundaries(H->P, H->q)) return;
+    if (H->q != 9 || !H->jit_kernel || one_node_boundaries(H->P, H->q)) return;
     const bool phys = H->P.mode == LBM_MODE_PHYSICS;
     if (H->P.storage != LBM_STORE_F32 && !(H->P.storage == LBM_STORE_F16S && phys)) return;
     int dev = 0, sms = 0, coop = 0;
