@@ -1,5 +1,5 @@
 // C ABI of the lattice-Boltzmann engine (include/thesis_lbm.h): handle
-// lifetime, device allocation, initial collision, the step loop (with a
+// lifetime, device allocation, initial collision, the step loop (with
 // captured CUDA graphs for short steps) and read-back.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -111,7 +111,7 @@ struct lbm_handle_s {
     // recorded after the steps of every lbm_step, on the stream they ran on;
     // the handle's own stream waits for it before reductions and read-back
     cudaEvent_t stepped = nullptr;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // GRAPH_STEPS steps from buffer 0 and from buffer 1
+    cudaGraphExec_t graph[2][2] = {};  // [short, long][buffer it starts from]
     int status = LBM_OK;
     bool initialised = false;
     bool pair_kernel = false;  // two nodes per thread (even nx, F32/F16S)
@@ -304,11 +304,18 @@ static const ResidentPlan &on_chip_plan(const lbm_handle_s *H, cudaStream_t s) {
     return H->res_plan[k];
 }
 
+static void free_graphs(lbm_handle_s *H) {
+    for (auto &pair : H->graph)
+        for (cudaGraphExec_t &g : pair) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+}
+
 static void free_handle(lbm_handle_s *H) {
     if (!H) return;
     on_chip_remove(H);
-    for (int c = 0; c < 2; ++c)
-        if (H->graph[c]) cudaGraphExecDestroy(H->graph[c]);
+    free_graphs(H);
     void *ptrs[] = {H->fbuf[0], H->fbuf[1], H->word, H->slot, H->mask, H->kind, H->uvw,
                     H->rho, H->ux, H->uy, H->uz, H->pux, H->puy, H->puz, H->partial, H->norms,
                     H->tma_row, H->tma_lmask, H->tma_omask, H->tma_err, H->mdiff_prev, H->fd_snap,
@@ -986,21 +993,23 @@ static int launch(lbm_handle_s *H, int from, int write_macro, cudaStream_t s) {
     return rc ? fail(LBM_ERR_UNSUPPORTED, "no kernel for this configuration") : LBM_OK;
 }
 
-// GRAPH_STEPS steps (from buffer c back to buffer c) captured once as a graph.
-// A replay costs about 2 us between graphs, which two steps per graph put on
-// every second step: a 75 x 61 x 47 MRT step took 9.7 us, 7.7 us with sixteen.
-// Calls shorter than two replays launch step by step.
-constexpr int GRAPH_STEPS = 16, GRAPH_MIN = 32;
-static int step_graph(lbm_handle_s *H, int c) {
-    if (H->graph[c]) return LBM_OK;
+// GRAPH_STEPS[which] steps (from buffer c back to buffer c) captured once as a
+// graph.  A replay costs about 2 us between graphs, which two steps per graph
+// put on every second step: a 75 x 61 x 47 MRT step took 9.7 us, 7.7 us with
+// sixteen.  Two still beat launches, so calls and remainders of 8 steps and
+// more too short for the long graph take those: 32^3, F32, 16 steps of a call
+// 89.6 us launched step by step, 75.9 so.  Shorter ones are launched step by step.
+constexpr int GRAPH_STEPS[2] = {2, 16}, GRAPH_MIN[2] = {8, 32};
+static int step_graph(lbm_handle_s *H, int which, int c) {
+    if (H->graph[which][c]) return LBM_OK;
     cudaGraph_t g;
     CUDA_TRY(cudaStreamBeginCapture(H->stream, cudaStreamCaptureModeThreadLocal));
     int rc = LBM_OK;
-    for (int k = 0; k < GRAPH_STEPS && !rc; ++k) rc = launch(H, c ^ (k & 1), 0, H->stream);
+    for (int k = 0; k < GRAPH_STEPS[which] && !rc; ++k) rc = launch(H, c ^ (k & 1), 0, H->stream);
     cudaError_t e = cudaStreamEndCapture(H->stream, &g);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&H->graph[c], g, 0);
+    e = cudaGraphInstantiate(&H->graph[which][c], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(LBM_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
     return LBM_OK;
@@ -1052,26 +1061,27 @@ int lbm_step(lbm_handle H, int nsteps, int write_macro_last, void *stream) {
     if (nsteps < 0) return fail(LBM_ERR_INVALID, "negative step count");
     if (int rc = check_on_chip(H)) return rc;
     cudaStream_t s = stream ? (cudaStream_t)stream : H->stream;
-    if (H->res_kern && nsteps >= RESIDENT_MIN_STEPS) {
-        // a stream under capture records plain launches, as it always did
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (stream && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
-        if (cap == cudaStreamCaptureStatusNone) {
-            const ResidentPlan &plan = on_chip_plan(H, s);
-            nsteps -= resident_steps(H, nsteps, write_macro_last, s, plan);
-            if (nsteps == 0) {
-                CUDA_TRY(cudaEventRecord(H->stepped, s));
-                on_chip_add(H, s, plan.tiles());
-                return LBM_OK;
-            }
+    // a stream under capture records a launch per step
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (stream && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (H->res_kern && nsteps >= RESIDENT_MIN_STEPS && !captured) {
+        const ResidentPlan &plan = on_chip_plan(H, s);
+        nsteps -= resident_steps(H, nsteps, write_macro_last, s, plan);
+        if (nsteps == 0) {
+            CUDA_TRY(cudaEventRecord(H->stepped, s));
+            on_chip_add(H, s, plan.tiles());
+            return LBM_OK;
         }
     }
     int plain = nsteps - (write_macro_last && nsteps > 0 ? 1 : 0);
     int rc;
     int done = 0;
-    if (plain >= GRAPH_MIN) {
-        if ((rc = step_graph(H, H->cur))) return rc;
-        for (; done + GRAPH_STEPS <= plain; done += GRAPH_STEPS) CUDA_TRY(cudaGraphLaunch(H->graph[H->cur], s));
+    for (int which = 1; which >= 0; --which) {
+        if (captured || plain - done < GRAPH_MIN[which]) continue;
+        if ((rc = step_graph(H, which, H->cur))) return rc;
+        for (; done + GRAPH_STEPS[which] <= plain; done += GRAPH_STEPS[which])
+            CUDA_TRY(cudaGraphLaunch(H->graph[which][H->cur], s));
     }
     for (; done < plain; ++done) {
         if ((rc = launch(H, H->cur, 0, s))) return rc;
@@ -1493,11 +1503,7 @@ int lbm_autotune(lbm_handle H, int trial_steps, int *block, int *hint, int *pred
     }
     H->jit_key = cand[best_i];
     H->jit_fn = fn[best_i];
-    for (int c = 0; c < 2; ++c)
-        if (H->graph[c]) {
-            cudaGraphExecDestroy(H->graph[c]);
-            H->graph[c] = nullptr;
-        }
+    free_graphs(H);
     {
         std::lock_guard<std::mutex> lock(g_tuned_mutex);
         g_tuned[tune_key(H->jit_key)] = TunedKnobs{H->jit_key.block, H->jit_key.hint, H->jit_key.pred,
