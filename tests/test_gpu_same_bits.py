@@ -92,3 +92,33 @@ def test_batch_sizes(monkeypatch, periodic, storage, dims):
             want = s.populations()
         fl = lat.node_type == 1
         assert np.array_equal(f[:, fl], want[:, fl])
+
+
+@pytest.mark.parametrize("coll", [N.BGKW, N.TRT, N.MRT])
+@pytest.mark.parametrize("storage", [N.STORE_F32, N.STORE_F16S])
+@pytest.mark.parametrize("domains,n,m", [(1, 40, 40), (8, 256, 256), (12, 192, 192), (3, 1024, 256)])
+def test_batch_forms(monkeypatch, coll, storage, domains, n, m):
+    """The forms of the D2Q9 batch kernel (blocks per SM, chosen by the active
+    domains' tiles: five, five, six, and seven for channels), and a batch that
+    goes from form to form as domains retire between replayed calls."""
+    channel = n != m
+    lat = lattice.channel2d(n, m, seed=2) if channel else lattice.cavity2d(n)
+    args = Arguments(u=0.05, viscosity=0.05, collision_model=coll, mode=N.MODE_PHYSICS, storage=storage,
+                     init_equilibrium=1, outlet_profile=N.OUTLET_PRESSURE if channel else N.OUTLET_ZOUHE, rho_out=1.0)
+    nn = lat.num_nodes
+    z = np.zeros(nn)
+    monkeypatch.setenv("THESIS_LBM_KERNEL", "jith")
+    with Solver(lat, args) as s, Batch([lat] * domains, [args] * domains) as b:
+        s.init(np.ones(nn), z, z, z)
+        b.init()
+        for d in range(domains):
+            b.init_fields(d, np.ones(nn), z, z, z)
+        s.step(20)
+        first = s.populations()
+        s.step(20)
+        second = s.populations()
+        b.step(20)
+        b.set_active([int(d == 0 or d % 3 > 0) for d in range(domains)])
+        b.step(20)
+        for d in range(domains):
+            assert np.array_equal(b.populations(d), second if d == 0 or d % 3 > 0 else first)

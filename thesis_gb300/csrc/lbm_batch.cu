@@ -13,6 +13,7 @@
 // stride over the tile table, so small domains fill the GPU together instead
 // of leaving it idle one launch at a time.
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <math.h>
 #include <string.h>
 
@@ -34,15 +35,16 @@ int launch_decode_q19(const StepParams &p, int st, double *out, long long n, cud
 
 namespace {
 
-// A tile is one warp's work: 32 consecutive nodes of a batch's tile rows
-// rows of one domain.  int4: x = domain, y = first row (y + ny z), z = first
-// x, w = node index of (first x, first row) in the batch's macroscopic arrays.
+// A tile is one warp's work: 32 consecutive nodes of some consecutive rows of
+// one domain.  int4: x = domain, y = first row (y + ny z), z = first x, w =
+// node index of (first x, first row) in the batch's macroscopic arrays.
 constexpr int BATCH_WARPS = STEP_BLOCK / 32;
-// consecutive rows.  The rows per tile follow the active domains
-// (batch_rows): as many as divide the work evenly over the resident warps.
+// The rows per tile follow the active domains (batch_rows): as many as divide
+// the work evenly over the resident warps.
 constexpr int BATCH_MIN_ROWS = 2, BATCH_MAX_ROWS = 32;
-// blocks per SM the step kernel is compiled for (D3Q19 nodes need the registers)
-constexpr int batch_resident(int q) { return q == 9 ? 7 : 4; }
+// blocks per SM the step kernel is compiled for: D2Q9 in three forms (batch_rows
+// chooses), D3Q19 in one, whose nodes need the registers
+constexpr int BATCH_FORMS = 3, BATCH_RESIDENT[BATCH_FORMS] = {6, 5, 7}, BATCH_RESIDENT3 = 4;
 constexpr int PARAM_WORDS = (int)(sizeof(StepParams) / 4);
 static_assert(sizeof(StepParams) % 4 == 0, "StepParams is copied as 32-bit words");
 
@@ -59,12 +61,19 @@ __device__ __forceinline__ void batch_load_params(StepParams *dst, const StepPar
 // D2Q9 advances two rows at a time on packed FP32x2 (h_ypair_w), which puts 18
 // loads in flight per thread where a row puts 9 and halves the FP32
 // instructions; a pair that holds a boundary-slot node goes row by row, as
-// D3Q19 does (two nodes would spill).  Latency-bound at 28 warps per SM.
-// Sixteen MRT cavities of sides 64..768, F16S: 60.2 us a step row by row with
-// 4-row tiles, 43.5 (6 or 8 blocks per SM: 43.7, 48.1); eight 1024 x 256 TRT
-// channels, F32: 51.9 and 46.9.
-template <int Q, int COLL, int ST, bool PHYS>
-__global__ void __launch_bounds__(STEP_BLOCK, batch_resident(Q))
+// D3Q19 does (two nodes would spill).  Latency-bound.  us a step, F16S MRT and
+// F32 TRT, row by row with 4-row tiles, then in pairs with RES = 7, 6, 5 blocks
+// per SM (72, 80, 96 registers; up to 60 bytes of spills at 72, 24 at 80, 4 at
+// 96):
+//   16 x 500^2   66.2: 48.8 46.7 49.8     74.3: 58.4 55.6 58.9
+//    4 x 736^2   26.9: 26.0 25.5 25.6     42.2: 33.8 32.3 34.3
+//    8 x 256^2   10.6:  9.5  9.5  8.3     10.5:  9.1  9.2  8.3
+//    3 x 320^2    6.9:  7.3  6.9  6.8      6.9:  7.0  6.7  6.6
+// and TRT channels, F32, whose inlet and outlet tiles go row by row:
+//    8 x 1024 x 256   50.9: 45.7 49.6 55.9
+//    5 x 736 x 184    13.7: 14.0 13.0 14.7
+template <int Q, int COLL, int ST, bool PHYS, int RES>
+__global__ void __launch_bounds__(STEP_BLOCK, RES)
 batch_step_kernel(const StepParams *__restrict__ tab, const int4 *__restrict__ tiles, const int *__restrict__ count) {
     __shared__ StepParams sp[BATCH_WARPS];
     const int ntiles = count[0], tile_rows = count[1];
@@ -187,13 +196,17 @@ batch_residual_final(const double2 *partial, const int2 *ranges, double *res) {
 
 using BatchKernel = void (*)(const StepParams *, const int4 *, const int *);
 
-BatchKernel batch_kernel(int q, int coll, int st, int phys) {
-#define B_CASE(Q, C, S, P) \
-    if (q == Q && coll == C && st == S && (phys != 0) == P) return batch_step_kernel<Q, C, S, P>;
-    B_CASE(9, 1, 0, true) B_CASE(9, 2, 0, true) B_CASE(9, 3, 0, true)
-    B_CASE(9, 1, 1, true) B_CASE(9, 2, 1, true) B_CASE(9, 3, 1, true)
-    B_CASE(19, 1, 0, true) B_CASE(19, 2, 0, true) B_CASE(19, 3, 0, true)
-    B_CASE(19, 1, 1, true) B_CASE(19, 2, 1, true) B_CASE(19, 3, 1, true)
+// The step kernel of a batch, D2Q9 in a form of BATCH_RESIDENT.
+BatchKernel batch_kernel(int q, int coll, int st, int phys, int form) {
+#define B_CASE(Q, C, S, P, F, R) \
+    if (q == Q && coll == C && st == S && (phys != 0) == P && form == F) return batch_step_kernel<Q, C, S, P, R>;
+#define B_CASE9(C, S) B_CASE(9, C, S, true, 0, BATCH_RESIDENT[0]) B_CASE(9, C, S, true, 1, BATCH_RESIDENT[1]) \
+    B_CASE(9, C, S, true, 2, BATCH_RESIDENT[2])
+#define B_CASE19(C, S) B_CASE(19, C, S, true, 0, BATCH_RESIDENT3)
+    B_CASE9(1, 0) B_CASE9(2, 0) B_CASE9(3, 0) B_CASE9(1, 1) B_CASE9(2, 1) B_CASE9(3, 1)
+    B_CASE19(1, 0) B_CASE19(2, 0) B_CASE19(3, 0) B_CASE19(1, 1) B_CASE19(2, 1) B_CASE19(3, 1)
+#undef B_CASE19
+#undef B_CASE9
 #undef B_CASE
     return nullptr;
 }
@@ -237,8 +250,9 @@ struct lbm_batch_s {
     std::vector<int> dom_buf;          // buffer holding each domain's state
     std::vector<std::vector<long long>> slot_node;  // per domain: node of each boundary slot
     std::vector<double> residual;
-    int grid = 0;
-    BatchKernel kern = nullptr;
+    BatchKernel kern[BATCH_FORMS] = {};  // forms of the step kernel (BATCH_RESIDENT)
+    int grids[BATCH_FORMS] = {}, form = 0;
+    std::vector<char> slot_rows;         // per domain: boundary-slot nodes in most rows
     cudaStream_t stream = nullptr;
     cudaEvent_t stepped = nullptr;  // after the last lbm_batch_step, on its stream
     cudaGraphExec_t graph = nullptr;
@@ -311,24 +325,44 @@ static long long batch_tiles_of(const lbm_batch_s *B, int d, int rows) {
     return (long long)((B->n[d] + 31) / 32) * (((long long)B->m[d] * B->h[d] + rows - 1) / rows);
 }
 
-// Rows per tile: each resident warp takes ceil(tiles / warps) tiles, and a
-// tile costs its rows and about one more (its parameters, the first flag
-// word); the even count that makes the busiest warp's share least.  Eight
-// 1024 x 256 channels: 4 rows leave the last of four rounds 85 % empty on
-// 3648 warps, 16 rows fill 4256 warps once.
-static int batch_rows(const lbm_batch_s *B) {
-    const long long warps = (long long)B->grid * BATCH_WARPS;
+// Rows per tile and form of the kernel: each resident warp takes
+// ceil(tiles / warps) tiles, and a tile costs its rows and about one more (its
+// parameters, the first flag word); the even count that makes the busiest
+// warp's share least.  Eight 1024 x 256 channels: 4 rows leave the last of four
+// rounds 85 % empty on 3648 warps, 20 rows nearly fill them once.  Where the
+// form with five blocks per SM does no worse by that count than the one with
+// six, its registers, which hold all of a pair, make it the faster (8 x 256^2
+// and 3 x 320^2 above).  Seven blocks pay for their spills only where shorter
+// tiles cut a tail: a sixth fewer rows, and domains with boundary-slot nodes in
+// most rows, whose tiles that hold them take twice as long as the others
+// (8 x 1024 x 256 above; 4 x 736^2, of the same tiles without such, 33.6 us with
+// seven, 32.3 with six).
+static int batch_rows(lbm_batch_s *B) {
+    const int form = B->form;
+    bool slot_rows = false;
+    for (int d = 0; d < B->ndom; ++d) slot_rows = slot_rows || (B->active[d] && B->slot_rows[d]);
     long long best = -1;
     int rows = BATCH_MIN_ROWS;
-    for (int r = BATCH_MIN_ROWS; r <= BATCH_MAX_ROWS; r += 2) {
-        long long t = 0;
-        for (int d = 0; d < B->ndom; ++d)
-            if (B->active[d]) t += batch_tiles_of(B, d, r);
-        const long long cost = (t + warps - 1) / warps * (r + 1);
-        if (best < 0 || cost < best) {
-            best = cost;
-            rows = r;
+    for (const int f : {1, 0, 2}) {
+        if (!B->kern[f] || (f == 2 && !slot_rows)) continue;
+        const long long warps = (long long)B->grids[f] * BATCH_WARPS;
+        const long long limit = f == 2 ? best * 5 / 6 : LLONG_MAX;
+        for (int r = BATCH_MIN_ROWS; r <= BATCH_MAX_ROWS; r += 2) {
+            long long t = 0;
+            for (int d = 0; d < B->ndom; ++d)
+                if (B->active[d]) t += batch_tiles_of(B, d, r);
+            const long long cost = (t + warps - 1) / warps * (r + 1);
+            if (best < 0 || (cost < best && cost <= limit)) {
+                best = cost;
+                rows = r;
+                B->form = f;
+            }
         }
+    }
+    if (B->form != form && B->graph) {  // it holds the other form
+        cudaGraphExecDestroy(B->graph);
+        B->graph = nullptr;
+        B->graph_steps = 0;
     }
     return rows;
 }
@@ -364,7 +398,8 @@ static int batch_upload_tiles(lbm_batch_s *B) {
 static cudaError_t batch_launch(lbm_batch_s *B, int parity, int write_macro, cudaStream_t s) {
     const StepParams *tab = B->tab + (size_t)(parity * 2 + write_macro) * B->ndom;
     void *args[] = {(void *)&tab, (void *)&B->tiles, (void *)&B->ntiles_d};
-    return cudaLaunchKernel((const void *)B->kern, dim3((unsigned)B->grid), dim3(STEP_BLOCK), args, 0, s);
+    return cudaLaunchKernel((const void *)B->kern[B->form], dim3((unsigned)B->grids[B->form]), dim3(STEP_BLOCK), args, 0,
+                            s);
 }
 
 extern "C" {
@@ -383,8 +418,9 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
     B->coll = params[0].collision_model;
     B->storage = params[0].storage;
     B->elem = B->storage == LBM_STORE_F32 ? 4 : (B->storage == LBM_STORE_F16S ? 2 : 8);
-    B->kern = batch_kernel(B->q, B->coll, B->storage, params[0].mode == LBM_MODE_PHYSICS);
-    if (!B->kern) {
+    for (int f = 0; f < BATCH_FORMS; ++f)
+        B->kern[f] = batch_kernel(B->q, B->coll, B->storage, params[0].mode == LBM_MODE_PHYSICS, f);
+    if (!B->kern[0]) {
         batch_free(B);
         return bfail(LBM_ERR_UNSUPPORTED, "batches run in physics mode with F32 or F16S storage");
     }
@@ -428,6 +464,9 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
         for (long long i = 0; i < N; ++i) fl += L.node_type[i] & 1;
         B->fluid.push_back(fl);
         B->total_fluid += fl;
+        std::vector<char> has((size_t)L.m * h, 0);
+        for (long long node : flags[d].slot_node) has[(size_t)(node / L.n)] = 1;
+        B->slot_rows.push_back(2 * std::count(has.begin(), has.end(), 1) > (long long)has.size());
     }
     const long long nslots = B->slot_off[count - 1] + (long long)flags[count - 1].slot_node.size();
     if (B->total_nodes >= (1ll << 31)) {
@@ -503,11 +542,14 @@ int lbm_batch_create(const lbm_lattice_desc *const *lattices, const lbm_params *
         batch_free(B);
         return bfail(LBM_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
     }
-    int dev = 0, sms = 0, bps = 0;
+    int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, B->kern, STEP_BLOCK, 0);
-    B->grid = std::max(1, sms * std::max(bps, 1));
+    for (int f = 0; f < BATCH_FORMS; ++f) {
+        int bps = 0;
+        if (B->kern[f]) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, B->kern[f], STEP_BLOCK, 0);
+        B->grids[f] = std::max(1, sms * std::max(bps, 1));
+    }
     int rc = batch_upload_tiles(B);
     if (rc) {
         batch_free(B);
@@ -594,7 +636,7 @@ int lbm_batch_step(lbm_batch B, int nsteps, int write_macro_last, void *stream) 
 int lbm_batch_residuals(lbm_batch B, double *res) {
     if (!B || !res) return bfail(LBM_ERR_INVALID, "null argument");
     cudaStreamWaitEvent(B->stream, B->stepped, 0);
-    batch_residual_partial<<<B->grid, STEP_BLOCK, 0, B->stream>>>(B->tab, B->tiles, B->ntiles_d, B->pu, B->partial);
+    batch_residual_partial<<<B->grids[0], STEP_BLOCK, 0, B->stream>>>(B->tab, B->tiles, B->ntiles_d, B->pu, B->partial);
     std::vector<double> r(B->residual);
     cudaError_t e = cudaMemcpyAsync(B->res_d, r.data(), sizeof(double) * B->ndom, cudaMemcpyHostToDevice, B->stream);
     batch_residual_final<<<(unsigned)B->ndom, RES_BLOCK, 0, B->stream>>>(B->partial, B->ranges_d, B->res_d);
