@@ -340,3 +340,30 @@ def test_cg_gpu_tile_edges(n, m, ho, enh):
         mac = s.macro()
     for g, o in zip([rf, bf] + list(mac), (orc.rfc, orc.bfc, orc.rr, orc.br, orc.u, orc.v)):
         assert np.abs(g - o).max() < 2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m", [(5, 5), (31, 7), (32, 8), (33, 5), (34, 13), (66, 6), (1000, 1024)])
+@pytest.mark.parametrize("ho,enh", [(0, 0), (1, 1)])
+@pytest.mark.parametrize("storage", ["f64", "f16s"])
+def test_cg_gpu_tile_edges_of_storages(n, m, ho, enh, storage):
+    """F64 storage, whose tiles are 32 x 4 nodes (32 x 8 where those divide the
+    lattice better over the SMs, as the last one), and F16S at the edges of
+    tiles.  Tolerances as test_cg_gpu_f64_storage_matches_fp64_oracle and
+    test_cg_gpu_f16s_storage_close_to_oracle."""
+    from thesis_gb300 import native as N
+    a, p, r0, b0 = _gpu_case(n, m, ho, enh, seed=n)
+    a.storage = N.STORE_F64 if storage == "f64" else N.STORE_F16S
+    orc = po.run_oracle_cg(n, m, p, r0, b0, 5, fp64=True, extra_collide=True)
+    with mp.CgSolver(n, m, a) as s:
+        s.init(r0, b0)
+        s.step(2, write_macro=False)
+        s.step(3, write_macro=True)
+        rf, bf = s.populations()
+        rr, br, u, v = s.macro()
+    ef = max(np.abs(rf - orc.rfc).max(), np.abs(bf - orc.bfc).max())
+    ed = max(np.abs(rr - orc.rr).max(), np.abs(br - orc.br).max())
+    assert ef < (1e-7 if storage == "f64" else 2e-3)
+    assert ed < (4e-7 if storage == "f64" else 5e-3)
+    if storage == "f64":
+        assert max(np.abs(u - orc.u).max(), np.abs(v - orc.v).max()) < 1e-7

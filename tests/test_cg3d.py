@@ -191,3 +191,28 @@ def test_cg3d_gpu_tile_edges(n, m, h, enh):
         mac = s.macro()
     for g, o in zip([rf, bf] + list(mac), (orc.rfc, orc.bfc, orc.rr, orc.br, orc.u, orc.v, orc.w)):
         assert np.abs(g - o).max() < 2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m,h", [(5, 5, 5), (31, 7, 6), (130, 5, 9)])
+@pytest.mark.parametrize("ho,enh", [(0, 0), (0, 1), (1, 0)])
+@pytest.mark.parametrize("storage", ["f64", "f16s"])
+def test_cg3d_gpu_storages(n, m, h, ho, enh, storage):
+    """F64 and F16S storage, two launches per step with either gradient, at the
+    edges of blocks.  Tolerances as the 2D tests of these storages."""
+    from thesis_gb300 import native as N
+    a, p, r0, b0 = _gpu_case(n, m, h, ho, enh, seed=n)
+    a.storage = N.STORE_F64 if storage == "f64" else N.STORE_F16S
+    orc = po.run_oracle_cg3(n, m, h, p, r0, b0, 5, fp64=True, extra_collide=True)
+    with mp.CgSolver(n, m, a, h=h) as s:
+        s.init(r0, b0)
+        s.step(2, write_macro=False)
+        s.step(3, write_macro=True)
+        rf, bf = s.populations()
+        mac = s.macro()
+    ef = max(np.abs(rf - orc.rfc).max(), np.abs(bf - orc.bfc).max())
+    ed = max(np.abs(mac[0] - orc.rr).max(), np.abs(mac[1] - orc.br).max())
+    assert ef < (1e-7 if storage == "f64" else 2e-3)
+    assert ed < (4e-7 if storage == "f64" else 5e-3)
+    if storage == "f64":
+        assert max(np.abs(g - o).max() for g, o in zip(mac[2:], (orc.u, orc.v, orc.w))) < 1e-7

@@ -44,7 +44,12 @@ struct CgArgs {
     CgModel<V> p;
 };
 
-constexpr int CG_TX = 32, CG_TY = 8;  // tile of a block, one node per thread
+// Tile of a block, 32 x TY nodes, one per thread, and the blocks per SM the step
+// kernel is compiled for.  FP32 and 16-bit storage: TY = 8 at 40 registers (six
+// blocks of 256 threads).  F64 is bound by FP64 operations and would spill 212
+// to 384 bytes at 40; it takes 80 registers and one of two heights (cg_tile_f64).
+constexpr int CG_TX = 32;
+constexpr int cg_resident(int st, int ty) { return st == LBM_STORE_F64 ? (ty == 8 ? 3 : 6) : 6; }
 // rest weights phi_k + theta_k alpha; in constant memory, where they cost an
 // operand: as literals they change which products the compiler fuses, and so
 // the last bits of a droplet's small velocities
@@ -85,18 +90,17 @@ __device__ __forceinline__ void cg_gather(const CgArgs<typename CgStore<ST>::R> 
     }
 }
 
-template <int ST, bool PULL, bool HO, bool ENH>
-__global__ void __launch_bounds__(CG_TX * CG_TY, 6) cg_step_kernel(const CgArgs<typename CgStore<ST>::R> a) {
+template <int ST, int TY, bool PULL, bool HO, bool ENH>
+__global__ void __launch_bounds__(CG_TX * TY, cg_resident(ST, TY)) cg_step_kernel(const CgArgs<typename CgStore<ST>::R> a) {
     using L = Lat<9>;
     using SP = CgStore<ST>;
     using T = typename SP::T;
     using R = typename SP::R;
-    constexpr int H = HO ? 2 : 1, W = CG_TX + 2 * H, RING = 2 * H * W + 2 * H * CG_TY;
-    static_assert(RING <= CG_TX * CG_TY, "one ring node per thread");
-    __shared__ R s_phi[(CG_TY + 2 * H) * W];
-    __shared__ R s_dn[ENH ? (CG_TY + 2 * H) * W : 1];
+    constexpr int H = HO ? 2 : 1, W = CG_TX + 2 * H, RING = 2 * H * W + 2 * H * TY;
+    __shared__ R s_phi[(TY + 2 * H) * W];
+    __shared__ R s_dn[ENH ? (TY + 2 * H) * W : 1];
     const int tid = threadIdx.x, lx = tid % CG_TX, ly = tid / CG_TX;
-    const int x0 = blockIdx.x * CG_TX, y0 = blockIdx.y * CG_TY, x = x0 + lx, y = y0 + ly;
+    const int x0 = blockIdx.x * CG_TX, y0 = blockIdx.y * TY, x = x0 + lx, y = y0 + ly;
     // colour field and density of tile position (cx, cy), from -H; past a
     // lattice face the position is the wrapped node's
     auto put = [&](int cx, int cy, R rr, R bb) {
@@ -121,17 +125,18 @@ __global__ void __launch_bounds__(CG_TX * CG_TY, 6) cg_step_kernel(const CgArgs<
             }
             put(lx, ly, r_r, b_r);
         }
-        if (tid < RING) {
+#pragma unroll 1
+        for (int t = tid; t < RING; t += CG_TX * TY) {
             // rows below and above the tile, then the columns beside it
             int cx, cy;
-            if (tid < 2 * H * W) {
-                const int row = tid / W;
-                cx = tid % W - H;
-                cy = row < H ? row - H : CG_TY + row - H;
+            if (t < 2 * H * W) {
+                const int row = t / W;
+                cx = t % W - H;
+                cy = row < H ? row - H : TY + row - H;
             } else {
-                const int j = tid - 2 * H * W, col = j / CG_TY;
+                const int j = t - 2 * H * W, col = j / TY;
                 cx = col < H ? col - H : CG_TX + col - H;
-                cy = j % CG_TY;
+                cy = j % TY;
             }
             const int gx = x0 + cx, gy = y0 + cy;
             if (gx < a.nx + H && gy < a.ny + H) {
@@ -324,10 +329,12 @@ struct lbm_cg_handle_s {
     int st = LBM_STORE_F32;          // population storage (lbm_cg_store.cuh)
     void *buf = nullptr;             // 2 buffers x 2 slots x q directions x N values
     float *R = nullptr, *B = nullptr, *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr;
-    void *phi = nullptr, *dn = nullptr;  // 3D high order: colour field and density (arithmetic type)
+    void *phi = nullptr, *dn = nullptr;  // 3D, two launches per step: colour field and density (arithmetic type)
     double *partial = nullptr, *sums = nullptr;
     int cur = 0;
     int sms = 1;
+    int tile = 8;                    // 2D: rows of a block's tile
+    int planes = 1;                  // 3D, one launch per step: planes a block marches over
     float scale = 1024.f;            // F16S: scale of the summed population's deviation
     cudaStream_t stream = nullptr;
     cudaEvent_t stepped = nullptr;  // after the last lbm_cg_step, on its stream
@@ -377,22 +384,21 @@ static Cg3Args<R> cg3_args(const lbm_cg_handle_s *H, int from, int write_macro, 
     return a;
 }
 
-template <int ST, bool PULL>
-static void cg3_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
-    const auto a = cg3_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
-    if (H->P.high_order) {
-        const dim3 grid((unsigned)((H->n + CG3_BLOCK - 1) / CG3_BLOCK), (unsigned)H->m, (unsigned)H->h);
-        cg3_density_kernel<ST, PULL><<<grid, CG3_BLOCK, 0, s>>>(a);
-        if (H->P.enhanced) cg3_collide_kernel<ST, PULL, true><<<grid, CG3_BLOCK, 0, s>>>(a);
-        else cg3_collide_kernel<ST, PULL, false><<<grid, CG3_BLOCK, 0, s>>>(a);
-        return;
-    }
-    // The planes a block marches over: the cut along z with the fewest plane
-    // steps in a row, waves of resident blocks times a block's planes and the
-    // two it pulls for phi alone (256^3: 10 blocks along z, against 1 that
-    // leaves a third of the SMs' places empty, 1.41 against 1.22 ms)
-    const unsigned tx = (unsigned)((H->n + CG3_TX - 1) / CG3_TX), ty = (unsigned)((H->m + CG3_TY - 1) / CG3_TY);
-    const long long tiles = (long long)tx * ty, places = (long long)H->sms * CG3_RESIDENT;
+// Where a 3D step is one launch (cg3_step_kernel): FP32 storage with the
+// 18-neighbour gradient.  F16S, whose ring pulls cost conversions, and F64, whose
+// registers spill, are faster in two launches; us a step, two / one: 128^3 F16S
+// 170 / 211, F64 2890 / 3560, FP32 185 / 162; 96 x 90 x 80 F16S 60.7 / 73.9, F64
+// 1016 / 1154, FP32 68.7 / 60.1 (160 x 131 x 97 F16S with the enhanced
+// equilibrium is the one measured the other way, 217 / 212).
+static constexpr bool cg3_one_launch(int st, int high_order) { return st == LBM_STORE_F32 && !high_order; }
+
+// The planes a block marches over: the cut along z with the fewest plane steps
+// in a row, waves of resident blocks times a block's planes and the two it pulls
+// for phi alone (256^3: 10 blocks along z, against 1 that leaves a third of the
+// SMs' places empty, 1.41 against 1.22 ms).
+static int cg3_planes(const lbm_cg_handle_s *H) {
+    const long long tiles = (long long)((H->n + CG3_TX - 1) / CG3_TX) * ((H->m + CG3_TY - 1) / CG3_TY);
+    const long long places = (long long)H->sms * CG3_RESIDENT;
     int planes = H->h;
     long long best = -1;
     for (int c = 1; c <= (H->h + 1) / 2; ++c) {
@@ -403,23 +409,65 @@ static void cg3_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, i
             planes = k;
         }
     }
-    const dim3 grid(tx, ty, (unsigned)((H->h + planes - 1) / planes));
-    if (H->P.enhanced) cg3_step_kernel<ST, PULL, true><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, planes);
-    else cg3_step_kernel<ST, PULL, false><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, planes);
+    return planes;
+}
+
+template <int ST, bool PULL>
+static void cg3_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
+    const auto a = cg3_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
+    if (!cg3_one_launch(ST, H->P.high_order)) {
+        const dim3 grid((unsigned)((H->n + CG3_BLOCK - 1) / CG3_BLOCK), (unsigned)H->m, (unsigned)H->h);
+        cg3_density_kernel<ST, PULL><<<grid, CG3_BLOCK, 0, s>>>(a);
+        if (H->P.high_order) {
+            if (H->P.enhanced) cg3_collide_kernel<ST, PULL, true, true><<<grid, CG3_BLOCK, 0, s>>>(a);
+            else cg3_collide_kernel<ST, PULL, true, false><<<grid, CG3_BLOCK, 0, s>>>(a);
+        } else if constexpr (!cg3_one_launch(ST, 0)) {
+            if (H->P.enhanced) cg3_collide_kernel<ST, PULL, false, true><<<grid, CG3_BLOCK, 0, s>>>(a);
+            else cg3_collide_kernel<ST, PULL, false, false><<<grid, CG3_BLOCK, 0, s>>>(a);
+        }
+        return;
+    }
+    if constexpr (cg3_one_launch(ST, 0)) {
+        const dim3 grid((unsigned)((H->n + CG3_TX - 1) / CG3_TX), (unsigned)((H->m + CG3_TY - 1) / CG3_TY),
+                        (unsigned)((H->h + H->planes - 1) / H->planes));
+        if (H->P.enhanced) cg3_step_kernel<ST, PULL, true><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, H->planes);
+        else cg3_step_kernel<ST, PULL, false><<<grid, CG3_TX * CG3_TY, 0, s>>>(a, H->planes);
+    }
+}
+
+template <int ST, int TY, bool PULL>
+static void cg_launch_tile(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
+    const auto a = cg_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
+    const dim3 grid((unsigned)((H->n + CG_TX - 1) / CG_TX), (unsigned)((H->m + TY - 1) / TY));
+    if (H->P.high_order) {
+        if (H->P.enhanced) cg_step_kernel<ST, TY, PULL, true, true><<<grid, CG_TX * TY, 0, s>>>(a);
+        else cg_step_kernel<ST, TY, PULL, true, false><<<grid, CG_TX * TY, 0, s>>>(a);
+    } else {
+        if (H->P.enhanced) cg_step_kernel<ST, TY, PULL, false, true><<<grid, CG_TX * TY, 0, s>>>(a);
+        else cg_step_kernel<ST, TY, PULL, false, false><<<grid, CG_TX * TY, 0, s>>>(a);
+    }
+}
+
+// Tile height of an F64 step: the one whose busiest SM has the least work, in
+// nodes, a ring node (one pull, no collision) counted as a sixteenth.  us a
+// step, plain gradient, two launches / TY = 8 / TY = 4: 1024^2 791 / 769 / 785,
+// 500 x 400 160 / 164 / 156, 200 x 180 49.5 / 55.6 / 45.5, 130 x 97 37.1 / 33.1 /
+// 20.7.
+static int cg_tile_f64(const lbm_cg_handle_s *H) {
+    auto busiest = [&](int ty) {
+        const long long tiles = (long long)((H->n + CG_TX - 1) / CG_TX) * ((H->m + ty - 1) / ty);
+        const int r = H->P.high_order ? 2 : 1, ring = 2 * r * (CG_TX + 2 * r + ty);
+        return (tiles + H->sms - 1) / H->sms * (16 * CG_TX * ty + ring);
+    };
+    return busiest(8) <= busiest(4) ? 8 : 4;
 }
 
 template <int ST, bool PULL>
 static void cg_launch_st(const lbm_cg_handle_s *H, int from, int write_macro, int write_rb, cudaStream_t s) {
-    const auto a = cg_args<typename CgStore<ST>::R>(H, from, write_macro, write_rb);
-    const dim3 grid((unsigned)((H->n + CG_TX - 1) / CG_TX), (unsigned)((H->m + CG_TY - 1) / CG_TY));
-    constexpr int CG_BLOCK = CG_TX * CG_TY;
-    if (H->P.high_order) {
-        if (H->P.enhanced) cg_step_kernel<ST, PULL, true, true><<<grid, CG_BLOCK, 0, s>>>(a);
-        else cg_step_kernel<ST, PULL, true, false><<<grid, CG_BLOCK, 0, s>>>(a);
-    } else {
-        if (H->P.enhanced) cg_step_kernel<ST, PULL, false, true><<<grid, CG_BLOCK, 0, s>>>(a);
-        else cg_step_kernel<ST, PULL, false, false><<<grid, CG_BLOCK, 0, s>>>(a);
+    if constexpr (ST == LBM_STORE_F64) {
+        if (H->tile == 4) return cg_launch_tile<ST, 4, PULL>(H, from, write_macro, write_rb, s);
     }
+    cg_launch_tile<ST, 8, PULL>(H, from, write_macro, write_rb, s);
 }
 
 // One step (PULL) or the first collision from a given post-stream state.
@@ -463,12 +511,15 @@ static int cg_create(int n, int m, int h, const lbm_cg_params *P, lbm_cg_handle 
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&H->sms, cudaDevAttrMultiProcessorCount, dev);
         if (H->sms < 1) H->sms = 1;
+        if (H->q == 19) H->planes = cg3_planes(H);
+        else if (H->st == LBM_STORE_F64) H->tile = cg_tile_f64(H);
     }
     const size_t N = (size_t)H->N;
     const size_t rbytes = H->st == LBM_STORE_F64 ? sizeof(double) : sizeof(float);
     cudaError_t e = cudaMalloc((void **)&H->buf, 4 * H->slot_bytes());
     if (e == cudaSuccess) e = cudaMalloc((void **)&H->R, sizeof(float) * 6 * N);
-    if (e == cudaSuccess && H->q == 19 && H->P.high_order) e = cudaMalloc((void **)&H->phi, rbytes * 2 * N);
+    if (e == cudaSuccess && H->q == 19 && !cg3_one_launch(H->st, H->P.high_order))
+        e = cudaMalloc((void **)&H->phi, rbytes * 2 * N);
     if (e == cudaSuccess) e = cudaMalloc((void **)&H->partial, sizeof(double) * (LAP_BLOCKS * 5 + 5));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&H->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&H->stepped, cudaEventDisableTiming);

@@ -4,10 +4,10 @@
 // streaming gpuStreaming3DCG, GpuStream.cu:196-250; densities and velocity
 // of gpuUpdateMacro3DCG, GpuUpdateMacro.cu:215-360).
 //
-// With the 18-neighbour gradient a step is one launch (cg3_step_kernel): a
-// block marches a 32 x 8 tile along z and pulls both colours of every node
-// once.  With the 104-point gradient, which reaches two planes away, a step is
-// two launches:
+// With FP32 storage and the 18-neighbour gradient a step is one launch
+// (cg3_step_kernel): a block marches a 32 x 4 tile along z and pulls both
+// colours of every node once.  With the 104-point gradient, which reaches two
+// planes away, and with the other storages a step is two launches:
 //   cg3_density_kernel  pull both colours, write the colour field
 //                       phi = (rho_r - rho_b)/rho and rho per node;
 //   cg3_collide_kernel  pull both colours again, take the neighbours' phi and
@@ -15,8 +15,9 @@
 //                       write both colours.
 // State between steps: post-collision red and blue populations, SoA by
 // direction (direction d of colour c at base + (c*19 + d) N), pull double
-// buffer.  HBM-bound: per FP32 update the one launch reads and writes 152 B of
-// populations per colour pair, the two launches read them twice.
+// buffer.  Per FP32 update the one launch reads and writes 152 B of populations,
+// the two launches read them twice; the first is bound by instructions and
+// latency, the second by HBM in FP32.
 #pragma once
 #include "lbm_cg_store.cuh"
 #include "lbm_device.cuh"
@@ -195,10 +196,11 @@ __device__ __forceinline__ void cg3_relax(const Cg3Args<typename CgStore<ST>::R>
     }
 }
 
-// The two-launch form's second kernel (104-point gradient): moments of the
-// streamed colours, the colour and density gradients from the neighbours'
-// fields, the collision.
-template <int ST, bool PULL, bool ENH>
+// The two-launch form's second kernel: moments of the streamed colours, the
+// colour and density gradients from the neighbours' fields (18 lattice
+// neighbours, weights 1/6 and 1/12, or the 104-point set when HO), the
+// collision.
+template <int ST, bool PULL, bool HO, bool ENH>
 __global__ void __launch_bounds__(CG3_BLOCK, CG3_MINB) cg3_collide_kernel(const Cg3Args<typename CgStore<ST>::R> a) {
     using L = Lat<19>;
     using SP = CgStore<ST>;
@@ -249,23 +251,30 @@ __global__ void __launch_bounds__(CG3_BLOCK, CG3_MINB) cg3_collide_kernel(const 
         cgy += a1 * (R)oy;
         cgz += a1 * (R)oz;
     };
-    int xo[5], yo[5], zo[5];
+    if (HO) {
+        int xo[5], yo[5], zo[5];
 #pragma unroll
-    for (int t = 0; t < 5; ++t) {
-        xo[t] = cg3_wrap(x + t - 2, a.nx);
-        yo[t] = a.nx * cg3_wrap(y + t - 2, a.ny);
-        zo[t] = plane * cg3_wrap(z + t - 2, a.nz);
+        for (int t = 0; t < 5; ++t) {
+            xo[t] = cg3_wrap(x + t - 2, a.nx);
+            yo[t] = a.nx * cg3_wrap(y + t - 2, a.ny);
+            zo[t] = plane * cg3_wrap(z + t - 2, a.nz);
+        }
+#pragma unroll
+        for (int ox = -2; ox <= 2; ++ox)
+#pragma unroll
+            for (int oy = -2; oy <= 2; ++oy)
+#pragma unroll
+                for (int oz = -2; oz <= 2; ++oz) {
+                    const R wt = cg3_ho_weight<R>(ox * ox + oy * oy + oz * oz);
+                    if (wt == (R)0) continue;
+                    add(xo[ox + 2] + yo[oy + 2] + zo[oz + 2], wt, ox, oy, oz);
+                }
+    } else {
+#pragma unroll
+        for (int k = 1; k < 19; ++k)
+            add(nb.at(L::cx(k), L::cy(k), L::cz(k)), k <= 6 ? (R)(1. / 6.) : (R)(1. / 12.), L::cx(k), L::cy(k),
+                L::cz(k));
     }
-#pragma unroll
-    for (int ox = -2; ox <= 2; ++ox)
-#pragma unroll
-        for (int oy = -2; oy <= 2; ++oy)
-#pragma unroll
-            for (int oz = -2; oz <= 2; ++oz) {
-                const R wt = cg3_ho_weight<R>(ox * ox + oy * oy + oz * oz);
-                if (wt == (R)0) continue;
-                add(xo[ox + 2] + yo[oy + 2] + zo[oz + 2], wt, ox, oy, oz);
-            }
     cg3_relax<ST, ENH>(a, node, f, r_r, b_r, rho, u, v, w, cgx, cgy, cgz, grx, gry, grz);
 }
 
