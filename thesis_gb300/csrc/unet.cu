@@ -349,15 +349,15 @@ __global__ void __launch_bounds__(1024) bias_final_kernel(const __grid_constant_
     }
 }
 
-// dpre[p][c] = g[p][c] * (act[p][c] > 0)
-__global__ void __launch_bounds__(256) relu_bwd_kernel(const bf16 *g, int g_cs, int g_co, const bf16 *act, int a_cs,
-                                                       int a_co, bf16 *dpre, int C, int npix, float *rows) {
+// dpre[p][c] *= (act[p][c] > 0), in place: an item is read and written by one thread
+__global__ void __launch_bounds__(256) relu_bwd_kernel(bf16 *dpre, const bf16 *act, int a_cs, int a_co, int C, int npix,
+                                                       float *rows) {
     BiasSum bs;
     const int G = C / 8, total = npix * G;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int v = i % G, p = i / G;
+        V8 o = unpack8(*(const uint4 *)(dpre + (size_t)i * 8));
         const V8 a = ld8(act + (size_t)p * a_cs + a_co + 8 * v);
-        V8 o = ld8(g + (size_t)p * g_cs + g_co + 8 * v);
 #pragma unroll
         for (int k = 0; k < 8; ++k) o.v[k] = a.v[k] > 0.f ? o.v[k] : 0.f;
         st8(dpre + (size_t)i * 8, o);
@@ -570,8 +570,8 @@ struct lbm_unet_s {
     // activations per level and their gradients: e_a[l] first encoder conv,
     // cat[l] = [upsampled decoder input | second encoder conv (the skip)],
     // p[l] pooled (level l + 1), d_a[l] / d_b[l] decoder convs, ba / bb bottleneck
-    Act x0, ba, bb, g_ba, g_bb;
-    std::vector<Act> e_a, cat, p, d_a, d_b, g_e_a, g_cat, g_p, g_d_a, g_d_b;
+    Act x0, ba, bb;
+    std::vector<Act> e_a, cat, p, d_a, d_b, g_cat, g_p;
     float *out32 = nullptr;     // [B][H][W][16] FP32 output
     bf16 *dout = nullptr;       // its gradient
     float *bias_part = nullptr;  // [layer][BIAS_ROWS][BIAS_STRIDE] partial bias gradients
@@ -1061,18 +1061,15 @@ void backward(lbm_unet_s *u, int B) {
         conv(u, L[k], view_of(cur, L[k].cout), gin, nullptr, nullptr, B, lev, true);
     };
     // data gradient of layer k through the ReLU of layer below (its
-    // activation act); g is the gradient's own buffer for the two-kernel form
-    auto dgrad_relu = [&](int k, int below, const Act &g, const Act &act, int lev) {
+    // activation act); the unmasked one of a convolution that does not mask is
+    // masked in place
+    auto dgrad_relu = [&](int k, int below, const Act &act, int lev) {
         const int C = L[k].cin;
         bf16 *next = other();
         const ReluMask mask{&act, rows(below), &plan.rows[below]};
-        const Act fused = view_of(next, C), in = view_of(cur, L[k].cout);
-        if (!conv(u, L[k], in, fused, nullptr, nullptr, B, lev, true, &mask)) {
-            // the convolution left the unmasked gradient in `next`
-            cudaMemcpyAsync(g.p, next, sizeof(bf16) * npix(lev) * C, cudaMemcpyDeviceToDevice, u->stream);
+        if (!conv(u, L[k], view_of(cur, L[k].cout), view_of(next, C), nullptr, nullptr, B, lev, true, &mask)) {
             const int grid = plan.rows[below] = sum_grid_for(npix(lev) * C / 8);
-            relu_bwd_kernel<<<grid, 256, 0, u->stream>>>(g.p, C, 0, act.p, act.cs, act.co, next, C, (int)npix(lev),
-                                                         rows(below));
+            relu_bwd_kernel<<<grid, 256, 0, u->stream>>>(next, act.p, act.cs, act.co, C, (int)npix(lev), rows(below));
         }
         cur = next;
     };
@@ -1093,19 +1090,19 @@ void backward(lbm_unet_s *u, int B) {
         cur = next;
     };
     wg(out_layer(u), u->d_b[0], 0);
-    dgrad_relu(out_layer(u), dec_b(u, 0), u->g_d_b[0], u->d_b[0], 0);
+    dgrad_relu(out_layer(u), dec_b(u, 0), u->d_b[0], 0);
     // decoder, from level 0 up; d_b[l] was upsampled into the first channels of cat[l-1]
     for (int l = 0; l < NL; ++l) {
         if (l > 0) up_bwd(dec_b(u, l), view(u->g_cat[l - 1], 0, ch_dec_b(u, l)), u->d_b[l], ch_dec_b(u, l), l);
         wg(dec_b(u, l), u->d_a[l], l);
-        dgrad_relu(dec_b(u, l), dec_a(u, l), u->g_d_a[l], u->d_a[l], l);
+        dgrad_relu(dec_b(u, l), dec_a(u, l), u->d_a[l], l);
         wg(dec_a(u, l), u->cat[l], l);
         dgrad(dec_a(u, l), u->g_cat[l], l);
     }
     // bottleneck
     up_bwd(bott_b(u), view(u->g_cat[NL - 1], 0, ch(u, NL)), u->bb, ch(u, NL), NL);
     wg(bott_b(u), u->ba, NL);
-    dgrad_relu(bott_b(u), bott_a(u), u->g_ba, u->ba, NL);
+    dgrad_relu(bott_b(u), bott_a(u), u->ba, NL);
     wg(bott_a(u), u->p[NL - 1], NL);
     dgrad(bott_a(u), u->g_p[NL - 1], NL);
     // encoder, from the deepest level down
@@ -1113,7 +1110,7 @@ void backward(lbm_unet_s *u, int B) {
         pool_skip(enc_b(l), u->g_p[l], view(u->g_cat[l], ch_up(u, l), ch(u, l)), view(u->cat[l], ch_up(u, l), ch(u, l)),
                   ch(u, l), l);
         wg(enc_b(l), u->e_a[l], l);
-        dgrad_relu(enc_b(l), enc_a(l), u->g_e_a[l], u->e_a[l], l);
+        dgrad_relu(enc_b(l), enc_a(l), u->e_a[l], l);
         wg(enc_a(l), l == 0 ? u->x0 : u->p[l - 1], l);
         if (l > 0) dgrad(enc_a(l), u->g_p[l - 1], l);
     }
@@ -1251,7 +1248,7 @@ int lbm_unet_create(const lbm_unet_config *cfg, lbm_unet *out) {
         rc = rc ? rc : alloc(u, (void **)&l.w, sizeof(bf16) * 9 * l.cin * l.cout);
         rc = rc ? rc : alloc(u, (void **)&l.wt, sizeof(bf16) * 9 * l.cin * l.cout);
     }
-    for (auto *v : {&u->e_a, &u->cat, &u->p, &u->d_a, &u->d_b, &u->g_e_a, &u->g_cat, &u->g_p, &u->g_d_a, &u->g_d_b})
+    for (auto *v : {&u->e_a, &u->cat, &u->p, &u->d_a, &u->d_b, &u->g_cat, &u->g_p})
         v->resize(NL);
     rc = rc ? rc : make_act(u, u->x0, 16, 0);
     for (int l = 0; l < NL; ++l) {
@@ -1260,16 +1257,11 @@ int lbm_unet_create(const lbm_unet_config *cfg, lbm_unet *out) {
         rc = rc ? rc : make_act(u, u->p[l], ch(u, l), l + 1);
         rc = rc ? rc : make_act(u, u->d_a[l], ch(u, l), l);
         rc = rc ? rc : make_act(u, u->d_b[l], ch_dec_b(u, l), l);
-        rc = rc ? rc : make_act(u, u->g_e_a[l], ch(u, l), l);
         rc = rc ? rc : make_act(u, u->g_cat[l], ch_up(u, l) + ch(u, l), l);
         rc = rc ? rc : make_act(u, u->g_p[l], ch(u, l), l + 1);
-        rc = rc ? rc : make_act(u, u->g_d_a[l], ch(u, l), l);
-        rc = rc ? rc : make_act(u, u->g_d_b[l], ch_dec_b(u, l), l);
     }
     rc = rc ? rc : make_act(u, u->ba, ch(u, NL), NL);
     rc = rc ? rc : make_act(u, u->bb, ch(u, NL), NL);
-    rc = rc ? rc : make_act(u, u->g_ba, ch(u, NL), NL);
-    rc = rc ? rc : make_act(u, u->g_bb, ch(u, NL), NL);
     const size_t np = (size_t)cfg->max_batch * cfg->height * cfg->width;
     rc = rc ? rc : alloc(u, (void **)&u->out32, np * 16 * sizeof(float));
     rc = rc ? rc : alloc(u, (void **)&u->dout, np * 16 * sizeof(bf16));
