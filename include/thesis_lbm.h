@@ -306,7 +306,7 @@ long long lbm_fluid_nodes(lbm_handle h);
  * variant the lattice does not admit falls back to 1, except jit and jit2,
  * whose build failure lbm_create reports.  With the default choice, calls of
  * several steps on a 2D lattice that fits the SMs' shared memory (about
- * 440,000 nodes; F32, or F16S in physics mode; boundaries that touch only
+ * 415,000 nodes on 152 SMs; F32, or F16S in physics mode; boundaries that touch only
  * the node's own populations) run in one cooperative launch with the same
  * node arithmetic (lbm_resident.cu); a stream under capture records a launch
  * per step, and so does a call whose cooperative launch the driver refuses. */

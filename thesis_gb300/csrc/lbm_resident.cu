@@ -3,8 +3,8 @@
 //
 // A small 2D lattice is bound by launches, not by work: a 128 x 128 step is
 // 1 MB of L2 traffic and 4 warps per SM, but a launch per step took 4.1 us.
-// Up to about 440,000 nodes both population buffers fit the SMs' shared
-// memory, so one cooperative launch runs all the steps of an lbm_step call:
+// Up to 2728 nodes per SM, with their halo (about 415,000 nodes on 152 SMs, the
+// largest square 632 x 632), both population buffers fit the shared memory, so one cooperative launch runs all the steps of an lbm_step call:
 // every block keeps a rectangular tile with a one-node halo and gathers from
 // it, and only the populations that cross a tile's edge travel through L2.
 //
@@ -216,10 +216,14 @@ __global__ void __launch_bounds__(MAX_COMPUTE + MAX_COMM, 1) resident_kernel(con
 #pragma unroll
                         for (int d = 0; d < 9; ++d) res[d] = S::encode(f[d], p.shift[d], p.scale);
                     }
-                } else {
+                } else if constexpr (PHYS) {
                     const float S0 = ST == LBM_STORE_F16S ? p.scale : 1.f;
 #pragma unroll
                     for (int d = 0; d < 9; ++d) h_put<ST>(&res[d], -p.sigma * p.shift[d] * S0);
+                } else {
+                    // as the f-space kernels: +0 unshifted, where the above is -0
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) res[d] = S::encode(0.f, p.shift[d], p.scale);
                 }
                 if constexpr (LAST) {
                     T *o = (T *)p.fout[0] + node % nx + (long long)g.pitch * (node / nx);
