@@ -192,3 +192,21 @@ def test_tuning_keeps_steps_on_chip(n, m):
     first = run(False)
     assert np.array_equal(first, run(True))
     assert np.array_equal(first, run(False))
+
+
+def test_reductions_beside_a_busy_handle():
+    """A handle that steps while another's launches are in flight reads its
+    residuals without an error: that the other is not ready yet is none."""
+    import torch
+    big, bargs = cavity(600, 600)
+    lat, args = cavity(96, 80)
+    stream = torch.cuda.Stream()
+    with Solver(big, bargs) as b, Solver(lat, args) as s:
+        b.init(*rest(big.num_nodes))
+        s.init(*rest(lat.num_nodes))
+        for _ in range(3):
+            b.step(4000, write_macro=False, stream=stream.cuda_stream)
+            s.step(8)
+            assert np.isfinite(s.residual()[0])
+            assert np.isfinite(s.macro_diff()[0]).all()
+            assert np.isfinite(s.residual_l2()[0])

@@ -284,7 +284,9 @@ static const ResidentPlan &on_chip_plan(const lbm_handle_s *H, cudaStream_t s) {
             const OnChip e = g_on_chip[i];
             if (e.H == H || e.H->res_dev != H->res_dev || e.stream == s) continue;
             if (!relaxed) relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
-            if (cudaEventQuery(e.H->stepped) != cudaErrorNotReady) {
+            const cudaError_t state = cudaEventQuery(e.H->stepped);
+            if (state != cudaSuccess) cudaGetLastError();  // "not ready" would be the next check's error
+            if (state != cudaErrorNotReady) {
                 g_on_chip.erase(g_on_chip.begin() + i--);
             } else {
                 ++others;

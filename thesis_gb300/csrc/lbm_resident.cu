@@ -4,9 +4,13 @@
 // A small 2D lattice is bound by launches, not by work: a 128 x 128 step is
 // 1 MB of L2 traffic and 4 warps per SM, but a launch per step took 4.1 us.
 // Up to 2728 nodes per SM, with their halo (about 415,000 nodes on 152 SMs, the
-// largest square 632 x 632), both population buffers fit the shared memory, so one cooperative launch runs all the steps of an lbm_step call:
-// every block keeps a rectangular tile with a one-node halo and gathers from
-// it, and only the populations that cross a tile's edge travel through L2.
+// largest square 632 x 632), both population buffers fit the shared memory, so
+// one cooperative launch runs all the steps of an lbm_step call: every block
+// keeps a rectangular tile with a one-node halo and gathers from it, and only
+// the populations that cross a tile's edge travel through L2.  Bound by one
+// message flight per step where tiles are small and by FP32 issue where they
+// are large; us a step, a launch per step and here: 61 x 47 MRT 4.1 and 1.5,
+// 128^2 reference BGK 4.1 and 1.6, 256^2 4.1 and 1.8, 1024 x 256 TRT 6.4 and 2.7.
 //
 // Roles.  The `compute` threads update the tile's nodes, the edge nodes
 // first; warps of `comm` threads then send the edge's outgoing populations
@@ -16,12 +20,12 @@
 // reader polls the word itself until it carries the tag of the state it
 // wants.  A tile reads its messages from slots of its own
 // (mail[parity][tile][link], numbered by tile_link), side by side for the lanes
-// that poll them.  Every link that crosses a tile edge is sent
-// and awaited in both directions, blocked or not: neighbouring tiles then
-// advance in lockstep, neither can be two states ahead of the other, and two
-// parities of the mailbox suffice.  The first step takes its halo from the
-// entry state in global memory, the last writes the state (and rho, u when
-// asked) there.
+// that poll them: 128^2, 1000 steps 1.88 -> 1.60 ms against slots by destination
+// node.  Every link that crosses a tile edge is sent and awaited in both
+// directions, blocked or not: neighbouring tiles then advance in lockstep,
+// neither can be two states ahead of the other, and two parities of the mailbox
+// suffice.  The first step takes its halo from the entry state in global memory,
+// the last writes the state (and rho, u when asked) there.
 //
 // Layout.  Direction d of the node at tile index t = lx + 1 + pitch (ly + 1)
 // sits at d * PLANE + t of a buffer: with PLANE fixed at compile time a
