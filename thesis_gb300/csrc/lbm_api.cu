@@ -265,13 +265,13 @@ static void on_chip_add(const lbm_handle_s *H, cudaStream_t s, int tiles) {
 // half, a quarter or an eighth of the SMs, as many parts as there are handles
 // at work: a step of a small lattice is mostly one message flight, whatever the
 // tile.  Handles on streams of their own, 100 steps a call, us for a step of all
-// of them (whole-chip launches one after another; a launch per step):
-//   128^2  x 4: 2.5 (7.3; 4.3)   x 8: 2.8 (14.6; 5.4)
-//   256^2  x 4: 3.2 (8.4; 5.3)   x 8: 6.3 (16.8; 6.5)
-//   400^2  x 4: 5.3 (9.3; 7.0)   x 8: 10.6 (19.2; 13.6)
-// 512^2 and larger fit no part; there the launches take turns (x 4: 9.7, against
-// 9.4 with a launch per step; x 8: 19.6 and 25.7).  Eight of 320^2 fit by fours
-// and are the case left slower than a launch per step: 9.0 and 7.2.
+// of them (whole-chip launches in turn, by the time of one; a launch per step):
+//   128^2  x 4: 2.1 (6.4; 4.3)   x 8: 2.4 (12.8; 5.4)
+//   256^2  x 4: 3.1 (7.3; 5.2)   x 8: 6.0 (14.6; 6.5)
+//   400^2  x 4: 5.1 (8.3; 7.0)   x 8: 10.0 (16.6; 13.6)
+// 512^2 and larger fit no part; there the launches take turns (x 4: 8.5, against
+// 9.4 with a launch per step; x 8: 17.2 and 25.7).  Eight of 320^2 fit by fours
+// and are the case left slower than a launch per step: 8.2 and 7.2.
 static const ResidentPlan &on_chip_plan(const lbm_handle_s *H, cudaStream_t s) {
     int others = 0, used = 0;
     {
