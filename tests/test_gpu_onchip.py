@@ -210,3 +210,20 @@ def test_reductions_beside_a_busy_handle():
             assert np.isfinite(s.residual()[0])
             assert np.isfinite(s.macro_diff()[0]).all()
             assert np.isfinite(s.residual_l2()[0])
+
+
+def test_calls_of_several_launches(monkeypatch):
+    """A call longer than a launch holds (512 steps), and one step longer, gives
+    the state of a launch per step."""
+    lat, args = cavity(70, 45)
+
+    def run():
+        with Solver(lat, args) as s:
+            s.init(*rest(lat.num_nodes))
+            s.step(513)
+            s.step(1100, write_macro=True)
+            return [s.get_state()] + list(s.macro())
+    got = run()
+    monkeypatch.setenv("THESIS_LBM_KERNEL", "jit")
+    for a, b in zip(got, run()):
+        assert np.array_equal(a, b)

@@ -1020,7 +1020,12 @@ static int step_graph(lbm_handle_s *H, int which, int c) {
 // Fewest steps of a call that the on-chip kernel takes: it moves the state
 // on and off the chip once per call.
 constexpr int RESIDENT_MIN_STEPS = 4;
-constexpr int RESIDENT_CHUNK = 8192;  // steps per launch, tens of milliseconds
+// Steps per launch, about a millisecond.  A kernel of another stream that needs
+// the shared memory waits for the launch it meets: beside 128^2 calls of 5000
+// steps a U-Net prediction of twenty kernels took 38 ms with 8192 steps per
+// launch, 15.5 with 512, 8.0 with 256 (0.6 beside a launch per step); a step of
+// 4096 took 1.475, 1.485 and 1.498 us.
+constexpr int RESIDENT_CHUNK = 512;
 
 // Runs up to nsteps steps and returns how many: where the driver refuses a
 // launch (a stream whose context holds fewer SMs than the device, another
